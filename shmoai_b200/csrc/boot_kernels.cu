@@ -145,16 +145,11 @@ void linear_combination(const Context &c, const LinTerms &t, uint64_t *out, uint
 
 void modraise(const Context &c, const uint64_t *in, uint64_t *out, uint32_t n_polys, uint32_t L, uint64_t *ws,
               cudaStream_t st) {
-    // limb 0 of each polynomial (already contiguous when the input has one limb)
-    SHM_CUDA(cudaMemcpyAsync(ws, in, (size_t)n_polys * c.n * 8, cudaMemcpyDeviceToDevice, st));
-    LimbMap m;
-    for (int i = 0; i < 512; i++) m.prime[i] = 255;
-    m.prime[0] = 0;
-    ntt_inverse(c, ws, n_polys, 1, m, nullptr, st);
+    ntt_inverse(c, ws, rows_of(c, n_polys, 1, 1), nullptr, st, in, c.n);
     SHM_LAUNCHED(1);
     modraise_spread<<<dim3(c.n / kT, L, n_polys), kT, 0, st>>>(ws, out, L, c.log_n, c.pc);
     SHM_CUDA(cudaGetLastError());
-    ntt_forward(c, out, n_polys * L, L, q_map(L), st);
+    ntt_forward(c, out, rows_of(c, n_polys, L, L), st);
 }
 
 }  // namespace shm

@@ -37,7 +37,7 @@ void push4(std::vector<uint64_t> &v, uint64_t c, uint64_t psi_half_inv, uint64_t
 Context::~Context() {
     cudaSetDevice(device);
     release_encode_tables(*this);
-    for (void *p : {(void *)pc, (void *)tw, (void *)twq, (void *)inv_scale_plain, (void *)moddown_scale, (void *)moddown_conv,
+    for (void *p : {(void *)pc, (void *)tw, (void *)twd, (void *)inv_scale_plain, (void *)moddown_scale, (void *)moddown_conv,
                     (void *)p_inv, (void *)p_mod, (void *)rescale_inv, arena})
         if (p) cudaFree(p);
     for (auto &l : ks)
@@ -101,6 +101,31 @@ void *Context::workspace(size_t bytes) {
     return arena;
 }
 
+// the tables of TwTab for the primes below kF64CentreLimit (zero for the others, which never read
+// them) from the integer tables [QP][4][N]
+template <int R>
+std::vector<double> fp64_twiddles(const std::vector<uint64_t> &primes, const std::vector<uint64_t> &tw) {
+    using T = TwTab<R>;
+    std::vector<double> out(primes.size() * 2 * T::DIR, 0.0);
+    for (size_t i = 0; i < primes.size(); i++) {
+        const uint64_t q = primes[i];
+        if (q >= kF64CentreLimit) continue;
+        for (int dir = 0; dir < 2; dir++) {
+            const uint64_t *t = tw.data() + (i * 4 + 2 * dir) * T::N;
+            double *d = out.data() + (i * 2 + dir) * T::DIR;
+            auto centred = [&](uint64_t w) { return w > q / 2 ? (double)w - (double)q : (double)w; };
+            for (uint32_t k = 0; k < T::NAT; k++) d[k] = centred(t[k]);
+            for (uint32_t b = 0; b < T::M; b++)
+                for (uint32_t g = 0; g < T::E; g++) {
+                    const uint32_t u = ((T::M + b) << R) + g;
+                    for (int r = 0; r < R; r++)
+                        for (uint32_t k = 0; k < (1u << r); k++) d[T::slot(b, g, (1u << r) + k)] = centred(t[(u << r) + k]);
+                }
+        }
+    }
+    return out;
+}
+
 Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uint32_t nq, uint32_t np, int device) {
     if (log_n != 12 && log_n != 16) throw std::invalid_argument("log_n must be 12 or 16");
     if (nq < 1 || nq + np != primes.size() || nq + np > 250) throw std::invalid_argument("bad prime counts");
@@ -123,7 +148,7 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
     c->s52 = *std::max_element(primes.begin(), primes.end()) < kS52PrimeLimit;
     {
         int fam = 0;
-        for (uint64_t q : primes) fam |= (1 << bf_mode_of(q)) | (1 << fwd_mode_of(q));
+        for (uint64_t q : primes) fam |= 1 << bf_mode_of(q);
         c->ntt_families = (fam & ~kFamSmall) == 0 ? kFamSmall : (fam & ~kFamLarge) == 0 ? kFamLarge : kFamAll;
     }
     // per-prime constants and twiddles
@@ -142,34 +167,13 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
         }
         p.n_inv = host::invmod(n, q);
         p.n_inv_shoup = host::shoup_of(p.n_inv, q);
+        p.qinv = 1.0 / (double)q;
         c->h_pc.push_back(p);
         push4(sc_plain, p.n_inv, psi_half_inv[i], q);
     }
     c->pc = upload(c->h_pc);
     c->tw = upload(tw);
-    {
-        // for the FP64 butterflies of the primes below kF64CentreLimit (other primes never read it):
-        // the forward and inverse w / q rounded to the nearest double (w and q are exact doubles
-        // below 2^53), then the forward w itself as a double.  The forward twiddles of the primes
-        // at or above kF64GrowLimit (the centred family) are kept within q/2 of zero (w - q for
-        // w > q/2), so that |w / q| <= 1/2.
-        std::vector<double> twq((size_t)QP * 3 * n, 0.0);
-        for (uint32_t i = 0; i < QP; i++) {
-            if (primes[i] >= kF64CentreLimit) continue;
-            const uint64_t q = primes[i];
-            const double qd = (double)q;
-            const bool centre = q >= kF64GrowLimit;
-            const uint64_t *t = tw.data() + (size_t)i * 4 * n;
-            double *d = twq.data() + (size_t)i * 3 * n;
-            for (uint32_t k = 0; k < n; k++) {
-                const double w = centre && t[k] > q / 2 ? (double)t[k] - qd : (double)t[k];
-                d[k] = w / qd;
-                d[n + k] = (double)t[2 * n + k] / qd;
-                d[2 * n + k] = w;
-            }
-        }
-        c->twq = upload(twq);
-    }
+    c->twd = upload(log_n == 16 ? fp64_twiddles<4>(primes, tw) : fp64_twiddles<3>(primes, tw));
     c->inv_scale_plain = upload(sc_plain);
 
     // rescale: row L-1 holds q_{L-1}^-1 mod q_j
@@ -395,7 +399,7 @@ int shm_ntt_forward(const shm_context *ctx, uint64_t *data, uint32_t n_polys, ui
         auto &c = ctx_of(ctx);
         check_level(c, L);
         set_device(c);
-        shm::ntt_forward(c, data, n_polys * L, L, shm::q_map(L), S(stream));
+        shm::ntt_forward(c, data, shm::rows_of(c, n_polys, L, L), S(stream));
     });
 }
 
@@ -404,7 +408,7 @@ int shm_ntt_inverse(const shm_context *ctx, uint64_t *data, uint32_t n_polys, ui
         auto &c = ctx_of(ctx);
         check_level(c, L);
         set_device(c);
-        shm::ntt_inverse(c, data, n_polys * L, L, shm::q_map(L), nullptr, S(stream));
+        shm::ntt_inverse(c, data, shm::rows_of(c, n_polys, L, L), nullptr, S(stream));
     });
 }
 
@@ -794,7 +798,7 @@ int shm_ntt_forward_ext(const shm_context *ctx, uint64_t *data, uint32_t n_polys
         check_ext(c, L);
         set_device(c);
         const uint32_t LP = L + c.np;
-        shm::ntt_forward(c, data, n_polys * LP, LP, shm::ext_map(L, c), S(stream));
+        shm::ntt_forward(c, data, shm::rows_of(c, n_polys, LP, L), S(stream));
     });
 }
 

@@ -77,7 +77,7 @@ struct Context {
     std::vector<PrimeConst> h_pc;       // host copy
     PrimeConst *pc = nullptr;           // [QP]
     uint64_t *tw = nullptr;             // [QP][4][N]
-    double *twq = nullptr;              // [QP][3][N]: the forward and inverse twiddles over q, and the forward twiddles, as doubles
+    double *twd = nullptr;              // [QP][2][TwTab::DIR]: the FP64 butterflies' twiddles (ntt.cuh), forward and inverse
     uint64_t *inv_scale_plain = nullptr;  // [QP][4]: N^-1 for a plain INTT, indexed by prime
     uint64_t *moddown_scale = nullptr;  // [np][4]: N^-1 * phat_k^-1
     uint64_t *moddown_conv = nullptr;   // [nq][np]: phat_k mod q_j
@@ -107,15 +107,23 @@ struct Context {
 Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uint32_t nq, uint32_t np, int device);
 
 // ---------------- launchers (all asynchronous on `st`) ----------------
-// NTT of `rows` limbs of N words; limb r uses prime map.prime[r % slots] (255 = skip).
-void ntt_forward(const Context &c, uint64_t *data, uint32_t rows, uint32_t slots, const LimbMap &map,
-                 cudaStream_t st);
-// Inverse NTT; `scale` is [slots - scale_base][4] (c, c', c*psi^-(N/2), shoup), or nullptr
-// for the plain N^-1 of each limb's prime.
-void ntt_inverse(const Context &c, uint64_t *data, uint32_t rows, uint32_t slots, const LimbMap &map,
-                 const uint64_t *scale, cudaStream_t st, uint32_t scale_base = 0);
+// rows of `slots` limbs each: limb j under prime j for j < lq, else under the special prime nq + j - lq
+NttRows rows_of(const Context &c, uint32_t polys, uint32_t slots, uint32_t lq);
+// the special-prime limbs (slots L .. L + np - 1) of polynomials over QlP
+inline NttRows special_rows(const Context &c, uint32_t polys, uint32_t L) {
+    NttRows r = rows_of(c, polys, L + c.np, L);
+    r.first = L;
+    r.count = c.np;
+    return r;
+}
+// in-place NTT of the rows of `data`
+void ntt_forward(const Context &c, uint64_t *data, const NttRows &rw, cudaStream_t st);
+// Inverse NTT of the rows into `data`, read from `src` (polynomials src_stride words apart) when given,
+// else in place; `scale` is [rw.count][4] (c, c', c*psi^-(N/2), shoup), or nullptr for the plain
+// N^-1 of each limb's prime.
+void ntt_inverse(const Context &c, uint64_t *data, const NttRows &rw, const uint64_t *scale, cudaStream_t st,
+                 const uint64_t *src = nullptr, size_t src_stride = 0);
 
-LimbMap q_map(uint32_t L);
 // forward NTT of the rescale's spread limbs fused with the spread and the combine (RescaleIO);
 // t: [n_polys][L-1][N] scratch between the two phases
 void ntt_forward_rescale(const Context &c, const RescaleIO &io, uint64_t *t, uint32_t n_polys, uint32_t L,
@@ -123,9 +131,9 @@ void ntt_forward_rescale(const Context &c, const RescaleIO &io, uint64_t *t, uin
 // ModDown's conversion, forward NTT and combine in one launch pair (ModDownIO); delta:
 // [n_polys][L][N] scratch between the two phases
 // ModUp's base conversion, forward NTT and the digit copies in one launch pair (ModUpIO): up
-// [n_cts][beta][LP][N] with map = the prime of every converted row, 255 on the digits' own rows
+// [n_cts][beta][LP][N]
 void ntt_forward_modup(const Context &c, const ModUpIO &mu, uint64_t *up, uint32_t n_cts, uint32_t beta,
-                       const LimbMap &map, cudaStream_t st);
+                       cudaStream_t st);
 void ntt_forward_moddown(const Context &c, const ModDownIO &md, uint64_t *delta, uint32_t n_polys, uint32_t L,
                          cudaStream_t st);
 
@@ -243,7 +251,6 @@ int ctpt_tc_error(void *ws, cudaStream_t st);
 size_t ctpt_ws_words(const Context &c, uint32_t n_in, uint32_t n_out, uint32_t L);
 // ---- the extended basis QlP: a polynomial at level L has L + np limbs, the Q limbs 0..L-1
 // (primes q_0 .. q_{L-1}) then the special primes p_0 .. p_{np-1} (shared.cu)
-LimbMap ext_map(uint32_t L, const Context &c);
 void extend(const Context &c, const uint64_t *in, uint64_t *out, uint32_t n_polys, uint32_t L, cudaStream_t st);
 void add_ext(const Context &c, const uint64_t *a, const uint64_t *b, uint64_t *out, uint32_t n_polys, uint32_t L,
              cudaStream_t st);

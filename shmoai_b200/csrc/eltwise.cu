@@ -118,13 +118,6 @@ __global__ void galois_kernel(const uint64_t *__restrict__ in, uint64_t *__restr
     out[(row << log_n) + k] = in[(row << log_n) + galois_index(k, elt, log_n)];
 }
 
-// copy the last limb of every polynomial into a contiguous buffer
-__global__ void gather_last(const uint64_t *__restrict__ in, uint64_t *__restrict__ last, uint32_t L, uint32_t log_n) {
-    const uint32_t poly = blockIdx.y;
-    const uint32_t k = blockIdx.x * kEwThreads + threadIdx.x;
-    last[((size_t)poly << log_n) + k] = in[(((size_t)poly * L + L - 1) << log_n) + k];
-}
-
 }  // namespace
 
 void elementwise(const Context &c, EwOp op, const uint64_t *a, const uint64_t *b, uint64_t *out, uint32_t n_polys,
@@ -192,13 +185,10 @@ void rescale(const Context &c, const uint64_t *in, uint64_t *out, uint32_t n_pol
     if (L < 2) throw std::invalid_argument("rescale needs at least two limbs");
     if (n_polys == 0) return;  // nothing to do; a grid with y = 0 would be an invalid launch
     uint64_t *last = ws, *t = ws + ((size_t)n_polys << c.log_n);
-    const uint32_t chunks = c.n / kEwThreads;
-    SHM_LAUNCHED(1); gather_last<<<dim3(chunks, n_polys), kEwThreads, 0, st>>>(in, last, L, c.log_n);
-    SHM_CUDA(cudaGetLastError());
-    LimbMap m;
-    for (int i = 0; i < 512; i++) m.prime[i] = 255;
-    m.prime[0] = (uint8_t)(L - 1);
-    ntt_inverse(c, last, n_polys, 1, m, nullptr, st);
+    // the last limbs in coefficient form: one row per polynomial, read from limb L - 1 of the input
+    NttRows rw = rows_of(c, n_polys, 1, 0);
+    rw.nq = L - 1;
+    ntt_inverse(c, last, rw, nullptr, st, in + ((size_t)(L - 1) << c.log_n), (size_t)L << c.log_n);
     // t_j = c_last mod q_j, its NTT and out_j = (c_j - t_j) q_last^-1 in one NTT launch pair
     RescaleIO io;
     io.last = last;

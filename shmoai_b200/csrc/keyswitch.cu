@@ -169,10 +169,10 @@ void relin_rescale(const Context &c, const uint64_t *ct3, uint32_t n_cts, uint32
     // ModDown by S = q_{L-1} P: INTT of rows L-1 .. LP-1 scaled by (S / s_k)^-1, the overflow
     // count of the conversion, exact conversion to the L - 1 remaining primes, NTT,
     // (y_j - conv_j) S^-1 = floor(y / S)
-    LimbMap mp;
-    for (uint32_t r = 0; r < 512; r++)
-        mp.prime[r] = r == L - 1 ? (uint8_t)(L - 1) : (r >= L && r < LP) ? (uint8_t)(c.nq + (r - L)) : 255;
-    ntt_inverse(c, acc, n_cts * 2 * LP, LP, mp, ks.rr_scale, st, L - 1);
+    NttRows rw = rows_of(c, n_cts * 2, LP, L);
+    rw.first = L - 1;
+    rw.count = np + 1;
+    ntt_inverse(c, acc, rw, ks.rr_scale, st);
     uint8_t *vrow = reinterpret_cast<uint8_t *>(x);  // x is free after the ModUp: [n_cts][2][N] bytes
     SHM_LAUNCHED(1);
     overflow_count_kernel<<<dim3(c.n / kThreads, n_cts * 2), kThreads, 0, st>>>(acc, vrow, LP, L - 1, np + 1,
@@ -223,9 +223,7 @@ void keyswitch(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n_
     // 4. inner product with the key digits
     launch_ip(c, n_cts, L, up, key, acc, nullptr, st);
     // 5. ModDown: INTT of the P limbs (scaled by phat_k^-1), convert to Ql, NTT, combine
-    LimbMap mp;
-    for (uint32_t s = 0; s < 512; s++) mp.prime[s] = (s >= L && s < LP) ? (uint8_t)(c.nq + (s - L)) : 255;
-    ntt_inverse(c, acc, n_cts * 2 * LP, LP, mp, c.moddown_scale, st, L);
+    ntt_inverse(c, acc, special_rows(c, n_cts * 2, L), c.moddown_scale, st);
     ntt_forward_moddown(c, moddown_io(c, acc, o), delta, n_cts * 2, L, st);
 }
 
@@ -235,20 +233,8 @@ void modup_into(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n
                 uint64_t *up, cudaStream_t st) {
     const uint32_t np = c.np, beta = (L + np - 1) / np, LP = L + np;
     if (np > kMaxAlpha || beta > kMaxBeta || LP > 64) throw std::invalid_argument("key-switching shape too large");
-    const size_t n = c.n, ln = (size_t)L * n;
     const LevelKS &ks = c.ks[L];
-    SHM_CUDA(cudaMemcpy2DAsync(x, ln * 8, d, d_stride * 8, ln * 8, n_cts, cudaMemcpyDeviceToDevice, st));
-    ntt_inverse(c, x, n_cts * L, L, q_map(L), ks.modup_scale, st);
-    LimbMap m;
-    for (uint32_t s = 0; s < 512; s++) {
-        if (s >= beta * LP) {
-            m.prime[s] = 255;
-            continue;
-        }
-        uint32_t b = s / LP, j = s % LP;
-        bool own = j >= b * np && j < std::min((b + 1) * np, L);
-        m.prime[s] = own ? 255 : (uint8_t)(j < L ? j : c.nq + (j - L));
-    }
+    ntt_inverse(c, x, rows_of(c, n_cts, L, L), ks.modup_scale, st, d, d_stride);
     // the conversion is computed in the forward NTT's load and the digits' own rows are copied by
     // the same launch: the converted limbs never go through HBM in coefficient form
     ModUpIO mu;
@@ -260,7 +246,7 @@ void modup_into(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n
     mu.np = np;
     mu.LP = LP;
     mu.s52 = c.s52 ? 1 : 0;
-    ntt_forward_modup(c, mu, up, n_cts, beta, m, st);
+    ntt_forward_modup(c, mu, up, n_cts, beta, st);
 }
 
 size_t hoisted_ws_words(const Context &c, uint32_t n_cts, uint32_t L) {
@@ -286,14 +272,11 @@ void apply_galois_hoisted(const Context &c, const uint64_t *ct, uint32_t n_cts, 
 
     // ModUp once (identical to keyswitch steps 1-3)
     modup_into(c, d, 2 * ln, n_cts, L, x, up, st);
-    LimbMap mp;
-    for (uint32_t s = 0; s < 512; s++) mp.prime[s] = (s >= L && s < LP) ? (uint8_t)(c.nq + (s - L)) : 255;
-
     // per element: permuted inner product, ModDown, combine with sigma(c0)
     for (uint32_t e = 0; e < n_elts; e++) {
         const uint32_t *perm = const_cast<Context &>(c).perm(elts[e]);
         launch_ip(c, n_cts, L, up, keys[e], acc, perm, st);
-        ntt_inverse(c, acc, n_cts * 2 * LP, LP, mp, c.moddown_scale, st, L);
+        ntt_inverse(c, acc, special_rows(c, n_cts * 2, L), c.moddown_scale, st);
         KsOutput o{outs[e], outs[e] + ln, ct, nullptr, 2 * ln, perm};
         ntt_forward_moddown(c, moddown_io(c, acc, o), delta, n_cts * 2, L, st);
     }

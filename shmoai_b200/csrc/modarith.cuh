@@ -20,6 +20,7 @@ struct PrimeConst {
     uint32_t red_m;  // floor(2^(32+s) / q), s = max(0, k - 25): the multiplier of reduce_small
     uint64_t n_inv;        // N^-1 mod q
     uint64_t n_inv_shoup;  // Shoup companion of n_inv
+    double qinv;           // 1 / q rounded (the FP64 paths; primes below 2^51)
 };
 
 __device__ __forceinline__ uint64_t mulhi64(uint64_t a, uint64_t b) { return __umul64hi(a, b); }

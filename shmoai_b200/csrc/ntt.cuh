@@ -13,7 +13,7 @@
 // one shared-memory exchange in between.  Global loads and stores move S consecutive words
 // per column row / per block segment (128 bytes at S = 16).  Values between the two
 // phases are lazy: below 36q (grow butterflies, q < 2^57), in [0, 4q) (Harvey), or signed
-// doubles below 7q in magnitude (the forward's FP64 butterflies, q < 2^52 / 36).
+// doubles (the FP64 butterflies, q < 2^51).
 //
 // The inverse's last stage folds a per-limb scale c (N^-1, or N^-1 times the
 // ModUp digit factor) into both outputs: (X+Y)*c and (X-Y)*psi^-(N/2)*c.
@@ -32,9 +32,23 @@ struct NttVariant {
 constexpr NttVariant kNttVariants[] = {{16, 4}, {16, 3}, {8, 8}, {8, 6}};
 constexpr int kNttVariantCount = 4;
 
-struct LimbMap {
-    uint8_t prime[512];  // limb slot within a polynomial -> prime index; 255 = leave untouched
+// The rows a launch transforms: slots [first, first + count) of each of `polys` polynomials of
+// `slots` limbs.  Slot s stands at position j = s % lp of its digit s / lp (lp = slots: one digit)
+// and uses prime j below lq, else the special prime nq + j - lq.  skip > 0 (ModUp): the limbs
+// [d skip, min((d + 1) skip, lq)) of digit d are left alone.
+struct NttRows {
+    uint32_t polys = 0, slots = 0, first = 0, count = 0, lp = 0, lq = 0, nq = 0, skip = 0;
 };
+constexpr uint32_t kNoPrime = 0xffffffffu;
+
+__host__ __device__ __forceinline__ uint32_t row_prime(const NttRows &r, uint32_t slot) {
+    const uint32_t j = slot % r.lp;
+    if (r.skip) {
+        const uint32_t s0 = slot / r.lp * r.skip;
+        if (j >= s0 && j < s0 + r.skip && j < r.lq) return kNoPrime;
+    }
+    return j < r.lq ? j : r.nq + (j - r.lq);
+}
 
 // The rescale's forward NTT (ntt_forward_rescale): rows (poly, j < L-1) are read as
 // last[poly] mod q_j and written as (in[poly][j] - NTT(...)) * q_{L-1}^-1 into out[poly][j]
@@ -71,7 +85,7 @@ struct ModDownIO {
 // outside digit b (limbs [b alpha, min((b+1) alpha, L))) the column kernel reads the base
 // conversion sum_i y_i (qhat_i mod t_j) of the digit's INTT'd, qhat^-1-scaled limbs
 // y = x[ct][b alpha ..] (coefficient form) and the row is transformed; for j inside the digit it
-// copies d[ct][j] (already NTT form) and the block kernel leaves the row alone (map 255).  The
+// copies d[ct][j] (already NTT form) and the block kernel leaves the row alone (NttRows::skip).  The
 // converted digits are never stored in coefficient form.
 struct ModUpIO {
     const uint64_t *x = nullptr;     // [n_cts][L][N]
@@ -89,11 +103,6 @@ struct NttIO {
     ModUpIO mu;
 };
 constexpr int kIoPlain = 0, kIoRescale = 1, kIoModDown = 2, kIoModUp = 3;
-
-// scale constants of the inverse's last stage, per limb slot: c, c', c*psi^-(N/2), (c*psi^-(N/2))'
-struct InvScale {
-    const uint64_t *c;  // [slots][4]
-};
 
 __device__ __forceinline__ void ct_bf(uint64_t &x, uint64_t &y, uint64_t w, uint64_t ws, uint64_t q) {
     uint64_t q2 = 2 * q;
@@ -116,90 +125,85 @@ __device__ __forceinline__ void ct_bf_grow(uint64_t &x, uint64_t &y, uint64_t w,
     y = a - t + 4 * q;
 }
 
-// Primes below kF64GrowLimit take the twiddle product's quotient from the FP64 pipe instead of the
-// integer multipliers (the quotient estimate of Shoup's NTL MulMod, with the product's remainder
-// formed by the 64-bit low products): with wq = w / q rounded to the nearest double and y < 2^52,
-// y is exact as a double (its bits under the exponent of 2^52, minus 2^52), and
-// Q = round(y wq) comes from the mantissa of fma(y, wq, 2^52).  |Q - y w / q| <= 1/2 + y 2^-54 < 3/4,
-// so Q is floor(y w / q) or one more and r = y w - Q q lies in [-q, q) (as a wrapped 64-bit value);
-// the inverse's butterflies add q to it.  The integer pipe keeps the two low products only.
+// ---- FP64 butterflies (primes below 2^51)
+//
+// Both directions of the transform run on the FP64 pipe for primes below kF64CentreLimit, on values
+// held as doubles (signed exact integers, in the uint64_t registers as their bit patterns; the first
+// phase's output keeps that form in memory for the second).  The product of y with a twiddle w, kept
+// within q/2 of zero, is t = y w - Q q with Q = round(hi / q): hi = y w rounded, lo = y w - hi exactly
+// (an fma), Q from fma(hi, qinv, 1.5 2^52), hi - Q q exact by another fma (an integer below 2^53), and
+// t = (hi - Q q) + lo exact: six FP64 operations, no integer multiply and one table word per twiddle.
+// With z = y w / q, |Q - z| <= 1/2 + |z| 2^-52 (the roundings of hi and of qinv = 1 / q), so
+// |t| <= q (1/2 + |y| 2^-53), for |z| < 2^51 (the rounding through 1.5 2^52 is then exact).
+//
+// What bounds it: the FP64 pipe (eight operations per butterfly and, for 51-bit primes, three per
+// centring) and HBM (each phase reads and writes every limb) within 1.5x of each other.  117 x 35
+// limbs at the bootstrapping primes, forward of one batch and inverse of another: 5.56 ms with two
+// table words per forward twiddle and integer Gentleman-Sande butterflies (whose low products kept
+// the integer-multiply pipe busy), 4.06 ms so.
+//
+// kBfF64, q < 2^52 / 36.  Forward: inputs below q, a stage adds less than 0.65 q, values stay below
+// 11 q over all 16 stages with no reduction.  Inverse (x + y, (x - y) w): from inputs below 1.8 q a
+// pass of four stages grows the value at index 0 to at most 29 q < 2^52, the product of any
+// difference stays below 0.9 q; indices 0 .. 3 (0 and 1 of a three-stage pass), which were last
+// multiplied two or more stages before the pass's end, are centred at its end, the others stay
+// below 1.8 q.
+//
+// kBfF64R, q < 2^51 (values below 4 q are exact).  Forward: values within q/2 of zero at the start of
+// a pass, three stages leave them below 1.13 q, 1.91 q and 2.88 q; the multiplicands of the pass's
+// last stage are centred before their products (a multiplicand must stay below 2 q), its outputs
+// stay below 3.51 q, and every value is centred for the next pass.  Inverse: values stay below
+// q + 3 at every stage: a sum of two such values is centred, a sum of two centred values is not.
 constexpr uint64_t kF64GrowLimit = (1ull << 52) / 36;
+constexpr uint64_t kF64CentreLimit = 1ull << 51;
+constexpr double kTwo52 = 4503599627370496.0, kMagic = 6755399441055744.0;  // 2^52, 1.5 2^52
 
-__device__ __forceinline__ uint64_t mulmod_f64_centred(uint64_t y, uint64_t w, double wq, uint64_t q) {
-    const double two52 = 4503599627370496.0;
-    const double yd = __dsub_rn(__longlong_as_double((long long)(0x4330000000000000ull | y)), two52);
-    const uint64_t Q = (uint64_t)__double_as_longlong(__fma_rn(yd, wq, two52)) & 0x000FFFFFFFFFFFFFull;
-    return y * w - Q * q;
-}
+__device__ __forceinline__ double as_dbl(uint64_t x) { return __longlong_as_double((long long)x); }
+__device__ __forceinline__ uint64_t as_bits(double x) { return (uint64_t)__double_as_longlong(x); }
 
-// The forward transform of the primes below kF64GrowLimit runs entirely on the FP64 pipe, on values
-// held as doubles (signed exact integers, stored in the uint64_t registers as their bit patterns;
-// the column phase's output keeps that form in memory for the block phase).  Cooley-Tukey:
-// t = y w - Q q with Q = round(y wq), |Q - y w / q| < 3/4 (|y| < 16q, so |y| 2^-53 < 1/4), hence
-// |t| < q; y w = hi + lo exactly (hi = y w rounded, lo from an fma), hi - Q q is exact by a second
-// fma (an integer below 2^47 in magnitude), and t = (hi - Q q) + lo exactly.  From inputs below q in
-// magnitude, values grow by less than 3q/4 per stage: below 13q < 2^51 after 16 stages.  Eight FP64
-// operations and no integer multiply per butterfly.
-__device__ __forceinline__ void ct_bf_dbl(uint64_t &xb, uint64_t &yb, double w, double wq, double q) {
-    const double magic = 6755399441055744.0;  // 1.5 2^52
-    const double x = __longlong_as_double((long long)xb), y = __longlong_as_double((long long)yb);
-    const double Q = __dsub_rn(__fma_rn(y, wq, magic), magic);
+// y w mod q as a signed value (see above)
+__device__ __forceinline__ double mul_dbl(double y, double w, double q, double qinv) {
     const double hi = __dmul_rn(y, w);
     const double lo = __fma_rn(y, w, -hi);
-    const double t = __dadd_rn(__fma_rn(-Q, q, hi), lo);
-    xb = (uint64_t)__double_as_longlong(__dadd_rn(x, t));
-    yb = (uint64_t)__double_as_longlong(__dsub_rn(x, t));
+    const double Q = __dsub_rn(__fma_rn(hi, qinv, kMagic), kMagic);
+    return __dadd_rn(__fma_rn(-Q, q, hi), lo);
 }
 
-// x < 2^52 as the bit pattern of the double x
-__device__ __forceinline__ uint64_t to_dbl_bits(uint64_t x) {
-    const double two52 = 4503599627370496.0;
-    return (uint64_t)__double_as_longlong(__dsub_rn(__longlong_as_double((long long)(0x4330000000000000ull | x)), two52));
+__device__ __forceinline__ void ct_bf_dbl(uint64_t &xb, uint64_t &yb, double w, double q, double qinv) {
+    const double x = as_dbl(xb), t = mul_dbl(as_dbl(yb), w, q, qinv);
+    xb = as_bits(__dadd_rn(x, t));
+    yb = as_bits(__dsub_rn(x, t));
 }
 
-// Primes in [kF64GrowLimit, 2^51) run the same butterfly on twiddles kept within q/2 of zero
-// (|wq| <= 1/2, |wq - w / q| <= 2^-55), with every value centred (dbl_centre) at the start and
-// after every pass of four stages, and the multiplicands of a pass's fourth stage centred before
-// their products.  |Q - y w / q| <= 1/2 + |y| 2^-55, so from |v| <= q/2 the multiplicands of the
-// first three stages stay below q/2, 1.03q and 1.6q (|y wq| < 2^51: the rounding through
-// 1.5 2^52 is exact), |t| below 0.53q, 0.57q and 0.6q, the fourth stage's below 0.53q, and every
-// value below 2.73q < 2^53: exact; |y w| < 2^102, so |lo| <= 2^48 and hi - Q q stays below 2^52.
-constexpr uint64_t kF64CentreLimit = 1ull << 51;
-
-// v (|v| < 2^52, a signed integer) -> v - round(v / q) q, within q/2 + 1 of zero (exact: an integer
-// below q); qinv = 1 / q rounded
-__device__ __forceinline__ uint64_t dbl_centre(uint64_t vb, double q, double qinv) {
-    const double magic = 6755399441055744.0;
-    const double v = __longlong_as_double((long long)vb);
-    const double Q = __dsub_rn(__fma_rn(v, qinv, magic), magic);
-    return (uint64_t)__double_as_longlong(__fma_rn(-Q, q, v));
+__device__ __forceinline__ void gs_bf_dbl(uint64_t &xb, uint64_t &yb, double w, double q, double qinv) {
+    const double x = as_dbl(xb), y = as_dbl(yb);
+    xb = as_bits(__dadd_rn(x, y));
+    yb = as_bits(mul_dbl(__dsub_rn(x, y), w, q, qinv));
 }
 
-// a centred double (|v| <= q/2 + 1) -> v mod q in [0, q) as an integer
-__device__ __forceinline__ uint64_t dbl_bits_canon(uint64_t vb, double q) {
-    const double two52 = 4503599627370496.0;
-    double v = __longlong_as_double((long long)vb);
-    v = v < 0.0 ? __dadd_rn(v, q) : v;
-    return (uint64_t)__double_as_longlong(__dadd_rn(v, two52)) & 0x000FFFFFFFFFFFFFull;
+// x < 2^52 as the double x
+__device__ __forceinline__ double to_dbl(uint64_t x) { return __dsub_rn(as_dbl(0x4330000000000000ull | x), kTwo52); }
+
+// x in [0, q) as a double within q/2 of zero
+__device__ __forceinline__ double to_dbl_centred(uint64_t x, uint64_t q) {
+    return __dsub_rn(as_dbl(0x4330000000000000ull | x), x > (q >> 1) ? __dadd_rn(kTwo52, (double)q) : kTwo52);
 }
 
-// a double holding a signed integer v (|v| < 2^51) -> v mod q in [0, q): v - round(v / q) q is exact
-// and within q/2 + 1 of zero, one conditional addition of q finishes it
-__device__ __forceinline__ uint64_t dbl_bits_mod(uint64_t vb, double q, double qinv) {
-    const double magic = 6755399441055744.0, two52 = 4503599627370496.0;
-    const double v = __longlong_as_double((long long)vb);
-    const double Q = __dsub_rn(__fma_rn(v, qinv, magic), magic);
-    double r = __fma_rn(-Q, q, v);
-    r = r < 0.0 ? __dadd_rn(r, q) : r;
-    return (uint64_t)__double_as_longlong(__dadd_rn(r, two52)) & 0x000FFFFFFFFFFFFFull;
+// v (|v| < 2^53, a signed integer) -> v - round(v / q) q, within q/2 + 1 of zero, exact
+__device__ __forceinline__ double dbl_centre(double v, double q, double qinv) {
+    const double Q = __dsub_rn(__fma_rn(v, qinv, kMagic), kMagic);
+    return __fma_rn(-Q, q, v);
 }
 
-// Gentleman-Sande butterfly on [0, 4q) with the FP64 quotient: x - y + 4q < 8q < 2^52
-__device__ __forceinline__ void gs_bf_f64(uint64_t &x, uint64_t &y, uint64_t w, double wq, uint64_t q) {
-    const uint64_t q4 = 4 * q;
-    const uint64_t a = x + y, d = x - y + q4;
-    x = csub(a, q4);
-    y = mulmod_f64_centred(d, w, wq, q) + q;
+// |v| < q -> v mod q in [0, q) as an integer (2^52 + q is exact: q < 2^51)
+__device__ __forceinline__ uint64_t dbl_canon(double v, double q) {
+    const double r = __dadd_rn(v, (int)(as_bits(v) >> 32) < 0 ? __dadd_rn(kTwo52, q) : kTwo52);
+    return as_bits(r) & 0x000FFFFFFFFFFFFFull;
+}
+
+// a signed integer |v| < 2^53 -> v mod q in [0, q)
+__device__ __forceinline__ uint64_t dbl_mod(double v, double q, double qinv) {
+    return dbl_canon(dbl_centre(v, q, qinv), q);
 }
 
 __device__ __forceinline__ void gs_bf(uint64_t &x, uint64_t &y, uint64_t w, uint64_t ws, uint64_t q) {
@@ -219,101 +223,159 @@ __device__ __forceinline__ void gs_bf4(uint64_t &x, uint64_t &y, uint64_t w, uin
     y = shoup_lazy4(d, w, ws, q);
 }
 
-// R forward stages on E = 2^R registers.  Stage r of the pass is global stage
-// s0 + r; the twiddle of the pair starting at m is tw[(tb << (s0 + r)) + (g << r) + (m >> (R - r))].
-// MODE kBfHarvey: Harvey butterflies that keep values in [0, 4q) (any prime); kBfGrow: ct_bf_grow
-// (primes below kGrowPrimeLimit); kBfF64: ct_bf_dbl (forward, primes below kF64GrowLimit) on values
-// held as doubles, with the twiddles wd (w as doubles) and wq (w / q as doubles); kBfF64R: the same
-// on centred twiddles, with the last stage's multiplicands centred before their products and
-// every value centred after the pass (forward, primes below kF64CentreLimit).  The inverse's kBfF64 is gs_bf_f64 (integer values,
-// FP64 quotient).
+// The butterfly family of a limb's prime, both directions.  kBfHarvey: values in [0, 4q) forward,
+// [0, 2q) inverse (any prime); kBfGrow: ct_bf_grow / gs_bf4 (below kGrowPrimeLimit).
 constexpr int kBfHarvey = 0, kBfGrow = 1, kBfF64 = 2, kBfF64R = 3;
 
-// the inverse's butterfly family of a limb's prime
 __host__ __device__ __forceinline__ int bf_mode_of(uint64_t q) {
-    return q < kF64GrowLimit ? kBfF64 : q < kGrowPrimeLimit ? kBfGrow : kBfHarvey;
-}
-
-// the forward's butterfly family of a limb's prime
-__host__ __device__ __forceinline__ int fwd_mode_of(uint64_t q) {
     return q < kF64GrowLimit ? kBfF64 : q < kF64CentreLimit ? kBfF64R : q < kGrowPrimeLimit ? kBfGrow : kBfHarvey;
 }
 
-// The families a kernel instantiation carries (a bit per family, forward and inverse together).
-// Every unrolled family adds a full copy of the transform's butterflies to the kernel, so a
-// context's launches use the instantiation with just the families its primes need: kFamSmall
-// (every prime below 2^57: the bootstrapping chains), kFamLarge (none below kF64GrowLimit),
-// kFamAll otherwise.
-constexpr int kFamSmall = (1 << kBfF64) | (1 << kBfF64R) | (1 << kBfGrow),
+// The families a kernel instantiation carries (a bit per family).  Every unrolled family adds a full
+// copy of the transform's butterflies to the kernel, so a context's launches use the instantiation
+// with just the families its primes need: kFamSmall (every prime below 2^51: the bootstrapping
+// chains), kFamLarge (none below kF64GrowLimit), kFamAll otherwise.
+constexpr int kFamSmall = (1 << kBfF64) | (1 << kBfF64R),
               kFamLarge = (1 << kBfF64R) | (1 << kBfGrow) | (1 << kBfHarvey), kFamAll = kFamSmall | kFamLarge;
+__host__ __device__ constexpr bool fam_has(int fam, int mode) { return (fam >> mode) & 1; }
+constexpr bool fam_fp(int fam) { return fam & kFamSmall; }
+constexpr bool fam_int(int fam) { return fam & ((1 << kBfGrow) | (1 << kBfHarvey)); }
 
-template <int R, int MODE = kBfHarvey>
-__device__ __forceinline__ void fwd_pass(uint64_t (&a)[1 << R], const uint64_t *__restrict__ w,
-                                         const uint64_t *__restrict__ ws, const double *__restrict__ wq,
-                                         const double *__restrict__ wd, uint32_t tb, uint32_t s0, uint32_t g,
-                                         uint64_t q) {
-    const double qd = (double)q;
-    const double qinv = MODE == kBfF64R ? __ldg(wq) : 0.0;  // wq[0] = 1 / q (the twiddle at index 0 is 1)
+// ---- FP64 twiddle tables: per prime and direction N / 2^R + N doubles (N = 2^(4R)), within q/2 of zero.
+// The first 2^(3R) entries are the bit-reversed table's (the column phase and the block phase's
+// first pass, whose threads read one entry per block or per column).  The rest are the block
+// phase's second pass, whose threads each need 2^R - 1 entries of their own: stage r of block b,
+// thread g reads entries ((M + b) 2^R + g) 2^r + i, i < 2^r, which lie 2^r words apart for
+// neighbouring threads.  They are stored as slots 2^r + i of a row of 2^R (slot 0 unused), slots
+// in pairs, pairs thread-minor: [b][slot / 2][g][slot % 2], so that a half-warp reads 256 contiguous
+// bytes: 16-byte loads of neighbouring threads instead of 8-byte loads up to 64 bytes apart
+// (the second pass's table loads were 340 of about 570 L1 wavefronts per warp of fwd_blk).
+template <int R>
+struct TwTab {
+    static constexpr uint32_t E = 1u << R, M = 1u << (2 * R), N = 1u << (4 * R), NAT = 1u << (3 * R);
+    static constexpr size_t DIR = (size_t)N + NAT;  // doubles per prime and direction
+    __host__ __device__ static size_t slot(uint32_t b, uint32_t g, uint32_t s) {
+        return NAT + (((size_t)b * (E / 2) + (s >> 1)) * E + g) * 2 + (s & 1);
+    }
+};
+
+// entries (u << r) + i of the natural part
+struct TwNatural {
+    const double *p;
+    uint32_t u;
+    __device__ __forceinline__ double one() const { return __ldg(p + u); }
+    __device__ __forceinline__ double2 pair(int r, int i) const {
+        return __ldg(reinterpret_cast<const double2 *>(p + ((u << r) + i)));
+    }
+};
+
+// the second block pass's slots of one thread (p = table of the prime and direction)
+template <int R>
+struct TwLane {
+    const double2 *p;
+    __device__ __forceinline__ TwLane(const double *t, uint32_t b, uint32_t g)
+        : p(reinterpret_cast<const double2 *>(t + TwTab<R>::slot(b, g, 0))) {}
+    __device__ __forceinline__ double one() const { return __ldg(reinterpret_cast<const double *>(p) + 1); }
+    __device__ __forceinline__ double2 pair(int r, int i) const {
+        return __ldg(p + (size_t)((((1 << r) + i) >> 1) << R));
+    }
+};
+
+// R forward stages on E = 2^R registers; stage r's pair starting at m uses entry m >> (R - r) of the
+// stage's 2^r.  LAST: the block phase's second pass, whose values are reduced by the caller.
+template <int R, bool CENTRED, bool LAST, class TW>
+__device__ __forceinline__ void fwd_pass_dbl(uint64_t (&a)[1 << R], const TW &tw, double q, double qinv) {
+    constexpr int E = 1 << R;
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int half = E >> (r + 1);
+#pragma unroll
+        for (int i = 0; i < (1 << r); i += 2) {
+            double2 w = r == 0 ? make_double2(tw.one(), 0.0) : tw.pair(r, i);
+#pragma unroll
+            for (int k = 0; k < (r == 0 ? 1 : 2); k++) {
+#pragma unroll
+                for (int h = 0; h < half; h++) {
+                    const int m = (i + k) * 2 * half + h;
+                    if (CENTRED && r == R - 1) a[m + half] = as_bits(dbl_centre(as_dbl(a[m + half]), q, qinv));
+                    ct_bf_dbl(a[m], a[m + half], k ? w.y : w.x, q, qinv);
+                }
+            }
+        }
+    }
+    if (CENTRED && !LAST) {
+#pragma unroll
+        for (int m = 0; m < E; m++) a[m] = as_bits(dbl_centre(as_dbl(a[m]), q, qinv));
+    }
+}
+
+// R inverse stages; skip_stage0 leaves the last one (the transform's final stage) to the caller.
+// Which values are centred is decided at compile time (see the bounds above).
+template <int R, bool CENTRED, bool SKIP0, class TW>
+__device__ __forceinline__ void inv_pass_dbl(uint64_t (&a)[1 << R], const TW &tw, double q, double qinv) {
+    constexpr int E = 1 << R;
+    bool small[E];  // within q/2 + 1 of zero
+#pragma unroll
+    for (int m = 0; m < E; m++) small[m] = false;
+#pragma unroll
+    for (int r = R - 1; r >= (SKIP0 ? 1 : 0); r--) {
+        const int half = E >> (r + 1);
+#pragma unroll
+        for (int i = 0; i < (1 << r); i += 2) {
+            double2 w = r == 0 ? make_double2(tw.one(), 0.0) : tw.pair(r, i);
+#pragma unroll
+            for (int k = 0; k < (r == 0 ? 1 : 2); k++) {
+#pragma unroll
+                for (int h = 0; h < half; h++) {
+                    const int m = (i + k) * 2 * half + h;
+                    gs_bf_dbl(a[m], a[m + half], k ? w.y : w.x, q, qinv);
+                    if (CENTRED) {
+                        const bool c = !small[m];
+                        if (c) a[m] = as_bits(dbl_centre(as_dbl(a[m]), q, qinv));
+                        small[m] = c;
+                        small[m + half] = false;
+                    }
+                }
+            }
+        }
+    }
+    if (!CENTRED && !SKIP0) {
+#pragma unroll
+        for (int m = 0; m < E / 4; m++) a[m] = as_bits(dbl_centre(as_dbl(a[m]), q, qinv));
+    }
+}
+
+// the integer families: stage r of the pass is global stage s0 + r, the twiddle of the pair starting
+// at m is entry (u << r) + (m >> (R - r)), u = (tb << s0) + g
+template <int R, int MODE>
+__device__ __forceinline__ void fwd_pass_int(uint64_t (&a)[1 << R], const uint64_t *__restrict__ w,
+                                             const uint64_t *__restrict__ ws, uint32_t u, uint64_t q) {
 #pragma unroll
     for (int r = 0; r < R; r++) {
         const int half = (1 << R) >> (r + 1);
-        const uint32_t base = (tb << (s0 + r)) + (g << r);
 #pragma unroll
         for (int m = 0; m < (1 << R); m++) {
             if (m & half) continue;
-            uint32_t idx = base + (m >> (R - r));
-            if (MODE == kBfF64)
-                ct_bf_dbl(a[m], a[m + half], __ldg(wd + idx), __ldg(wq + idx), qd);
-            else if (MODE == kBfF64R) {
-                if (r == R - 1) a[m + half] = dbl_centre(a[m + half], qd, qinv);
-                ct_bf_dbl(a[m], a[m + half], __ldg(wd + idx), __ldg(wq + idx), qd);
-            }
-            else if (MODE == kBfGrow)
+            const uint32_t idx = (u << r) + (m >> (R - r));
+            if (MODE == kBfGrow)
                 ct_bf_grow(a[m], a[m + half], __ldg(w + idx), __ldg(ws + idx), q);
             else
                 ct_bf(a[m], a[m + half], __ldg(w + idx), __ldg(ws + idx), q);
         }
     }
-    if (MODE == kBfF64R) {
-#pragma unroll
-        for (int m = 0; m < (1 << R); m++) a[m] = dbl_centre(a[m], qd, qinv);
-    }
 }
 
-// fwd_pass in the butterfly family `mode` (uniform per CTA: one limb), one of the families FAM carries
-template <int R, int FAM>
-__device__ __forceinline__ void fwd_pass_any(int mode, uint64_t (&a)[1 << R], const uint64_t *__restrict__ w,
-                                             const uint64_t *__restrict__ ws, const double *__restrict__ wq,
-                                             const double *__restrict__ wd, uint32_t tb, uint32_t s0, uint32_t g,
-                                             uint64_t q) {
-    if ((FAM & (1 << kBfF64)) && mode == kBfF64)
-        fwd_pass<R, kBfF64>(a, w, ws, wq, wd, tb, s0, g, q);
-    else if ((FAM & (1 << kBfF64R)) && mode == kBfF64R)
-        fwd_pass<R, kBfF64R>(a, w, ws, wq, wd, tb, s0, g, q);
-    else if (!(FAM & (1 << kBfHarvey)) || mode == kBfGrow)
-        fwd_pass<R, kBfGrow>(a, w, ws, wq, wd, tb, s0, g, q);
-    else
-        fwd_pass<R, kBfHarvey>(a, w, ws, wq, wd, tb, s0, g, q);
-}
-
-// MODE kBfGrow: gs_bf4 on [0, 4q) (primes below kGrowPrimeLimit); kBfF64: gs_bf_f64 on [0, 4q);
-// kBfHarvey: gs_bf on [0, 2q)
-template <int R, int MODE = kBfHarvey>
-__device__ __forceinline__ void inv_pass(uint64_t (&a)[1 << R], const uint64_t *__restrict__ w,
-                                         const uint64_t *__restrict__ ws, const double *__restrict__ wq, uint32_t tb,
-                                         uint32_t s0, uint32_t g, uint64_t q, int skip_stage0) {
+template <int R, int MODE, bool SKIP0>
+__device__ __forceinline__ void inv_pass_int(uint64_t (&a)[1 << R], const uint64_t *__restrict__ w,
+                                             const uint64_t *__restrict__ ws, uint32_t u, uint64_t q) {
 #pragma unroll
-    for (int r = R - 1; r >= 0; r--) {
-        if (r == 0 && skip_stage0) break;
+    for (int r = R - 1; r >= (SKIP0 ? 1 : 0); r--) {
         const int half = (1 << R) >> (r + 1);
-        const uint32_t base = (tb << (s0 + r)) + (g << r);
 #pragma unroll
         for (int m = 0; m < (1 << R); m++) {
             if (m & half) continue;
-            uint32_t idx = base + (m >> (R - r));
-            if (MODE == kBfF64)
-                gs_bf_f64(a[m], a[m + half], __ldg(w + idx), __ldg(wq + idx), q);
-            else if (MODE == kBfGrow)
+            const uint32_t idx = (u << r) + (m >> (R - r));
+            if (MODE == kBfGrow)
                 gs_bf4(a[m], a[m + half], __ldg(w + idx), __ldg(ws + idx), q);
             else
                 gs_bf(a[m], a[m + half], __ldg(w + idx), __ldg(ws + idx), q);
@@ -321,16 +383,33 @@ __device__ __forceinline__ void inv_pass(uint64_t (&a)[1 << R], const uint64_t *
     }
 }
 
-template <int R, int FAM>
-__device__ __forceinline__ void inv_pass_any(int mode, uint64_t (&a)[1 << R], const uint64_t *__restrict__ w,
-                                             const uint64_t *__restrict__ ws, const double *__restrict__ wq,
-                                             uint32_t tb, uint32_t s0, uint32_t g, uint64_t q, int skip_stage0) {
-    if ((FAM & (1 << kBfF64)) && mode == kBfF64)
-        inv_pass<R, kBfF64>(a, w, ws, wq, tb, s0, g, q, skip_stage0);
-    else if (!(FAM & (1 << kBfHarvey)) || mode == kBfGrow)
-        inv_pass<R, kBfGrow>(a, w, ws, wq, tb, s0, g, q, skip_stage0);
-    else
-        inv_pass<R, kBfHarvey>(a, w, ws, wq, tb, s0, g, q, skip_stage0);
+// a pass in the family `mode` (uniform per CTA: one limb), one of the families FAM carries
+template <int R, int FAM, bool LAST, class TW>
+__device__ __forceinline__ void fwd_pass(int mode, uint64_t (&a)[1 << R], const TW &tw, double qd, double qinv,
+                                         const uint64_t *__restrict__ w, const uint64_t *__restrict__ ws, uint32_t u,
+                                         uint64_t q) {
+    if (fam_has(FAM, kBfF64) && mode == kBfF64)
+        fwd_pass_dbl<R, false, LAST>(a, tw, qd, qinv);
+    else if (fam_has(FAM, kBfF64R) && (FAM == kFamSmall || mode == kBfF64R))
+        fwd_pass_dbl<R, true, LAST>(a, tw, qd, qinv);
+    else if (fam_has(FAM, kBfGrow) && mode == kBfGrow)
+        fwd_pass_int<R, kBfGrow>(a, w, ws, u, q);
+    else if (fam_has(FAM, kBfHarvey))
+        fwd_pass_int<R, kBfHarvey>(a, w, ws, u, q);
+}
+
+template <int R, int FAM, bool SKIP0, class TW>
+__device__ __forceinline__ void inv_pass(int mode, uint64_t (&a)[1 << R], const TW &tw, double qd, double qinv,
+                                         const uint64_t *__restrict__ w, const uint64_t *__restrict__ ws, uint32_t u,
+                                         uint64_t q) {
+    if (fam_has(FAM, kBfF64) && mode == kBfF64)
+        inv_pass_dbl<R, false, SKIP0>(a, tw, qd, qinv);
+    else if (fam_has(FAM, kBfF64R) && (FAM == kFamSmall || mode == kBfF64R))
+        inv_pass_dbl<R, true, SKIP0>(a, tw, qd, qinv);
+    else if (fam_has(FAM, kBfGrow) && mode == kBfGrow)
+        inv_pass_int<R, kBfGrow, SKIP0>(a, w, ws, u, q);
+    else if (fam_has(FAM, kBfHarvey))
+        inv_pass_int<R, kBfHarvey, SKIP0>(a, w, ws, u, q);
 }
 
 }  // namespace shm

@@ -1,0 +1,8 @@
+#include "ntt_kernels.cuh"
+
+namespace shm {
+
+template void launch_fwd<4, kFamSmall>(const Context &, int, uint64_t *, const NttRows &, cudaStream_t, const NttIO &);
+template void launch_inv<4, kFamSmall>(const Context &, const InvArgs &, const NttRows &, cudaStream_t);
+
+}  // namespace shm

@@ -201,11 +201,9 @@ void check_shape(const Context &c, uint32_t L, uint32_t beta, uint32_t H) {
 // inner products, ModDown and combine for one target; acc/delta are workspace
 void apply_target(const Context &c, const uint64_t *up, uint32_t n_cts, uint32_t L, uint32_t beta, uint32_t H,
                   const Target &t, uint64_t *acc, uint64_t *delta, cudaStream_t st) {
-    const uint32_t np = c.np, LP = L + np;
+    const uint32_t np = c.np;
     ip_multi(c, up, t.key, acc, n_cts, L, beta, H, t.perm, st);
-    LimbMap mp;
-    for (uint32_t s = 0; s < 512; s++) mp.prime[s] = (s >= L && s < LP) ? (uint8_t)(c.nq + (s - L)) : 255;
-    ntt_inverse(c, acc, n_cts * H * LP, LP, mp, c.moddown_scale, st, L);
+    ntt_inverse(c, acc, special_rows(c, n_cts * H, L), c.moddown_scale, st);
     // conversion of the special-prime limbs, NTT and (acc - delta) P^-1 + sigma(add) fused
     ModDownIO md;
     md.acc = acc;
@@ -265,15 +263,12 @@ void fmt_forward(const Context &c, const uint64_t *cts, uint32_t n_groups, uint3
     uint64_t *delta = acc + (size_t)n_groups * H * LP * N;
     ExtConsts e = ext_consts(const_cast<Context &>(c), L);
     // y = INTT(a_j) * qhat^-1 ; the Ql rows of ext keep a_j in NTT form
-    SHM_CUDA(cudaMemcpy2DAsync(y, ln * 8, cts + ln, 2 * ln * 8, ln * 8, m, cudaMemcpyDeviceToDevice, st));
-    ntt_inverse(c, y, m * L, L, q_map(L), e.scale, st);
+    ntt_inverse(c, y, rows_of(c, m, L, L), e.scale, st, cts + ln, 2 * ln);
     SHM_CUDA(cudaMemcpy2DAsync(ext, LP * N * 8, cts + ln, 2 * ln * 8, ln * 8, m, cudaMemcpyDeviceToDevice, st));
     SHM_LAUNCHED(1);
     exact_ext_kernel<<<dim3(N / kT, m), kT, 0, st>>>(y, ext, e.tab, e.qd, L, c.np, c.nq, c.log_n, c.pc);
     SHM_CUDA(cudaGetLastError());
-    LimbMap mp;
-    for (uint32_t s = 0; s < 512; s++) mp.prime[s] = (s >= L && s < LP) ? (uint8_t)(c.nq + (s - L)) : 255;
-    ntt_forward(c, ext, m * LP, LP, mp, st);
+    ntt_forward(c, ext, special_rows(c, m, L), st);
     // digits = the n members of a group: ext is [G][n][LP][N]
     Target t{key, nullptr, out, (size_t)H * ln, ln, cts, (size_t)n * 2 * ln, 2 * ln, n};
     apply_target(c, ext, n_groups, L, n, H, t, acc, delta, st);
@@ -350,10 +345,7 @@ __global__ void combine_ext_kernel(const uint64_t *__restrict__ acc, uint64_t *_
 // inverse NTT) into out [n_polys][L][N]; delta: [n_polys][L][N] scratch
 void moddown_rows(const Context &c, uint64_t *ext, uint64_t *out, uint32_t n_polys, uint32_t L, uint64_t *delta,
                   cudaStream_t st) {
-    const uint32_t LP = L + c.np;
-    LimbMap mp;
-    for (uint32_t s = 0; s < 512; s++) mp.prime[s] = (s >= L && s < LP) ? (uint8_t)(c.nq + (s - L)) : 255;
-    ntt_inverse(c, ext, n_polys * LP, LP, mp, c.moddown_scale, st, L);
+    ntt_inverse(c, ext, special_rows(c, n_polys, L), c.moddown_scale, st);
     ModDownIO md;
     md.acc = ext;
     md.conv = c.moddown_conv;
@@ -367,12 +359,6 @@ void moddown_rows(const Context &c, uint64_t *ext, uint64_t *out, uint32_t n_pol
 }
 
 }  // namespace
-
-LimbMap ext_map(uint32_t L, const Context &c) {
-    LimbMap m;
-    for (uint32_t s = 0; s < 512; s++) m.prime[s] = s < L ? (uint8_t)s : (s < L + c.np ? (uint8_t)(c.nq + (s - L)) : 255);
-    return m;
-}
 
 void extend(const Context &c, const uint64_t *in, uint64_t *out, uint32_t n_polys, uint32_t L, cudaStream_t st) {
     if (!n_polys) return;

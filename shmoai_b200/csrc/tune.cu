@@ -74,8 +74,8 @@ uint32_t tune_ntt_tile(Context &c, uint32_t rows, std::vector<float> &ms) {
     for (int v = 0; v < kNttVariantCount; v++) {
         c.ntt_variant = v;
         ms.push_back(time_ms(s.st, 5, [&] {
-            ntt_forward(c, x, polys * L, L, q_map(L), s.st);
-            ntt_inverse(c, x, polys * L, L, q_map(L), nullptr, s.st);
+            ntt_forward(c, x, rows_of(c, polys, L, L), s.st);
+            ntt_inverse(c, x, rows_of(c, polys, L, L), nullptr, s.st);
         }));
     }
     c.ntt_variant = (int)argmin(ms);
