@@ -38,15 +38,16 @@ Context::~Context() {
     cudaSetDevice(device);
     release_encode_tables(*this);
     for (void *p : {(void *)pc, (void *)tw, (void *)twd, (void *)inv_scale_plain, (void *)moddown_scale, (void *)moddown_conv,
-                    (void *)p_inv, (void *)p_mod, (void *)rescale_inv, arena})
+                    (void *)moddown_bytes, (void *)p_inv, (void *)p_mod, (void *)rescale_inv, arena})
         if (p) cudaFree(p);
     for (auto &l : ks)
         for (void *p : {(void *)l.modup_scale, (void *)l.modup_conv, (void *)l.rr_scale, (void *)l.rr_conv,
-                        (void *)l.rr_sinv, (void *)l.rr_vs, (void *)l.rr_inv_s})
+                        (void *)l.rr_sinv, (void *)l.rr_vs, (void *)l.rr_inv_s, (void *)l.modup_bytes, (void *)l.rr_bytes})
             if (p) cudaFree(p);
     for (auto &kv : galois_perm) cudaFree(kv.second);
     for (auto &kv : ext_consts)
         for (void *p : kv.second) cudaFree(p);
+    if (fault) cudaFreeHost(fault);
     if (pool) {
         cudaDeviceSynchronize();
         cudaMemPoolDestroy(pool);
@@ -126,12 +127,31 @@ std::vector<double> fp64_twiddles(const std::vector<uint64_t> &primes, const std
     return out;
 }
 
+// Row j's block of ConvIO::bytes: slot i's constant c[i] (below q) times 2^(8b) mod q, cut into bytes
+void push_conv_bytes(std::vector<uint8_t> &out, const std::vector<uint64_t> &c, uint64_t q) {
+    const size_t base = out.size();
+    out.resize(base + 512, 0);
+    for (uint32_t i = 0; i < c.size(); i++) {
+        uint64_t v = c[i];
+        for (uint32_t b = 0; b < 8; b++, v = host::mulmod(v, 256, q)) {
+            const uint32_t k = 8 * i + b;
+            for (uint32_t o = 0; o < 8; o++) out[base + k / 16 * 128 + o * 16 + k % 16] = (uint8_t)(v >> (8 * o));
+        }
+    }
+}
+
 Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uint32_t nq, uint32_t np, int device) {
     if (log_n != 12 && log_n != 16) throw std::invalid_argument("log_n must be 12 or 16");
     if (nq < 1 || nq + np != primes.size() || nq + np > 250) throw std::invalid_argument("bad prime counts");
     std::unique_ptr<Context> c(new Context);
     c->device = device;
     SHM_CUDA(cudaSetDevice(device));
+    int sms = 0;
+    SHM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    c->sms = (uint32_t)sms;
+    SHM_CUDA(cudaHostAlloc(&c->fault, sizeof(int), cudaHostAllocMapped));
+    *c->fault = 0;
+    SHM_CUDA(cudaHostGetDevicePointer(&c->fault_dev, c->fault, 0));
     c->log_n = log_n;
     c->n = 1u << log_n;
     c->nq = nq;
@@ -214,6 +234,12 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
         }
         c->moddown_scale = upload(mds);
         c->moddown_conv = upload(mdc);
+        if (np <= kConvSlots) {
+            std::vector<uint8_t> by;
+            for (uint32_t j = 0; j < nq; j++)
+                push_conv_bytes(by, {mdc.begin() + (size_t)j * np, mdc.begin() + (size_t)(j + 1) * np}, primes[j]);
+            c->moddown_bytes = upload(by);
+        }
         c->p_inv = upload(pinv);
         c->p_mod = upload(pmod);
         c->h_p_mod = pmod;
@@ -240,6 +266,16 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
             }
             ks.modup_scale = upload(msc);
             ks.modup_conv = upload(conv);
+            if (np <= kConvSlots) {
+                std::vector<uint8_t> by;
+                for (uint32_t b = 0; b < ks.beta; b++) {
+                    for (uint32_t j = 0; j < LP; j++) {
+                        const auto r = conv.begin() + ((size_t)b * LP + j) * np;
+                        push_conv_bytes(by, {r, r + np}, primes[j < L ? j : nq + (j - L)]);
+                    }
+                }
+                ks.modup_bytes = upload(by);
+            }
             if (L < 2) continue;
             // ModDown by S = q_{L-1} P
             std::vector<uint64_t> S{primes[L - 1]};
@@ -270,6 +306,16 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
                 uint64_t Sq = 1;
                 for (uint32_t k = 0; k <= np; k++) Sq = host::mulmod(Sq, S[k] % q, q);
                 for (uint32_t v = 0; v < 16; v++) rvs[(size_t)j * 16 + v] = host::mulmod(v, Sq, q);
+            }
+            if (np + 2 <= kConvSlots) {  // np + 1 limbs and the overflow count, whose constant is -S
+                std::vector<uint8_t> by;
+                for (uint32_t j = 0; j + 1 < L; j++) {
+                    const uint64_t q = primes[j];
+                    std::vector<uint64_t> r(rconv.begin() + (size_t)j * (np + 1), rconv.begin() + (size_t)(j + 1) * (np + 1));
+                    r.push_back(q - rvs[(size_t)j * 16 + 1]);
+                    push_conv_bytes(by, r, q);
+                }
+                ks.rr_bytes = upload(by);
             }
             std::vector<double> rinvs(np + 1);
             for (uint32_t k = 0; k <= np; k++) rinvs[k] = 1.0 / (double)S[k];

@@ -44,6 +44,7 @@ struct LevelKS {
     uint64_t *rr_sinv = nullptr;   // [L - 1][2]: S^-1 mod q_j and its Shoup companion
     uint64_t *rr_vs = nullptr;     // [L - 1][16]: (v S) mod q_j for v < 16 (exact conversion)
     double *rr_inv_s = nullptr;    // [np + 1]: 1 / s_k rounded to double
+    uint8_t *modup_bytes = nullptr, *rr_bytes = nullptr;  // the conversions' constants as ConvIO::bytes
 };
 
 // the slot that an NTT-domain automorphism X -> X^elt moves to slot k (N = 2^log_n):
@@ -68,6 +69,7 @@ __host__ __device__ __forceinline__ uint32_t galois_index(uint32_t k, uint32_t e
 
 struct Context {
     int device = 0;
+    uint32_t sms = 148;                 // multiprocessors of the device
     uint32_t log_n = 0, n = 0, nq = 0, np = 0, dnum = 0;
     std::vector<uint64_t> primes;       // nq + np
     bool s52 = false;                   // every prime below kS52PrimeLimit (Acc<true> kernels)
@@ -81,6 +83,7 @@ struct Context {
     uint64_t *inv_scale_plain = nullptr;  // [QP][4]: N^-1 for a plain INTT, indexed by prime
     uint64_t *moddown_scale = nullptr;  // [np][4]: N^-1 * phat_k^-1
     uint64_t *moddown_conv = nullptr;   // [nq][np]: phat_k mod q_j
+    uint8_t *moddown_bytes = nullptr;   // the same as ConvIO::bytes
     uint64_t *p_inv = nullptr;          // [nq][2]: P^-1 mod q_j and Shoup companion
     uint64_t *p_mod = nullptr;          // [nq][2]: P mod q_j and Shoup companion (extended basis)
     std::vector<uint64_t> h_p_mod;      // host copy
@@ -89,6 +92,7 @@ struct Context {
     std::map<uint32_t, uint32_t *> galois_perm;  // elt -> [N] permutation
     std::map<uint32_t, std::vector<void *>> ext_consts;  // L -> exact Ql->P extension tables (shared.cu)
     std::mutex mu;
+    int *fault = nullptr, *fault_dev = nullptr;  // set by a kernel whose wait ran out (host-mapped)
 
     // internal arena for calls that pass no workspace
     void *arena = nullptr;
@@ -124,6 +128,8 @@ void ntt_forward(const Context &c, uint64_t *data, const NttRows &rw, cudaStream
 void ntt_inverse(const Context &c, uint64_t *data, const NttRows &rw, const uint64_t *scale, cudaStream_t st,
                  const uint64_t *src = nullptr, size_t src_stride = 0);
 
+// base conversions on the tensor cores (conv.cu)
+void conv_rows(const Context &c, const ConvIO &io, cudaStream_t st);
 // forward NTT of the rescale's spread limbs fused with the spread and the combine (RescaleIO);
 // t: [n_polys][L-1][N] scratch between the two phases
 void ntt_forward_rescale(const Context &c, const RescaleIO &io, uint64_t *t, uint32_t n_polys, uint32_t L,
@@ -229,7 +235,14 @@ void sample_uniform(const Context &c, uint64_t *out, uint32_t n_polys, uint32_t 
 void sample_cbd(const Context &c, uint64_t *out, uint32_t n_polys, uint32_t L, uint64_t seed, cudaStream_t st);
 void lift_signed(const Context &c, const int64_t *in, uint64_t *out, uint32_t n_polys, uint32_t L, cudaStream_t st);
 
-// ModUp of n_cts polynomials d (stride d_stride words) into up [n_cts][beta][LP][N]; x: [n_cts][L][N] scratch
+// The polynomials a ModUp extended (ciphertext ct's at p + ct stride): an inner product reads a digit's
+// own limbs there; p null: every limb of every digit is in `up`.
+struct OwnLimbs {
+    const uint64_t *p = nullptr;
+    size_t stride = 0;
+};
+// ModUp of n_cts polynomials d (stride d_stride words) into up [n_cts][beta][LP][N], all but the digits'
+// own limbs (NTT form already: OwnLimbs{d, d_stride}); x: [n_cts][L][N] scratch
 void modup_into(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n_cts, uint32_t L, uint64_t *x,
                 uint64_t *up, cudaStream_t st);
 
@@ -265,7 +278,7 @@ void lift_signed_ext(const Context &c, const int64_t *in, uint64_t *out, uint32_
                      cudaStream_t st);
 
 // acc [n_cts][H][LP][N] = inner products of up [n_cts][beta][LP][N] with key [beta][H][QP][N]
-void ip_multi(const Context &c, const uint64_t *up, const uint64_t *key, uint64_t *acc, uint32_t n_cts, uint32_t L,
+void ip_multi(const Context &c, const uint64_t *up, OwnLimbs own, const uint64_t *key, uint64_t *acc, uint32_t n_cts, uint32_t L,
               uint32_t beta, uint32_t H, const uint32_t *perm, cudaStream_t st);
 
 // autotuning (tune.cu): time the candidates of one knob, keep the fastest in the context

@@ -29,6 +29,7 @@
 
 #include "core.hpp"
 #include "host_math.hpp"
+#include "tcgen05.cuh"  // kKB: K bytes per stage (two k32 MMAs)
 
 namespace shm {
 
@@ -37,13 +38,11 @@ namespace {
 constexpr int kMaxMods = 20;
 constexpr uint32_t kBM = 128;   // outputs per tile (MMA M: A = the weight residues)
 constexpr uint32_t kBN = 256;   // X columns per tile (MMA N: B = the X residues)
-constexpr uint32_t kKB = 64;    // K bytes per stage (two k32 MMAs)
 constexpr int kStages = 4;
 constexpr uint32_t kStageA = kBM * kKB;  // 8 KB
 constexpr uint32_t kStageB = kBN * kKB;  // 16 KB
 constexpr uint32_t kSmem = kStages * (kStageA + kStageB) + 1024;
 constexpr uint32_t kThreads = 256;  // two warpgroups: loads shared, epilogue split by output columns
-constexpr long long kSpinLimit = 1ll << 24;
 
 // The constants of every candidate modulus, and the CRT fractions for every modulus count T
 // (M = m_0 .. m_{T-1}): the table does not depend on the call, so concurrent calls that
@@ -59,8 +58,6 @@ struct ModTab {
 };
 
 __constant__ ModTab c_mods;
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // ---------------------------------------------------------------- residues
 __device__ __forceinline__ int8_t balanced(uint32_t r, uint32_t m) { return (int8_t)(r > m / 2 ? (int)r - (int)m : (int)r); }
@@ -207,17 +204,6 @@ __global__ void wres_kernel(const int64_t *__restrict__ W, int8_t *__restrict__ 
 
 // ---------------------------------------------------------------- tcgen05 GEMM
 
-// K-major, no-swizzle ("interleaved") operand: core matrices of 8 rows x 16 bytes,
-// K-adjacent core matrices 128 B apart (LBO), 8-row groups (KB / 16) * 128 B apart (SBO).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFF);
-    d |= (uint64_t)(128 >> 4) << 16;             // leading byte offset (K direction)
-    d |= (uint64_t)((kKB / 16 * 128) >> 4) << 32;  // stride byte offset (M/N direction)
-    d |= (uint64_t)1 << 46;                      // descriptor version for sm_100
-    return d;                                    // base offset 0, lbo mode 0, layout SWIZZLE_NONE
-}
-
 // K-major operand written by TMA with the 64-byte swizzle (rows of kKB = 64 bytes, 8-row groups
 // 512 bytes apart); the MMA over K bytes [32 k, 32 k + 32) starts 32 k bytes into the atom
 __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
@@ -230,27 +216,8 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
     return d;
 }
 
-// byte offset of (row, k-chunk) inside one stage operand of `rows` x kKB bytes
-__device__ __forceinline__ uint32_t core_off(uint32_t row, uint32_t kc) {
-    return ((row >> 3) * (kKB / 16) + kc) * 128 + (row & 7) * 16;
-}
-
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
-}
-
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (long long it = 0; it < kSpinLimit; it++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity));
-        if (ok) return true;
-    }
-    return false;
 }
 
 // grid: (Np / 128, R_chunk / 256, T); one modulus per blockIdx.z.  D[o][r] = W[o] . X[r]: the

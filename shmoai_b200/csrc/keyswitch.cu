@@ -21,13 +21,14 @@ constexpr int kThreads = 256;
 constexpr int kMaxAlpha = 16;
 constexpr int kMaxBeta = 16;
 
-// acc[ct][h][j][k] = sum_b up[ct][b][j][perm[k]] * key[b][h][prime(j)][k]   (perm = identity if null)
+// acc[ct][h][j][k] = sum_b up[ct][b][j][perm[k]] * key[b][h][prime(j)][k]   (perm = identity if null);
+// limb j of its own digit j / np is read from d (ModUp leaves it there: it is unchanged)
 // An NTT-domain automorphism maps every aligned block of 32 slots onto an aligned block
 // of 32 slots, so the permuted read of a warp stays within one 256-byte segment.
 // B = beta at compile time: the key rows held in registers for the whole batch are
 // exactly 2B words, so small digit counts keep more warps resident.
 template <int B, bool S52>
-__global__ void inner_product_kernel(const uint64_t *__restrict__ up, const uint64_t *__restrict__ key,
+__global__ void inner_product_kernel(const uint64_t *__restrict__ up, OwnLimbs d, const uint64_t *__restrict__ key,
                                      uint64_t *__restrict__ acc, uint32_t n_cts, uint32_t L, uint32_t np, uint32_t nq,
                                      uint32_t log_n, const PrimeConst *__restrict__ pc,
                                      const uint32_t *__restrict__ perm) {
@@ -38,6 +39,7 @@ __global__ void inner_product_kernel(const uint64_t *__restrict__ up, const uint
     const uint32_t LP = L + np, QP = nq + np;
     const uint32_t pj = j < L ? j : nq + (j - L);
     const PrimeConst p = pc[pj];
+    const uint32_t own = j < L ? j / np : B;
     uint64_t k0[B], k1[B];
 #pragma unroll
     for (int b = 0; b < B; b++) {
@@ -46,10 +48,10 @@ __global__ void inner_product_kernel(const uint64_t *__restrict__ up, const uint
         k1[b] = kb[((size_t)QP + pj) * n + k];
     }
     for (uint32_t ct = 0; ct < n_cts; ct++) {
-        const uint64_t *u = up + (size_t)ct * B * LP * n + (size_t)j * n + ks;
+        const uint64_t *u = up + (size_t)ct * B * LP * n + (size_t)j * n + ks, *o_ = d.p + ct * d.stride + (size_t)j * n + ks;
         uint64_t v[B];
 #pragma unroll
-        for (int b = 0; b < B; b++) v[b] = u[(size_t)b * LP * n];
+        for (int b = 0; b < B; b++) v[b] = *((uint32_t)b == own ? o_ : u + (size_t)b * LP * n);
         Acc<S52> a0, a1;
 #pragma unroll
         for (int b = 0; b < B; b++) {
@@ -63,12 +65,12 @@ __global__ void inner_product_kernel(const uint64_t *__restrict__ up, const uint
 }
 
 template <bool S52>
-void launch_inner_product(dim3 grid, cudaStream_t st, const uint64_t *up, const uint64_t *key, uint64_t *acc,
+void launch_inner_product(dim3 grid, cudaStream_t st, const uint64_t *up, OwnLimbs d, const uint64_t *key, uint64_t *acc,
                           uint32_t n_cts, uint32_t L, uint32_t np, uint32_t nq, uint32_t beta, uint32_t log_n,
                           const PrimeConst *pc, const uint32_t *perm) {
 #define SHM_IP_CASE(B)                                                                                               \
     case B:                                                                                                          \
-        inner_product_kernel<B, S52><<<grid, kThreads, 0, st>>>(up, key, acc, n_cts, L, np, nq, log_n, pc, perm); \
+        inner_product_kernel<B, S52><<<grid, kThreads, 0, st>>>(up, d, key, acc, n_cts, L, np, nq, log_n, pc, perm); \
         break;
     switch (beta) {
         SHM_IP_CASE(1) SHM_IP_CASE(2) SHM_IP_CASE(3) SHM_IP_CASE(4) SHM_IP_CASE(5) SHM_IP_CASE(6) SHM_IP_CASE(7)
@@ -81,15 +83,15 @@ void launch_inner_product(dim3 grid, cudaStream_t st, const uint64_t *up, const 
 }
 
 // the inner product for one context: Acc<true> when every prime is below 2^52
-void launch_ip(const Context &c, uint32_t n_cts, uint32_t L, const uint64_t *up, const uint64_t *key, uint64_t *acc,
+void launch_ip(const Context &c, uint32_t n_cts, uint32_t L, const uint64_t *up, OwnLimbs d, const uint64_t *key, uint64_t *acc,
                const uint32_t *perm, cudaStream_t st) {
     const uint32_t np = c.np, beta = (L + np - 1) / np, LP = L + np;
     const dim3 grid(c.n / kThreads, LP);
     SHM_LAUNCHED(1);
     if (c.s52)
-        launch_inner_product<true>(grid, st, up, key, acc, n_cts, L, np, c.nq, beta, c.log_n, c.pc, perm);
+        launch_inner_product<true>(grid, st, up, d, key, acc, n_cts, L, np, c.nq, beta, c.log_n, c.pc, perm);
     else
-        launch_inner_product<false>(grid, st, up, key, acc, n_cts, L, np, c.nq, beta, c.log_n, c.pc, perm);
+        launch_inner_product<false>(grid, st, up, d, key, acc, n_cts, L, np, c.nq, beta, c.log_n, c.pc, perm);
     SHM_CUDA(cudaGetLastError());
 }
 
@@ -112,6 +114,7 @@ ModDownIO moddown_io(const Context &c, const uint64_t *acc, const KsOutput &o) {
     md.H = 2;
     md.np = c.np;
     md.s52 = c.s52 ? 1 : 0;
+    md.bytes = c.moddown_bytes;
     return md;
 }
 
@@ -158,7 +161,7 @@ void relin_rescale(const Context &c, const uint64_t *ct3, uint32_t n_cts, uint32
     const LevelKS &ks = c.ks[L];
 
     modup_into(c, ct3 + 2 * ln, 3 * ln, n_cts, L, x, up, st);
-    launch_ip(c, n_cts, L, up, key, acc, nullptr, st);
+    launch_ip(c, n_cts, L, up, {ct3 + 2 * ln, 3 * ln}, key, acc, nullptr, st);
     // y = P c + ks over QlP: P c vanishes mod every p_k; on the limbs j < L - 1 it is folded
     // into the ModDown's store as c_j q_{L-1}^-1 (= P c_j S^-1); limb L - 1 gets it here
     const uint64_t ql = c.primes[L - 1];
@@ -193,6 +196,7 @@ void relin_rescale(const Context &c, const uint64_t *ct3, uint32_t n_cts, uint32
     md.H = 2;
     md.np = np + 1;
     md.s52 = c.s52 ? 1 : 0;
+    md.bytes = ks.rr_bytes;
     md.vrow = vrow;
     md.vs = ks.rr_vs;
     ntt_forward_moddown(c, md, delta, n_cts * 2, L - 1, st);
@@ -221,31 +225,30 @@ void keyswitch(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n_
     // the rest of QlP, NTT of the converted limbs (digit rows are already NTT form)
     modup_into(c, d, d_stride, n_cts, L, x, up, st);
     // 4. inner product with the key digits
-    launch_ip(c, n_cts, L, up, key, acc, nullptr, st);
+    launch_ip(c, n_cts, L, up, {d, d_stride}, key, acc, nullptr, st);
     // 5. ModDown: INTT of the P limbs (scaled by phat_k^-1), convert to Ql, NTT, combine
     ntt_inverse(c, acc, special_rows(c, n_cts * 2, L), c.moddown_scale, st);
     ntt_forward_moddown(c, moddown_io(c, acc, o), delta, n_cts * 2, L, st);
 }
 
-// ModUp of n_cts polynomials d (stride d_stride words) into up [n_cts][beta][LP][N]; x is
-// an [n_cts][L][N] scratch.  Shared by the shared-a operations (shared.cu).
+// ModUp of n_cts polynomials d (stride d_stride words) into up [n_cts][beta][LP][N], all but the digits'
+// own limbs; x is an [n_cts][L][N] scratch.  Shared by the shared-a operations (shared.cu).
 void modup_into(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n_cts, uint32_t L, uint64_t *x,
                 uint64_t *up, cudaStream_t st) {
     const uint32_t np = c.np, beta = (L + np - 1) / np, LP = L + np;
     if (np > kMaxAlpha || beta > kMaxBeta || LP > 64) throw std::invalid_argument("key-switching shape too large");
     const LevelKS &ks = c.ks[L];
     ntt_inverse(c, x, rows_of(c, n_cts, L, L), ks.modup_scale, st, d, d_stride);
-    // the conversion is computed in the forward NTT's load and the digits' own rows are copied by
-    // the same launch: the converted limbs never go through HBM in coefficient form
+    // the conversion is computed in the forward NTT's load: the converted limbs never go through HBM in
+    // coefficient form.  The digits' own rows of up are not written: the inner products read d.
     ModUpIO mu;
     mu.x = x;
-    mu.d = d;
-    mu.d_stride = (long long)d_stride;
     mu.conv = ks.modup_conv;
     mu.L = L;
     mu.np = np;
     mu.LP = LP;
     mu.s52 = c.s52 ? 1 : 0;
+    mu.bytes = ks.modup_bytes;
     ntt_forward_modup(c, mu, up, n_cts, beta, st);
 }
 
@@ -275,7 +278,7 @@ void apply_galois_hoisted(const Context &c, const uint64_t *ct, uint32_t n_cts, 
     // per element: permuted inner product, ModDown, combine with sigma(c0)
     for (uint32_t e = 0; e < n_elts; e++) {
         const uint32_t *perm = const_cast<Context &>(c).perm(elts[e]);
-        launch_ip(c, n_cts, L, up, keys[e], acc, perm, st);
+        launch_ip(c, n_cts, L, up, {d, 2 * ln}, keys[e], acc, perm, st);
         ntt_inverse(c, acc, special_rows(c, n_cts * 2, L), c.moddown_scale, st);
         KsOutput o{outs[e], outs[e] + ln, ct, nullptr, 2 * ln, perm};
         ntt_forward_moddown(c, moddown_io(c, acc, o), delta, n_cts * 2, L, st);

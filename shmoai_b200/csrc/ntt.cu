@@ -34,7 +34,7 @@ void dispatch(const Context &c, F &&f) {
     SHM_CUDA(cudaGetLastError());
 }
 
-void forward(const Context &c, int kind, uint64_t *data, const NttRows &rw, cudaStream_t st, const NttIO &io) {
+void forward(const Context &c, int kind, uint64_t *data, const NttRows &rw, cudaStream_t st, const NttIO &io = {}) {
     if (rw.polys == 0 || rw.count == 0) return;
     dispatch(c, [&](auto r, auto fam) { launch_fwd<decltype(r)::value, decltype(fam)::value>(c, kind, data, rw, st, io); });
 }
@@ -51,7 +51,7 @@ NttRows rows_of(const Context &c, uint32_t polys, uint32_t slots, uint32_t lq) {
 }
 
 void ntt_forward(const Context &c, uint64_t *data, const NttRows &rw, cudaStream_t st) {
-    forward(c, kIoPlain, data, rw, st, NttIO{});
+    forward(c, kIoPlain, data, rw, st);
 }
 
 void ntt_forward_rescale(const Context &c, const RescaleIO &rs, uint64_t *t, uint32_t n_polys, uint32_t L,
@@ -67,6 +67,19 @@ void ntt_forward_moddown(const Context &c, const ModDownIO &md, uint64_t *delta,
     if (md.np > 16 || md.H == 0) throw std::invalid_argument("ModDown: shape out of range");
     NttIO io;
     io.md = md;
+    if (md.bytes) {
+        ConvIO cv;
+        cv.src = md.acc + (size_t)L * c.n;
+        cv.src_ct = (size_t)(L + md.np) * c.n;
+        cv.bytes = md.bytes;
+        cv.out = delta;
+        cv.vrow = md.vrow;
+        cv.sets = n_polys;
+        cv.na = cv.total = md.np;
+        cv.rows = cv.lq = L;
+        conv_rows(c, cv, st);
+        io.converted = 1;
+    }
     forward(c, kIoModDown, delta, rows_of(c, n_polys, L, L), st, io);
 }
 
@@ -79,6 +92,23 @@ void ntt_forward_modup(const Context &c, const ModUpIO &mu, uint64_t *up, uint32
     NttRows rw = rows_of(c, n_cts, beta * mu.LP, mu.L);
     rw.lp = mu.LP;
     rw.skip = mu.np;
+    if (mu.bytes) {
+        ConvIO cv;
+        cv.src = mu.x;
+        cv.src_ct = (size_t)mu.L * c.n;
+        cv.bytes = mu.bytes;
+        cv.out = up;
+        cv.skip_own = true;
+        cv.sets = n_cts * beta;
+        cv.per = beta;
+        cv.na = mu.np;
+        cv.total = mu.L;
+        cv.rows = mu.LP;
+        cv.lq = mu.L;
+        cv.nq = c.nq;
+        conv_rows(c, cv, st);
+        io.converted = 1;
+    }
     forward(c, kIoModUp, up, rw, st, io);
 }
 

@@ -79,21 +79,39 @@ struct ModDownIO {
     long long out_ct = 0, out_h = 0, add_ct = 0, add_h = 0;  // word strides
     uint32_t H = 2, np = 0, n_add = 0, n_perm = 0;
     int s52 = 0;  // every prime below 2^52: Acc<true>
+    const uint8_t *bytes = nullptr;  // the conversion's (and v's) constants for ConvIO; null: the load transform
 };
 
 // ModUp's forward NTT (ntt_forward_modup): row (ct, b, j) of up [n_cts][beta][LP][N].  For j
 // outside digit b (limbs [b alpha, min((b+1) alpha, L))) the column kernel reads the base
 // conversion sum_i y_i (qhat_i mod t_j) of the digit's INTT'd, qhat^-1-scaled limbs
-// y = x[ct][b alpha ..] (coefficient form) and the row is transformed; for j inside the digit it
-// copies d[ct][j] (already NTT form) and the block kernel leaves the row alone (NttRows::skip).  The
-// converted digits are never stored in coefficient form.
+// y = x[ct][b alpha ..] (coefficient form) and the row is transformed; rows j inside the digit are
+// left alone (NttRows::skip).  The converted digits are never stored in coefficient form.
 struct ModUpIO {
     const uint64_t *x = nullptr;     // [n_cts][L][N]
-    const uint64_t *d = nullptr;     // ciphertext ct's polynomial at d + ct * d_stride, [L][N]
     const uint64_t *conv = nullptr;  // [beta][LP][np]: qhat_i mod t_j of the level's digits
-    long long d_stride = 0;
     uint32_t L = 0, np = 0, LP = 0;
     int s52 = 0;
+    const uint8_t *bytes = nullptr;  // as ModDownIO's
+};
+
+// The same conversions with the products on the tensor cores (conv.cu).  Set s (ciphertext
+// s / per, digit s % per) has the coefficient-form limbs y_i at src + ct src_ct + (digit na + i) N,
+// i < na (fewer in the last digit: total limbs in all); output row j (prime j below lq, else
+// nq + j - lq) is sum_i y_i c_ij, plus v c_(na)j when an overflow count v is given per coefficient,
+// at out[s][j] in the form the row's butterflies take; with skip_own a row j of the digit's own limbs is left alone.
+// bytes: [per][rows][512], row j's constants: byte o of (c_ij 2^(8b) mod q_j) at
+// (k / 16) 128 + 16 o + k % 16, k = 8 i + b.
+constexpr uint32_t kConvSlots = 8;  // limbs and overflow count of a set
+struct ConvIO {
+    const uint64_t *src = nullptr;
+    size_t src_ct = 0;
+    const uint8_t *bytes = nullptr;
+    uint64_t *out = nullptr;
+    const uint8_t *vrow = nullptr;  // [sets][N]
+    uint32_t sets = 0, per = 1, na = 1, total = 1, rows = 0, lq = 0, nq = 0;
+    bool skip_own = false;
+    __host__ __device__ __forceinline__ uint32_t prime(uint32_t j) const { return j < lq ? j : nq + (j - lq); }
 };
 
 // the optional load / store transforms of the forward NTT kernels
@@ -101,8 +119,9 @@ struct NttIO {
     RescaleIO rs;
     ModDownIO md;
     ModUpIO mu;
+    int converted = 0;  // ModUp, ModDown: the rows have been converted (conv_rows)
 };
-constexpr int kIoPlain = 0, kIoRescale = 1, kIoModDown = 2, kIoModUp = 3;
+constexpr int kIoPlain = 0, kIoRescale = 1, kIoModDown = 2, kIoModUp = 3, kIoConverted = 4;
 
 __device__ __forceinline__ void ct_bf(uint64_t &x, uint64_t &y, uint64_t w, uint64_t ws, uint64_t q) {
     uint64_t q2 = 2 * q;

@@ -1,6 +1,8 @@
 // The NTT kernels (see ntt.cuh for the decomposition) and their launches, a template over the ring
 // (R: N = 2^(4R)) and the butterfly families; every instantiation is a translation unit of its own.
 #pragma once
+#include <algorithm>
+
 #include "core.hpp"
 
 namespace shm {
@@ -66,7 +68,7 @@ __device__ __forceinline__ uint64_t conv_sum(const uint64_t *__restrict__ x, con
 // ---------------- forward, phase 1: columns (global stages 0 .. LOGM-1)
 // IOK = kIoRescale: row (poly, j) is read as c_last[poly] mod q_j from the coefficient-form
 // last limbs; kIoModDown: as the base conversion of the special-prime limbs (ModDownIO);
-// kIoPlain: from `data`
+// kIoPlain: from `data`; kIoConverted: from `data`, as conv_rows leaves it
 template <int R, int S, int MINB, int IOK, int FAM>
 __global__ void __launch_bounds__(Geo<R, S>::THREADS, MINB)
     fwd_col(uint64_t *__restrict__ data, NttRows rw, const uint64_t *__restrict__ tw, const double *__restrict__ twd,
@@ -81,17 +83,7 @@ __global__ void __launch_bounds__(Geo<R, S>::THREADS, MINB)
     const uint32_t pidx = row_prime(rw, slot);
     const uint32_t sig = threadIdx.x % S, lane = threadIdx.x / S;
     uint64_t *x = data + ((size_t)(poly * rw.slots + slot) << G::LOGN) + chunk * S;
-    if (pidx == kNoPrime) {
-        if constexpr (IOK == kIoModUp) {  // a limb of the digit itself: the NTT-form input, copied
-            const uint64_t *src = io.mu.d + poly * io.mu.d_stride + ((size_t)(slot % rw.lp) << G::LOGN) + chunk * S;
-#pragma unroll
-            for (int m = 0; m < G::E; m++) {
-                const size_t pos = sig + (size_t)G::M * (lane + m * G::E);
-                x[pos] = src[pos];
-            }
-        }
-        return;
-    }
+    if (pidx == kNoPrime) return;  // ModUp: a limb of the digit itself
     const Limb<R> lb(pidx, false, tw, twd, pc);
     uint64_t a[G::E];
     if constexpr (IOK == kIoModUp) {
@@ -137,7 +129,9 @@ __global__ void __launch_bounds__(Geo<R, S>::THREADS, MINB)
 #pragma unroll
         for (int m = 0; m < G::E; m++) a[m] = x[sig + (size_t)G::M * (lane + m * G::E)];
     }
-    if (fam_has(FAM, kBfF64) && lb.mode == kBfF64) {  // [0, q) -> doubles for the FP64 butterflies
+    if (IOK == kIoConverted) {
+        // already doubles within about q/2 of zero, or in [0, q) for the integer families
+    } else if (fam_has(FAM, kBfF64) && lb.mode == kBfF64) {  // [0, q) -> doubles for the FP64 butterflies
 #pragma unroll
         for (int m = 0; m < G::E; m++) a[m] = as_bits(to_dbl(a[m]));
     } else if (fam_has(FAM, kBfF64R) && lb.mode == kBfF64R) {
@@ -359,7 +353,11 @@ void launch_fwd_v(const Context &c, uint64_t *data, const NttRows &rw, cudaStrea
     dim3 grid(rw.polys * rw.count * G::CHUNKS);
     constexpr int BLK = IOK == kIoModUp ? kIoPlain : IOK;  // ModUp's block phase is a plain one
     SHM_LAUNCHED(1);
-    fwd_col<R, S, MINB, IOK, FAM><<<grid, G::THREADS, 0, st>>>(data, rw, c.tw, c.twd, c.pc, io);
+    // rows converted by conv_rows: the plain column phase, whose input is in the butterflies' form
+    if ((IOK == kIoModUp || IOK == kIoModDown) && io.converted)
+        fwd_col<R, S, MINB, kIoConverted, FAM><<<grid, G::THREADS, 0, st>>>(data, rw, c.tw, c.twd, c.pc, io);
+    else
+        fwd_col<R, S, MINB, IOK, FAM><<<grid, G::THREADS, 0, st>>>(data, rw, c.tw, c.twd, c.pc, io);
     SHM_LAUNCHED(1);
     fwd_blk<R, S, MINB, BLK, FAM><<<grid, G::THREADS, 0, st>>>(data, rw, c.tw, c.twd, c.pc, io);
 }
@@ -388,7 +386,8 @@ void launch_fwd_f(const Context &c, uint64_t *data, const NttRows &rw, cudaStrea
     }
 }
 
-// the butterfly families FAM in the ring R
+// A forward transform of the rows of `data` in the butterfly families FAM and the ring R; kind: the load and
+// store transforms
 template <int R, int FAM>
 void launch_fwd(const Context &c, int kind, uint64_t *data, const NttRows &rw, cudaStream_t st, const NttIO &io) {
     switch (kind) {

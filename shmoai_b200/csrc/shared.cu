@@ -29,7 +29,8 @@ namespace {
 constexpr int kT = 256;
 constexpr int kMaxB = 16;
 
-// acc[ct][h][j][k] = sum_b up[ct][b][j][perm(k)] * key[b][h][prime(j)][k], h < H.
+// acc[ct][h][j][k] = sum_b up[ct][b][j][perm(k)] * key[b][h][prime(j)][k], h < H (limb j of digit j / np
+// from own, when given).
 // A block handles `chunk` groups: each thread stages its own extended-digit words of those
 // groups in shared memory (a column per thread, so no synchronisation), then, half by
 // half, holds the key digits in registers and serves every group of the chunk: the key
@@ -39,7 +40,7 @@ constexpr int kIpT = 128;
 constexpr size_t kIpSmemMax = 96 * 1024;  // largest chunk the autotuner may pick
 
 template <bool S52>
-__global__ void __launch_bounds__(kIpT) ip_multi_kernel(const uint64_t *__restrict__ up,
+__global__ void __launch_bounds__(kIpT) ip_multi_kernel(const uint64_t *__restrict__ up, OwnLimbs own,
                                                         const uint64_t *__restrict__ key, uint64_t *__restrict__ acc,
                                                         uint32_t n_cts, uint32_t chunk, uint32_t L, uint32_t np,
                                                         uint32_t nq, uint32_t beta, uint32_t H, uint32_t log_n,
@@ -54,9 +55,12 @@ __global__ void __launch_bounds__(kIpT) ip_multi_kernel(const uint64_t *__restri
     const uint32_t pj = j < L ? j : nq + (j - L);
     const PrimeConst p = pc[pj];
     const uint32_t c0 = blockIdx.z * chunk, nc = min(chunk, n_cts - c0);
+    const uint32_t ob = own.p && j < L ? j / np : beta;
     for (uint32_t ct = 0; ct < nc; ct++) {
         const uint64_t *up_c = up + (size_t)(c0 + ct) * beta * LP * n + (size_t)j * n + ks;
-        for (uint32_t b = 0; b < beta; b++) su[(ct * beta + b) * kIpT + threadIdx.x] = up_c[(size_t)b * LP * n];
+        const uint64_t *own_c = own.p + (c0 + ct) * own.stride + (size_t)j * n + ks;
+        for (uint32_t b = 0; b < beta; b++)
+            su[(ct * beta + b) * kIpT + threadIdx.x] = *(b == ob ? own_c : up_c + (size_t)b * LP * n);
     }
     for (uint32_t h = 0; h < H; h++) {
         uint64_t kk[kMaxB];
@@ -167,7 +171,7 @@ ExtConsts ext_consts(Context &c, uint32_t L) {
 
 // The Sh-Rot / FmtSwitch inner products: groups are served in chunks that fit
 // c.ip_chunk_bytes of shared memory, each chunk reading the key once.
-void ip_multi(const Context &c, const uint64_t *up, const uint64_t *key, uint64_t *acc, uint32_t n_cts, uint32_t L,
+void ip_multi(const Context &c, const uint64_t *up, OwnLimbs own, const uint64_t *key, uint64_t *acc, uint32_t n_cts, uint32_t L,
               uint32_t beta, uint32_t H, const uint32_t *perm, cudaStream_t st) {
     static std::once_flag attr;
     std::call_once(attr, [] {
@@ -181,10 +185,10 @@ void ip_multi(const Context &c, const uint64_t *up, const uint64_t *key, uint64_
     const size_t smem = (size_t)chunk * beta * kIpT * 8;
     SHM_LAUNCHED(1);
     if (c.s52)
-        ip_multi_kernel<true><<<grid, kIpT, smem, st>>>(up, key, acc, n_cts, chunk, L, np, c.nq, beta, H, c.log_n,
+        ip_multi_kernel<true><<<grid, kIpT, smem, st>>>(up, own, key, acc, n_cts, chunk, L, np, c.nq, beta, H, c.log_n,
                                                         c.pc, perm);
     else
-        ip_multi_kernel<false><<<grid, kIpT, smem, st>>>(up, key, acc, n_cts, chunk, L, np, c.nq, beta, H, c.log_n,
+        ip_multi_kernel<false><<<grid, kIpT, smem, st>>>(up, own, key, acc, n_cts, chunk, L, np, c.nq, beta, H, c.log_n,
                                                          c.pc, perm);
     SHM_CUDA(cudaGetLastError());
 }
@@ -199,10 +203,10 @@ void check_shape(const Context &c, uint32_t L, uint32_t beta, uint32_t H) {
 }
 
 // inner products, ModDown and combine for one target; acc/delta are workspace
-void apply_target(const Context &c, const uint64_t *up, uint32_t n_cts, uint32_t L, uint32_t beta, uint32_t H,
+void apply_target(const Context &c, const uint64_t *up, OwnLimbs own, uint32_t n_cts, uint32_t L, uint32_t beta, uint32_t H,
                   const Target &t, uint64_t *acc, uint64_t *delta, cudaStream_t st) {
     const uint32_t np = c.np;
-    ip_multi(c, up, t.key, acc, n_cts, L, beta, H, t.perm, st);
+    ip_multi(c, up, own, t.key, acc, n_cts, L, beta, H, t.perm, st);
     ntt_inverse(c, acc, special_rows(c, n_cts * H, L), c.moddown_scale, st);
     // conversion of the special-prime limbs, NTT and (acc - delta) P^-1 + sigma(add) fused
     ModDownIO md;
@@ -221,6 +225,7 @@ void apply_target(const Context &c, const uint64_t *up, uint32_t n_cts, uint32_t
     md.H = H;
     md.np = np;
     md.s52 = c.s52 ? 1 : 0;
+    md.bytes = c.moddown_bytes;
     ntt_forward_moddown(c, md, delta, n_cts * H, L, st);
 }
 
@@ -244,7 +249,7 @@ void shared_rotate_hoisted(const Context &c, const uint64_t *sh, uint32_t n_grou
     for (uint32_t e = 0; e < n_elts; e++) {
         Target t{keys[e], const_cast<Context &>(c).perm(elts[e]), outs[e], (size_t)H * ln, ln, sh, (size_t)H * ln,
                  ln, n};
-        apply_target(c, up, n_groups, L, beta, H, t, acc, delta, st);
+        apply_target(c, up, {sh + (size_t)n * ln, (size_t)H * ln}, n_groups, L, beta, H, t, acc, delta, st);
     }
 }
 
@@ -271,7 +276,7 @@ void fmt_forward(const Context &c, const uint64_t *cts, uint32_t n_groups, uint3
     ntt_forward(c, ext, special_rows(c, m, L), st);
     // digits = the n members of a group: ext is [G][n][LP][N]
     Target t{key, nullptr, out, (size_t)H * ln, ln, cts, (size_t)n * 2 * ln, 2 * ln, n};
-    apply_target(c, ext, n_groups, L, n, H, t, acc, delta, st);
+    apply_target(c, ext, {}, n_groups, L, n, H, t, acc, delta, st);
 }
 
 size_t fmt_backward_ws_words(const Context &c, uint32_t n_groups, uint32_t n, uint32_t L) {
@@ -293,7 +298,7 @@ void fmt_backward(const Context &c, const uint64_t *sh, uint32_t n_groups, uint3
         // member i of group g -> ordinary ciphertext g * n + i = (b_i + cx0, cx1)
         Target t{keys[i], nullptr, out + (size_t)i * 2 * ln, (size_t)n * 2 * ln, ln, sh + (size_t)i * ln,
                  (size_t)H * ln, 0, 1};
-        apply_target(c, up, n_groups, L, beta, 2, t, acc, delta, st);
+        apply_target(c, up, {sh + (size_t)n * ln, (size_t)H * ln}, n_groups, L, beta, 2, t, acc, delta, st);
     }
 }
 
@@ -355,6 +360,7 @@ void moddown_rows(const Context &c, uint64_t *ext, uint64_t *out, uint32_t n_pol
     md.H = 1;
     md.np = c.np;
     md.s52 = c.s52 ? 1 : 0;
+    md.bytes = c.moddown_bytes;
     ntt_forward_moddown(c, md, delta, n_polys, L, st);
 }
 
@@ -401,18 +407,21 @@ void shared_rotate_ext(const Context &c, const uint64_t *in, bool in_ext, uint32
     uint64_t *arow = acc + (size_t)n_groups * H * LP * N, *aq = arow + (size_t)n_groups * LP * N;
     uint64_t *delta = aq + (size_t)n_groups * ln;
     const size_t g_words = (size_t)H * (in_ext ? LP : L) * N;  // one input group
+    OwnLimbs own;
     if (in_ext) {
         // ModDown of the a row of every group, then ModUp of it
         SHM_CUDA(cudaMemcpy2DAsync(arow, LP * N * 8, in + (size_t)n * LP * N, g_words * 8, LP * N * 8, n_groups,
                                    cudaMemcpyDeviceToDevice, st));
         moddown_rows(c, arow, aq, n_groups, L, delta, st);
         modup_into(c, aq, ln, n_groups, L, x, up, st);
+        own = {aq, ln};
     } else {
         modup_into(c, in + (size_t)n * ln, g_words, n_groups, L, x, up, st);
+        own = {in + (size_t)n * ln, g_words};
     }
     for (uint32_t e = 0; e < n_elts; e++) {
         const uint32_t *perm = const_cast<Context &>(c).perm(elts[e]);
-        ip_multi(c, up, keys[e], acc, n_groups, L, beta, H, perm, st);
+        ip_multi(c, up, own, keys[e], acc, n_groups, L, beta, H, perm, st);
         SHM_LAUNCHED(1);
         combine_ext_kernel<<<dim3(N / kT, LP, n_groups * H), kT, 0, st>>>(acc, outs[e], in, in_ext ? 1 : 0, perm, H, L,
                                                                           c.np, c.nq, c.log_n, c.pc, c.p_mod);

@@ -97,7 +97,7 @@ uint32_t tune_ip_chunk(Context &c, uint32_t groups, uint32_t L, uint32_t members
     ms.clear();
     for (uint32_t b : kIpChunkCandidates) {
         c.ip_chunk_bytes = b;
-        ms.push_back(time_ms(s.st, 5, [&] { ip_multi(c, up, key, acc, groups, L, beta, H, nullptr, s.st); }));
+        ms.push_back(time_ms(s.st, 5, [&] { ip_multi(c, up, {}, key, acc, groups, L, beta, H, nullptr, s.st); }));
     }
     const uint32_t best = argmin(ms);
     c.ip_chunk_bytes = kIpChunkCandidates[best];
