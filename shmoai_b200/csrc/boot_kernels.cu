@@ -47,6 +47,7 @@ __global__ void add_scalar_kernel(const uint64_t *__restrict__ a, uint64_t *__re
 // Limb-major block order: blockIdx.y = limb * n_polys + poly, so the polynomials that share a
 // plaintext limb run together and the k plaintext limbs stay in L2 for all of them.
 // L = limbs per row; limb l uses prime l when l < Lq, else the special prime nq + l - Lq
+template <bool S52>
 __global__ void mul_plain_acc_kernel(PtrTab X, PtrTab P, uint32_t k, uint64_t *__restrict__ out, uint32_t L,
                                      uint32_t log_n, const PrimeConst *__restrict__ pc, int accumulate, uint32_t Lq,
                                      uint32_t nq) {
@@ -54,12 +55,12 @@ __global__ void mul_plain_acc_kernel(PtrTab X, PtrTab P, uint32_t k, uint64_t *_
     const PrimeConst p = pc[limb < Lq ? limb : nq + (limb - Lq)];
     const size_t off = ((size_t)row << log_n) + blockIdx.x * kT + threadIdx.x;
     const size_t poff = ((size_t)limb << log_n) + blockIdx.x * kT + threadIdx.x;
-    u128 acc = {0, 0};
+    Acc<S52> acc;
     // unrolled so that a group of terms' loads is in flight together (the loads, not the
     // multiplies, bound this kernel)
 #pragma unroll 8
-    for (uint32_t t = 0; t < k; t++) mac(acc, X.p[t][off], P.p[t][poff]);
-    uint64_t r = barrett(acc, p);
+    for (uint32_t t = 0; t < k; t++) acc.add(X.p[t][off], P.p[t][poff]);
+    uint64_t r = acc.reduce(p);
     if (accumulate) r = add_mod(r, out[off], p.q);
     out[off] = r;
 }
@@ -126,8 +127,8 @@ void mul_plain_acc(const Context &c, const PtrTab &X, const PtrTab &P, uint32_t 
     if (!n_polys || !k) return;
     const uint32_t rows = ext ? L + c.np : L;
     SHM_LAUNCHED(1);
-    mul_plain_acc_kernel<<<dim3(c.n / kT, n_polys * rows), kT, 0, st>>>(X, P, k, out, rows, c.log_n, c.pc,
-                                                                         accumulate ? 1 : 0, L, c.nq);
+    const auto f = c.s52 ? mul_plain_acc_kernel<true> : mul_plain_acc_kernel<false>;
+    f<<<dim3(c.n / kT, n_polys * rows), kT, 0, st>>>(X, P, k, out, rows, c.log_n, c.pc, accumulate ? 1 : 0, L, c.nq);
     SHM_CUDA(cudaGetLastError());
 }
 

@@ -9,6 +9,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "modarith.cuh"
@@ -72,7 +73,7 @@ struct Context {
     uint32_t sms = 148;                 // multiprocessors of the device
     uint32_t log_n = 0, n = 0, nq = 0, np = 0, dnum = 0;
     std::vector<uint64_t> primes;       // nq + np
-    bool s52 = false;                   // every prime below kS52PrimeLimit (Acc<true> kernels)
+    bool s52 = false;                   // every prime in [kS52PrimeMin, kS52PrimeLimit) (Acc<true> kernels)
     int ntt_variant = 0;                // index into kNttVariants (set by the autotuner)
     int ntt_families = 0;               // the NTT instantiation for the primes' butterfly families (kFam*)
     uint32_t ip_chunk_bytes = 32768;    // shared memory per Sh-Rot inner-product block (autotuned)
@@ -234,6 +235,56 @@ void release_encode_tables(const Context &c);
 void sample_uniform(const Context &c, uint64_t *out, uint32_t n_polys, uint32_t L, uint64_t seed, cudaStream_t st);
 void sample_cbd(const Context &c, uint64_t *out, uint32_t n_polys, uint32_t L, uint64_t seed, cudaStream_t st);
 void lift_signed(const Context &c, const int64_t *in, uint64_t *out, uint32_t n_polys, uint32_t L, cudaStream_t st);
+
+// How an inner product of `beta` digits with key rows is summed: on doubles when every prime is below 2^51
+// and the digits fit AccDbl (the bootstrapping chains), in 26-bit halves for the other chains of
+// Context::s52, else in 128 bits.
+constexpr int kIpWide = 0, kIpS52 = 1, kIpDbl = 2;
+
+template <int A>
+struct IpSum {
+    using Acc = shm::Acc<A == kIpS52>;
+    using Op = Operand<A == kIpS52>;
+    using T = typename Op::type;
+    const PrimeConst p;
+    __device__ __forceinline__ explicit IpSum(const PrimeConst &p_) : p(p_) {}
+    __device__ __forceinline__ T operand(uint64_t x) const { return Op::of(x); }
+    __device__ __forceinline__ void add(Acc &a, int, T x, T y) const { a.add(x, y); }
+    __device__ __forceinline__ uint64_t reduce(const Acc &a) const { return a.reduce(p); }
+};
+template <>
+struct IpSum<kIpDbl> {
+    using Acc = AccDbl;
+    using T = double;
+    const uint64_t q;
+    const double qd, qinv, c;
+    __device__ __forceinline__ explicit IpSum(const PrimeConst &p)
+        : q(p.q), qd((double)p.q), qinv(p.qinv), c(AccDbl::two51_mod((double)p.q, p.qinv)) {}
+    __device__ __forceinline__ T operand(uint64_t x) const { return to_dbl_centred(x, q); }
+    __device__ __forceinline__ void add(Acc &a, int i, T x, T y) const { a.add(i, x, y); }
+    __device__ __forceinline__ uint64_t reduce(const Acc &a) const { return a.reduce(qd, qinv, c); }
+};
+
+// f(beta, summation) with both as compile-time constants
+template <class F>
+void ip_dispatch(const Context &c, uint32_t beta, F &&f) {
+    auto go = [&](auto b) {
+        constexpr int B = decltype(b)::value;
+        if constexpr (B <= kMaxDblTerms)
+            if (c.ntt_families == kFamSmall) return f(b, std::integral_constant<int, kIpDbl>{});
+        if (c.s52) f(b, std::integral_constant<int, kIpS52>{});
+        else f(b, std::integral_constant<int, kIpWide>{});
+    };
+#define SHM_IP_CASE(B) \
+    case B: go(std::integral_constant<int, B>{}); break;
+    switch (beta) {
+        SHM_IP_CASE(1) SHM_IP_CASE(2) SHM_IP_CASE(3) SHM_IP_CASE(4) SHM_IP_CASE(5) SHM_IP_CASE(6) SHM_IP_CASE(7)
+        SHM_IP_CASE(8) SHM_IP_CASE(9) SHM_IP_CASE(10) SHM_IP_CASE(11) SHM_IP_CASE(12) SHM_IP_CASE(13)
+        SHM_IP_CASE(14) SHM_IP_CASE(15) SHM_IP_CASE(16)
+        default: throw std::invalid_argument("key-switching digit count out of range");
+    }
+#undef SHM_IP_CASE
+}
 
 // The polynomials a ModUp extended (ciphertext ct's at p + ct stride): an inner product reads a digit's
 // own limbs there; p null: every limb of every digit is in `up`.

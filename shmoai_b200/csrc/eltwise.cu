@@ -79,7 +79,7 @@ __global__ void tensor_kernel(const uint64_t *__restrict__ a, const uint64_t *__
 // out[ct] (+)= sum_{t < k} A_t[ct a_step] x B_t[ct b_step]: the size-3 tensor products of k
 // ciphertext pairs summed before one reduction (step 0 broadcasts one ciphertext over the batch).
 // The host bounds k so that each sum (2k products for the middle term) stays below the Barrett
-// bound; S52: the products' 32-bit partials summed in three 64-bit words (every prime < 2^52).
+// bound; S52: Context::s52.
 template <bool S52>
 __global__ void tensor_acc_kernel(PtrTab A, PtrTab B, uint32_t k, uint32_t a_step, uint32_t b_step,
                                   uint64_t *__restrict__ out, uint32_t L, uint32_t log_n,
@@ -91,14 +91,15 @@ __global__ void tensor_acc_kernel(PtrTab A, PtrTab B, uint32_t k, uint32_t a_ste
     Acc<S52> s0, s1, s2;
     for (uint32_t t = 0; t < k; t++) {
         const uint64_t *a = A.p[t] + (size_t)ct * a_step * 2 * ln, *b = B.p[t] + (size_t)ct * b_step * 2 * ln;
-        const uint64_t a0 = a[kk], a1 = a[ln + kk], b0 = b[kk], b1 = b[ln + kk];
+        using Op = Operand<S52>;
+        const auto a0 = Op::of(a[kk]), a1 = Op::of(a[ln + kk]), b0 = Op::of(b[kk]), b1 = Op::of(b[ln + kk]);
         s0.add(a0, b0);
         s1.add(a0, b1);
         s1.add(a1, b0);
         s2.add(a1, b1);
     }
     uint64_t *O = out + (size_t)ct * 3 * ln;
-    uint64_t r0 = barrett(s0.get(), p), r1 = barrett(s1.get(), p), r2 = barrett(s2.get(), p);
+    uint64_t r0 = s0.reduce(p), r1 = s1.reduce(p), r2 = s2.reduce(p);
     if (accumulate) {
         r0 = add_mod(r0, O[kk], p.q);
         r1 = add_mod(r1, O[ln + kk], p.q);

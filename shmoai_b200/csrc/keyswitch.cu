@@ -26,72 +26,65 @@ constexpr int kMaxBeta = 16;
 // An NTT-domain automorphism maps every aligned block of 32 slots onto an aligned block
 // of 32 slots, so the permuted read of a warp stays within one 256-byte segment.
 // B = beta at compile time: the key rows held in registers for the whole batch are
-// exactly 2B words, so small digit counts keep more warps resident.
-template <int B, bool S52>
+// exactly 2B words, so small digit counts keep more warps resident.  A: how the products are summed
+// (core.hpp).
+template <int B, int A>
 __global__ void inner_product_kernel(const uint64_t *__restrict__ up, OwnLimbs d, const uint64_t *__restrict__ key,
                                      uint64_t *__restrict__ acc, uint32_t n_cts, uint32_t L, uint32_t np, uint32_t nq,
                                      uint32_t log_n, const PrimeConst *__restrict__ pc,
                                      const uint32_t *__restrict__ perm) {
+    using I = IpSum<A>;
     const uint32_t j = blockIdx.y;
     const uint32_t k = blockIdx.x * kThreads + threadIdx.x;
     const uint32_t ks = perm ? __ldg(perm + k) : k;
     const size_t n = (size_t)1 << log_n;
     const uint32_t LP = L + np, QP = nq + np;
     const uint32_t pj = j < L ? j : nq + (j - L);
-    const PrimeConst p = pc[pj];
+    const I ip(pc[pj]);
     const uint32_t own = j < L ? j / np : B;
-    uint64_t k0[B], k1[B];
+    typename I::T k0[B], k1[B];
 #pragma unroll
     for (int b = 0; b < B; b++) {
         const uint64_t *kb = key + (size_t)b * 2 * QP * n;
-        k0[b] = kb[(size_t)pj * n + k];
-        k1[b] = kb[((size_t)QP + pj) * n + k];
+        k0[b] = ip.operand(kb[(size_t)pj * n + k]);
+        k1[b] = ip.operand(kb[((size_t)QP + pj) * n + k]);
     }
-    for (uint32_t ct = 0; ct < n_cts; ct++) {
-        const uint64_t *u = up + (size_t)ct * B * LP * n + (size_t)j * n + ks, *o_ = d.p + ct * d.stride + (size_t)j * n + ks;
-        uint64_t v[B];
+    const uint64_t *u = up + (size_t)j * n + ks, *o_ = d.p + (size_t)j * n + ks;
+    uint64_t *o = acc + (size_t)j * n + k;  // output in natural slot order
+    uint64_t v[B];
 #pragma unroll
-        for (int b = 0; b < B; b++) v[b] = *((uint32_t)b == own ? o_ : u + (size_t)b * LP * n);
-        Acc<S52> a0, a1;
+    for (int b = 0; b < B; b++) v[b] = *((uint32_t)b == own ? o_ : u + (size_t)b * LP * n);
+    for (uint32_t ct = 0; ct < n_cts; ct++, o += (size_t)2 * LP * n) {
+        typename I::T x[B];
+#pragma unroll
+        for (int b = 0; b < B; b++) x[b] = ip.operand(v[b]);
+        if (ct + 1 < n_cts) {  // the next ciphertext's words are in flight during this one's products
+            u += (size_t)B * LP * n;
+            o_ += d.stride;
+#pragma unroll
+            for (int b = 0; b < B; b++) v[b] = *((uint32_t)b == own ? o_ : u + (size_t)b * LP * n);
+        }
+        typename I::Acc a0, a1;
 #pragma unroll
         for (int b = 0; b < B; b++) {
-            a0.add(v[b], k0[b]);
-            a1.add(v[b], k1[b]);
+            ip.add(a0, b, x[b], k0[b]);
+            ip.add(a1, b, x[b], k1[b]);
         }
-        uint64_t *o = acc + (size_t)ct * 2 * LP * n + (size_t)j * n + k;  // output in natural slot order
-        o[0] = barrett(a0.get(), p);
-        o[(size_t)LP * n] = barrett(a1.get(), p);
+        o[0] = ip.reduce(a0);
+        o[(size_t)LP * n] = ip.reduce(a1);
     }
 }
 
-template <bool S52>
-void launch_inner_product(dim3 grid, cudaStream_t st, const uint64_t *up, OwnLimbs d, const uint64_t *key, uint64_t *acc,
-                          uint32_t n_cts, uint32_t L, uint32_t np, uint32_t nq, uint32_t beta, uint32_t log_n,
-                          const PrimeConst *pc, const uint32_t *perm) {
-#define SHM_IP_CASE(B)                                                                                               \
-    case B:                                                                                                          \
-        inner_product_kernel<B, S52><<<grid, kThreads, 0, st>>>(up, d, key, acc, n_cts, L, np, nq, log_n, pc, perm); \
-        break;
-    switch (beta) {
-        SHM_IP_CASE(1) SHM_IP_CASE(2) SHM_IP_CASE(3) SHM_IP_CASE(4) SHM_IP_CASE(5) SHM_IP_CASE(6) SHM_IP_CASE(7)
-        SHM_IP_CASE(8) SHM_IP_CASE(9) SHM_IP_CASE(10) SHM_IP_CASE(11) SHM_IP_CASE(12) SHM_IP_CASE(13)
-        SHM_IP_CASE(14) SHM_IP_CASE(15) SHM_IP_CASE(16)
-        default:
-            throw std::invalid_argument("key-switching digit count out of range");
-    }
-#undef SHM_IP_CASE
-}
-
-// the inner product for one context: Acc<true> when every prime is below 2^52
-void launch_ip(const Context &c, uint32_t n_cts, uint32_t L, const uint64_t *up, OwnLimbs d, const uint64_t *key, uint64_t *acc,
-               const uint32_t *perm, cudaStream_t st) {
+// the inner product for one context
+void launch_ip(const Context &c, uint32_t n_cts, uint32_t L, const uint64_t *up, OwnLimbs d, const uint64_t *key,
+               uint64_t *acc, const uint32_t *perm, cudaStream_t st) {
     const uint32_t np = c.np, beta = (L + np - 1) / np, LP = L + np;
     const dim3 grid(c.n / kThreads, LP);
     SHM_LAUNCHED(1);
-    if (c.s52)
-        launch_inner_product<true>(grid, st, up, d, key, acc, n_cts, L, np, c.nq, beta, c.log_n, c.pc, perm);
-    else
-        launch_inner_product<false>(grid, st, up, d, key, acc, n_cts, L, np, c.nq, beta, c.log_n, c.pc, perm);
+    ip_dispatch(c, beta, [&](auto b, auto a) {
+        inner_product_kernel<decltype(b)::value, decltype(a)::value><<<grid, kThreads, 0, st>>>(
+            up, d, key, acc, n_cts, L, np, c.nq, c.log_n, c.pc, perm);
+    });
     SHM_CUDA(cudaGetLastError());
 }
 

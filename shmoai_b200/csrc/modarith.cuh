@@ -76,40 +76,6 @@ __device__ __forceinline__ void mac(u128 &acc, uint64_t a, uint64_t b) {
     asm("add.cc.u64 %0, %0, %2;\n\taddc.u64 %1, %1, %3;" : "+l"(acc.lo), "+l"(acc.hi) : "l"(lo), "l"(hi));
 }
 
-// Sum of products, generic (Acc<false>: 128-bit accumulator, any 64-bit operands) or for
-// operands below 2^52 (Acc<true>, the limbs of primes below 2^52).  With a = a1 2^32 + a0
-// and b = b1 2^32 + b0 (a1, b1 < 2^20), Acc<true> adds the 32 x 32-bit partial products into
-// three 64-bit sums, hi = sum a1 b1, mid = sum (a0 b1 + a1 b0 + hi32(a0 b0)) and
-// lo = sum lo32(a0 b0), which cannot overflow below 2^11 terms: four wide multiplies and no
-// carry chain per term, one fold at the end.
-template <bool S52>
-struct Acc {
-    u128 v{0, 0};
-    __device__ __forceinline__ void add(uint64_t a, uint64_t b) { mac(v, a, b); }
-    __device__ __forceinline__ u128 get() const { return v; }
-};
-
-template <>
-struct Acc<true> {
-    uint64_t lo = 0, mid = 0, hi = 0;
-    __device__ __forceinline__ void add(uint64_t a, uint64_t b) {
-        const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
-        const uint64_t t = (uint64_t)a0 * b0;
-        lo += (uint32_t)t;
-        mid += (t >> 32) + (uint64_t)a0 * b1 + (uint64_t)a1 * b0;
-        hi += (uint64_t)a1 * b1;
-    }
-    __device__ __forceinline__ u128 get() const {
-        u128 x;
-        x.lo = lo + (mid << 32);
-        x.hi = hi + (mid >> 32) + (x.lo < lo ? 1 : 0);
-        return x;
-    }
-};
-
-// every prime of the chain below 2^52: the kernels may use Acc<true>
-constexpr uint64_t kS52PrimeLimit = 1ull << 52;
-
 __device__ __forceinline__ uint64_t barrett(u128 x, const PrimeConst &p) {
     uint64_t t = (x.hi << (64 - p.shift)) | (x.lo >> p.shift);
     uint64_t qh = mulhi64(t, p.mu);
@@ -117,6 +83,61 @@ __device__ __forceinline__ uint64_t barrett(u128 x, const PrimeConst &p) {
     r = csub(r, 2 * p.q);
     return csub(r, p.q);
 }
+
+// Sum of products: Acc<false> for any operands (a 128-bit accumulator, one Barrett reduction), or
+// Acc<true> for residues of primes in [2^40, 2^52).  There an operand is split at bit 26 into halves
+// below 2^26, and the 32 x 32-bit products go into three 64-bit sums of weights 1, 2^26 and 2^52 (hi,
+// mid, lo; no overflow below 2^10 terms): four wide multiply-adds per term with nothing beside them (split
+// at bit 32, each term's low product had to be taken apart and added in two places).  reduce() takes two
+// quotients from the FP64 pipe: hi 2^26 and then ((hi 2^26 mod q) + mid) 2^26 + lo are each brought within
+// about q/2 of zero.  With n terms both quotients stay below n 2^27, far inside the 2^51 that the rounding
+// through 1.5 2^52 takes exactly, and their errors (two roundings of a double) below 2^-17.  A 64 x 64-bit
+// high product as Barrett's quotient needs issues at 7 a clock per SM, a wide multiply at 32.
+constexpr uint64_t kS52PrimeMin = 1ull << 40, kS52PrimeLimit = 1ull << 52;
+constexpr uint32_t kMask26 = (1u << 26) - 1;
+
+__device__ __forceinline__ uint2 split26(uint64_t a) { return make_uint2((uint32_t)a & kMask26, (uint32_t)(a >> 26)); }
+
+template <bool S52>
+struct Acc {
+    u128 v{0, 0};
+    __device__ __forceinline__ void add(uint64_t a, uint64_t b) { mac(v, a, b); }
+    __device__ __forceinline__ uint64_t reduce(const PrimeConst &p) const { return barrett(v, p); }
+};
+
+template <>
+struct Acc<true> {
+    uint64_t lo = 0, mid = 0, hi = 0;
+    __device__ __forceinline__ void add(uint2 a, uint2 b) {
+        lo += (uint64_t)a.x * b.x;
+        mid += (uint64_t)a.x * b.y;
+        mid += (uint64_t)a.y * b.x;
+        hi += (uint64_t)a.y * b.y;
+    }
+    __device__ __forceinline__ void add(uint64_t a, uint64_t b) { add(split26(a), split26(b)); }
+    __device__ __forceinline__ uint64_t reduce(const PrimeConst &p) const {
+        const double two52 = 4503599627370496.0, magic = 6755399441055744.0, k = __dmul_rn(67108864.0, p.qinv);
+        const uint64_t q1 =
+            (uint64_t)__double_as_longlong(__fma_rn(__ull2double_rn(hi), k, two52)) & 0x000FFFFFFFFFFFFFull;
+        const uint64_t m = (hi << 26) - q1 * p.q + mid + (lo >> 26);  // as a signed value
+        const uint64_t q2 = (uint64_t)__double_as_longlong(__fma_rn(__ll2double_rn((long long)m), k, magic)) -
+                            0x4338000000000000ull;
+        const uint64_t r = (m << 26) + (lo & kMask26) - q2 * p.q;
+        return r + ((uint64_t)((int64_t)r >> 63) & p.q);
+    }
+};
+
+// an operand as the accumulator takes it
+template <bool S52>
+struct Operand {
+    using type = uint64_t;
+    __device__ __forceinline__ static type of(uint64_t a) { return a; }
+};
+template <>
+struct Operand<true> {
+    using type = uint2;
+    __device__ __forceinline__ static type of(uint64_t a) { return split26(a); }
+};
 
 __device__ __forceinline__ uint64_t mul_mod(uint64_t a, uint64_t b, const PrimeConst &p) {
     return barrett(mul_wide(a, b), p);

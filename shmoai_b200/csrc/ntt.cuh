@@ -78,7 +78,7 @@ struct ModDownIO {
     const uint64_t *vs = nullptr;  // [slots][16]
     long long out_ct = 0, out_h = 0, add_ct = 0, add_h = 0;  // word strides
     uint32_t H = 2, np = 0, n_add = 0, n_perm = 0;
-    int s52 = 0;  // every prime below 2^52: Acc<true>
+    int s52 = 0;  // Context::s52: Acc<true>
     const uint8_t *bytes = nullptr;  // the conversion's (and v's) constants for ConvIO; null: the load transform
 };
 
@@ -224,6 +224,32 @@ __device__ __forceinline__ uint64_t dbl_canon(double v, double q) {
 __device__ __forceinline__ uint64_t dbl_mod(double v, double q, double qinv) {
     return dbl_canon(dbl_centre(v, q, qinv), q);
 }
+
+// Sum of up to eight products of centred residues (to_dbl_centred) of a prime below 2^51, on the FP64 pipe.
+// H starts at 1.5 2^103, where doubles are multiples of 2^51: H' = H + a b rounded, the step H' - H is exact,
+// and so is the rest a b - (H' - H) (an integer, at most 2^50), which goes to L.  Two chains of four
+// products (each below 2^100) keep H inside [2^103, 2^104) and L below 2^53 in all.  At the end
+// h = H - 1.5 2^103 (both chains: 2^51 times an integer below 2^52) is taken mod q as a product with
+// 2^51 mod q and L is centred.  Four operations a term on a pipe that takes 64 a clock per SM; as 32-bit
+// halves a term is four wide multiply-adds at 32 a clock.
+constexpr int kMaxDblTerms = 8;
+constexpr double kTwo103 = 10141204801825835211973625643008.0;  // 2^103
+struct AccDbl {
+    double H[2] = {1.5 * kTwo103, 1.5 * kTwo103}, L[2] = {0.0, 0.0};
+    __device__ __forceinline__ void add(int i, double a, double b) {  // term i
+        const double h = __fma_rn(a, b, H[i & 1]);
+        L[i & 1] = __dadd_rn(L[i & 1], __fma_rn(a, b, __dsub_rn(H[i & 1], h)));
+        H[i & 1] = h;
+    }
+    // c = 2^51 mod q within q/2 + 1 of zero, times 2^-51
+    __device__ __forceinline__ uint64_t reduce(double q, double qinv, double c) const {
+        const double h = __dadd_rn(__dsub_rn(H[0], 1.5 * kTwo103), __dsub_rn(H[1], 1.5 * kTwo103));
+        return dbl_mod(__dadd_rn(mul_dbl(h, c, q, qinv), dbl_centre(__dadd_rn(L[0], L[1]), q, qinv)), q, qinv);
+    }
+    __device__ __forceinline__ static double two51_mod(double q, double qinv) {
+        return __dmul_rn(dbl_centre(2251799813685248.0, q, qinv), 1.0 / 2251799813685248.0);
+    }
+};
 
 __device__ __forceinline__ void gs_bf(uint64_t &x, uint64_t &y, uint64_t w, uint64_t ws, uint64_t q) {
     uint64_t q2 = 2 * q;

@@ -58,7 +58,7 @@ __device__ __forceinline__ uint64_t conv_sum(const uint64_t *__restrict__ x, con
     for (uint32_t i = 0; i < kBatch; i++)
         if (i < n) acc.add(v[i], c[i]);
     for (uint32_t i = kBatch; i < n; i++) acc.add(x[(size_t)i << log_n], c[i]);
-    return barrett(acc.get(), p);
+    return acc.reduce(p);
 }
 
 // CTAs are issued limb-major: consecutive CTAs work on the same slot (one prime) of successive

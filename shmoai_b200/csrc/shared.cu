@@ -17,6 +17,7 @@
 //   FmtSwitch backward (FmtSwitch.cu:396-429): n ordinary key switches of the
 //     shared a from s'_i to s, hoisted: one ModUp(a), per member one inner product
 //     with its key [dnum][2][QP][N], ModDown, combine with b_i.
+#include <atomic>
 #include <mutex>
 
 #include "core.hpp"
@@ -32,49 +33,63 @@ constexpr int kMaxB = 16;
 // acc[ct][h][j][k] = sum_b up[ct][b][j][perm(k)] * key[b][h][prime(j)][k], h < H (limb j of digit j / np
 // from own, when given).
 // A block handles `chunk` groups: each thread stages its own extended-digit words of those
-// groups in shared memory (a column per thread, so no synchronisation), then, half by
-// half, holds the key digits in registers and serves every group of the chunk: the key
-// (n + 1 halves of dnum x QP limbs, far larger than L2 at the top level) is read once per
-// chunk instead of once per group.
+// groups in shared memory, as the accumulator takes them (a column per thread, so no
+// synchronisation), then, half by half, holds the key digits in registers (the next half's loads
+// in flight) and serves every group of the chunk: the key (n + 1 halves of dnum x QP limbs, far
+// larger than L2 at the top level) is read once per chunk instead of once per group.  B = beta at
+// compile time: with a loop bounded by the largest digit count and guarded, a block issued the guarded
+// iterations too (41 instructions per term; four groups of eight at 35 limbs 1.06 ms, 0.41 ms of it DRAM).
 constexpr int kIpT = 128;
 constexpr size_t kIpSmemMax = 96 * 1024;  // largest chunk the autotuner may pick
 
-template <bool S52>
+template <int B, int A>
 __global__ void __launch_bounds__(kIpT) ip_multi_kernel(const uint64_t *__restrict__ up, OwnLimbs own,
                                                         const uint64_t *__restrict__ key, uint64_t *__restrict__ acc,
                                                         uint32_t n_cts, uint32_t chunk, uint32_t L, uint32_t np,
-                                                        uint32_t nq, uint32_t beta, uint32_t H, uint32_t log_n,
+                                                        uint32_t nq, uint32_t H, uint32_t log_n,
                                                         const PrimeConst *__restrict__ pc,
                                                         const uint32_t *__restrict__ perm) {
-    extern __shared__ uint64_t su[];  // [chunk * beta][kIpT]
+    using I = IpSum<A>;
+    using T = typename I::T;
+    extern __shared__ uint64_t smem[];
+    T *su = reinterpret_cast<T *>(smem) + threadIdx.x;  // [chunk * B][kIpT]
     const uint32_t j = blockIdx.y;
     const uint32_t k = blockIdx.x * kIpT + threadIdx.x;
     const uint32_t ks = perm ? __ldg(perm + k) : k;
     const size_t n = (size_t)1 << log_n;
     const uint32_t LP = L + np, QP = nq + np;
     const uint32_t pj = j < L ? j : nq + (j - L);
-    const PrimeConst p = pc[pj];
+    const I ip(pc[pj]);
     const uint32_t c0 = blockIdx.z * chunk, nc = min(chunk, n_cts - c0);
-    const uint32_t ob = own.p && j < L ? j / np : beta;
+    const uint32_t ob = own.p && j < L ? j / np : B;
+    const uint64_t *kp = key + (size_t)pj * n + k;
+    uint64_t next[B];
+#pragma unroll
+    for (int b = 0; b < B; b++) next[b] = __ldg(kp + (size_t)b * H * QP * n);
     for (uint32_t ct = 0; ct < nc; ct++) {
-        const uint64_t *up_c = up + (size_t)(c0 + ct) * beta * LP * n + (size_t)j * n + ks;
+        const uint64_t *up_c = up + (size_t)(c0 + ct) * B * LP * n + (size_t)j * n + ks;
         const uint64_t *own_c = own.p + (c0 + ct) * own.stride + (size_t)j * n + ks;
-        for (uint32_t b = 0; b < beta; b++)
-            su[(ct * beta + b) * kIpT + threadIdx.x] = *(b == ob ? own_c : up_c + (size_t)b * LP * n);
+        uint64_t v[B];
+#pragma unroll
+        for (int b = 0; b < B; b++) v[b] = *((uint32_t)b == ob ? own_c : up_c + (size_t)b * LP * n);
+#pragma unroll
+        for (int b = 0; b < B; b++) su[(ct * B + b) * kIpT] = ip.operand(v[b]);
     }
-    for (uint32_t h = 0; h < H; h++) {
-        uint64_t kk[kMaxB];
-        const uint64_t *kp = key + ((size_t)h * QP + pj) * n + k;
+    uint64_t *out = acc + (((size_t)c0 * H) * LP + j) * n + k;
+    for (uint32_t h = 0; h < H; h++, out += (size_t)LP * n) {
+        T kk[B];
 #pragma unroll
-        for (int b = 0; b < kMaxB; b++)
-            if (b < (int)beta) kk[b] = __ldg(kp + (size_t)b * H * QP * n);
+        for (int b = 0; b < B; b++) kk[b] = ip.operand(next[b]);
+        if (h + 1 < H) {
+            kp += (size_t)QP * n;
+#pragma unroll
+            for (int b = 0; b < B; b++) next[b] = __ldg(kp + (size_t)b * H * QP * n);
+        }
         for (uint32_t ct = 0; ct < nc; ct++) {
-            Acc<S52> a;
-            const uint64_t *s = su + ct * beta * kIpT + threadIdx.x;
+            typename I::Acc a;
 #pragma unroll
-            for (int b = 0; b < kMaxB; b++)
-                if (b < (int)beta) a.add(s[b * kIpT], kk[b]);
-            acc[(((size_t)(c0 + ct) * H + h) * LP + j) * n + k] = barrett(a.get(), p);
+            for (int b = 0; b < B; b++) ip.add(a, b, su[(ct * B + b) * kIpT], kk[b]);
+            out[(size_t)ct * H * LP * n] = ip.reduce(a);
         }
     }
 }
@@ -171,25 +186,24 @@ ExtConsts ext_consts(Context &c, uint32_t L) {
 
 // The Sh-Rot / FmtSwitch inner products: groups are served in chunks that fit
 // c.ip_chunk_bytes of shared memory, each chunk reading the key once.
-void ip_multi(const Context &c, const uint64_t *up, OwnLimbs own, const uint64_t *key, uint64_t *acc, uint32_t n_cts, uint32_t L,
-              uint32_t beta, uint32_t H, const uint32_t *perm, cudaStream_t st) {
-    static std::once_flag attr;
-    std::call_once(attr, [] {
-        for (const void *f : {(const void *)ip_multi_kernel<true>, (const void *)ip_multi_kernel<false>})
-            SHM_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kIpSmemMax));
-    });
-    const uint32_t np = c.np, LP = L + np;
+void ip_multi(const Context &c, const uint64_t *up, OwnLimbs own, const uint64_t *key, uint64_t *acc, uint32_t n_cts,
+              uint32_t L, uint32_t beta, uint32_t H, const uint32_t *perm, cudaStream_t st) {
+    const uint32_t LP = L + c.np;
     const size_t cap = std::min<size_t>(c.ip_chunk_bytes, kIpSmemMax);
     const uint32_t chunk = std::max<uint32_t>(1, std::min<uint32_t>(n_cts, (uint32_t)(cap / (beta * kIpT * 8))));
     const dim3 grid(c.n / kIpT, LP, (n_cts + chunk - 1) / chunk);
     const size_t smem = (size_t)chunk * beta * kIpT * 8;
     SHM_LAUNCHED(1);
-    if (c.s52)
-        ip_multi_kernel<true><<<grid, kIpT, smem, st>>>(up, own, key, acc, n_cts, chunk, L, np, c.nq, beta, H, c.log_n,
-                                                        c.pc, perm);
-    else
-        ip_multi_kernel<false><<<grid, kIpT, smem, st>>>(up, own, key, acc, n_cts, chunk, L, np, c.nq, beta, H, c.log_n,
-                                                         c.pc, perm);
+    ip_dispatch(c, beta, [&](auto b, auto a) {
+        const auto f = ip_multi_kernel<decltype(b)::value, decltype(a)::value>;
+        static std::atomic<uint64_t> ready{0};  // a bit per device: the attribute belongs to the device's module
+        const uint64_t bit = 1ull << (c.device & 63);
+        if (!(ready.load(std::memory_order_acquire) & bit)) {
+            SHM_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kIpSmemMax));
+            ready.fetch_or(bit, std::memory_order_release);
+        }
+        f<<<grid, kIpT, smem, st>>>(up, own, key, acc, n_cts, chunk, L, c.np, c.nq, H, c.log_n, c.pc, perm);
+    });
     SHM_CUDA(cudaGetLastError());
 }
 
