@@ -151,7 +151,10 @@ __global__ void __launch_bounds__(Geo<R, S>::THREADS, MINB)
 
 // ---------------- forward, phase 2: blocks (global stages LOGM .. 2*LOGM-1), fully reduced output
 // IOK = kIoRescale: instead of storing t = NTT(...) of row (poly, j), write (c_j - t) q_last^-1
-// to io.rs.out; kIoModDown: write (acc_j - t) P^-1 (+ add) to io.md.out
+// to io.rs.out; kIoModDown: write (acc_j - t) P^-1 (+ add) to io.md.out.  The words that the store
+// combines are asked for (into L2) before the transform and read before its last barrier, and on the FP64
+// rows t stays a double: the combination is one more twiddle-like product (27 limbs of 16 polynomials, ModDown:
+// 0.294 ms with loads after the barrier and Shoup products, 0.189 ms so; rescale 0.189 and 0.129 ms).
 template <int R, int S, int MINB, int IOK, int FAM>
 __global__ void __launch_bounds__(Geo<R, S>::THREADS, MINB)
     fwd_blk(uint64_t *__restrict__ data, NttRows rw, const uint64_t *__restrict__ tw, const double *__restrict__ twd,
@@ -170,6 +173,39 @@ __global__ void __launch_bounds__(Geo<R, S>::THREADS, MINB)
     uint64_t *x = xc + (size_t)sig * G::M;
     uint64_t *s = sm + sig * G::PAD_M;
 
+    // where the store reads and writes: out = (in - t) mul (+ add[perm] add_mul)
+    const size_t off = (size_t)chunk * S * G::M;
+    const uint64_t *cin = nullptr, *mul = nullptr, *ad = nullptr, *amul = nullptr;
+    const uint32_t *perm = nullptr;
+    uint64_t *o = xc;
+    if constexpr (IOK == kIoRescale) {
+        cin = io.rs.in + (((size_t)poly * (rw.slots + 1) + slot) << G::LOGN) + off;
+        o = io.rs.out + ((size_t)row << G::LOGN) + off;
+        mul = io.rs.inv + 2 * slot;
+    } else if constexpr (IOK == kIoModDown) {
+        const ModDownIO &md = io.md;
+        const uint32_t ct = poly / md.H, h = poly % md.H;
+        cin = md.acc + (((size_t)poly * (rw.slots + md.np) + slot) << G::LOGN) + off;
+        o = md.out + ct * md.out_ct + h * md.out_h + ((size_t)slot << G::LOGN) + off;
+        mul = md.pinv + 2 * slot;
+        if (h < md.n_add) {
+            ad = md.add + ct * md.add_ct + h * md.add_h + ((size_t)slot << G::LOGN);
+            if (h < md.n_perm && md.perm) perm = md.perm + off;
+            if (md.add_mul) amul = md.add_mul + 2 * slot;
+        }
+    }
+    if constexpr (IOK != kIoPlain) {
+        constexpr uint32_t LINES = S * G::M / 16;  // 128-byte lines of the tile
+        if (threadIdx.x < LINES) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(cin + 16 * threadIdx.x));
+            if (ad) {  // an automorphism maps aligned blocks of 32 words onto such blocks
+                const size_t at = perm ? (__ldg(perm + (threadIdx.x / 2) * 32) & ~31u) + (threadIdx.x & 1) * 16
+                                       : off + 16 * threadIdx.x;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(ad + at));
+            }
+        }
+    }
+
     uint64_t a[G::E];
 #pragma unroll
     for (int m = 0; m < G::E; m++) a[m] = x[lane + m * G::E];
@@ -181,9 +217,17 @@ __global__ void __launch_bounds__(Geo<R, S>::THREADS, MINB)
     for (int m = 0; m < G::E; m++) a[m] = s[padded(lane * G::E + m)];
     fwd_pass<R, FAM, true>(lb.mode, a, TwLane<R>(lb.t, b, lane), lb.qd, lb.qinv, lb.w, lb.ws,
                            ((G::M + b) << R) + lane, lb.q);
-    if (fam_fp(FAM) && (!fam_int(FAM) || lb.fp())) {
+    const bool fp = fam_fp(FAM) && (!fam_int(FAM) || lb.fp());
+    if (fp) {
+        if constexpr (IOK == kIoPlain) {
 #pragma unroll
-        for (int m = 0; m < G::E; m++) s[padded(lane * G::E + m)] = dbl_mod(as_dbl(a[m]), lb.qd, lb.qinv);
+            for (int m = 0; m < G::E; m++) s[padded(lane * G::E + m)] = dbl_mod(as_dbl(a[m]), lb.qd, lb.qinv);
+        } else {  // |t| < 11 q (kBfF64), centred (kBfF64R): in - t stays inside mul_dbl's range
+#pragma unroll
+            for (int m = 0; m < G::E; m++)
+                s[padded(lane * G::E + m)] =
+                    lb.mode == kBfF64 ? a[m] : as_bits(dbl_centre(as_dbl(a[m]), lb.qd, lb.qinv));
+        }
     } else if (fam_has(FAM, kBfGrow) && lb.mode == kBfGrow) {
         const PrimeConst p = pc[pidx];
 #pragma unroll
@@ -193,52 +237,49 @@ __global__ void __launch_bounds__(Geo<R, S>::THREADS, MINB)
 #pragma unroll
         for (int m = 0; m < G::E; m++) s[padded(lane * G::E + m)] = csub(csub(a[m], q2), lb.q);
     }
-    __syncthreads();
-    const uint64_t q = lb.q;
-    const size_t off = (size_t)chunk * S * G::M;
-    if constexpr (IOK == kIoRescale) {
-        const uint64_t *cin = io.rs.in + (((size_t)poly * (rw.slots + 1) + slot) << G::LOGN) + off;
-        uint64_t *o = io.rs.out + ((size_t)row << G::LOGN) + off;
-        const uint64_t iw = io.rs.inv[2 * slot], iws = io.rs.inv[2 * slot + 1];
+    auto at = [&](int i) { return threadIdx.x + i * G::THREADS; };
+    auto result = [&](int i) { return sm[(at(i) / G::M) * G::PAD_M + padded(at(i) % G::M)]; };
+    if constexpr (IOK == kIoPlain) {
+        __syncthreads();
 #pragma unroll
-        for (int i = 0; i < G::E; i++) {
-            uint32_t e = threadIdx.x + i * G::THREADS;
-            const uint64_t t = sm[(e / G::M) * G::PAD_M + padded(e % G::M)];
-            o[e] = shoup(sub_mod(cin[e], t, q), iw, iws, q);
-        }
-    } else if constexpr (IOK == kIoModDown) {
-        const ModDownIO &md = io.md;
-        const uint32_t j = slot, ct = poly / md.H, h = poly % md.H;
-        const uint64_t *ain = md.acc + (((size_t)poly * (rw.slots + md.np) + j) << G::LOGN) + off;
-        uint64_t *o = md.out + ct * md.out_ct + h * md.out_h + ((size_t)j << G::LOGN) + off;
-        const uint64_t iw = md.pinv[2 * j], iws = md.pinv[2 * j + 1];
-        const bool add = h < md.n_add, perm = add && h < md.n_perm && md.perm;
-        const uint64_t *ad = add ? md.add + ct * md.add_ct + h * md.add_h + ((size_t)j << G::LOGN) : nullptr;
-        if (md.add_mul) {
-            const uint64_t mw = md.add_mul[2 * j], mws = md.add_mul[2 * j + 1];
+        for (int i = 0; i < G::E; i++) xc[at(i)] = result(i);
+    } else {
+        const uint64_t q = lb.q;
+        uint64_t v[G::E];
 #pragma unroll
-            for (int i = 0; i < G::E; i++) {
-                uint32_t e = threadIdx.x + i * G::THREADS;
-                const uint64_t t = sm[(e / G::M) * G::PAD_M + padded(e % G::M)];
-                uint64_t r = shoup(sub_mod(ain[e], t, q), iw, iws, q);
-                if (add) r = add_mod(r, shoup(ad[perm ? __ldg(md.perm + off + e) : off + e], mw, mws, q), q);
-                o[e] = r;
+        for (int i = 0; i < G::E; i++) v[i] = cin[at(i)];
+        __syncthreads();
+        if (fp) {
+            const double w = to_dbl_centred(mul[0], q);
+#pragma unroll
+            for (int i = 0; i < G::E; i++)
+                v[i] = as_bits(mul_dbl(__dsub_rn(to_dbl(v[i]), as_dbl(result(i))), w, lb.qd, lb.qinv));
+            if (!ad) {
+#pragma unroll
+                for (int i = 0; i < G::E; i++) o[at(i)] = dbl_canon(as_dbl(v[i]), lb.qd);
+            } else if (amul) {
+                const double aw = to_dbl_centred(amul[0], q);
+#pragma unroll
+                for (int i = 0; i < G::E; i++) {
+                    const double u = mul_dbl(to_dbl(ad[perm ? __ldg(perm + at(i)) : off + at(i)]), aw, lb.qd, lb.qinv);
+                    o[at(i)] = dbl_mod(__dadd_rn(as_dbl(v[i]), u), lb.qd, lb.qinv);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < G::E; i++)
+                    o[at(i)] = add_mod(dbl_canon(as_dbl(v[i]), lb.qd), ad[perm ? __ldg(perm + at(i)) : off + at(i)], q);
             }
         } else {
+            const uint64_t w = mul[0], ws = mul[1], aw = amul ? amul[0] : 0, aws = amul ? amul[1] : 0;
 #pragma unroll
             for (int i = 0; i < G::E; i++) {
-                uint32_t e = threadIdx.x + i * G::THREADS;
-                const uint64_t t = sm[(e / G::M) * G::PAD_M + padded(e % G::M)];
-                uint64_t r = shoup(sub_mod(ain[e], t, q), iw, iws, q);
-                if (add) r = add_mod(r, ad[perm ? __ldg(md.perm + off + e) : off + e], q);
-                o[e] = r;
+                uint64_t r = shoup(sub_mod(v[i], result(i), q), w, ws, q);
+                if (ad) {
+                    const uint64_t u = ad[perm ? __ldg(perm + at(i)) : off + at(i)];
+                    r = add_mod(r, amul ? shoup(u, aw, aws, q) : u, q);
+                }
+                o[at(i)] = r;
             }
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < G::E; i++) {
-            uint32_t e = threadIdx.x + i * G::THREADS;
-            xc[e] = sm[(e / G::M) * G::PAD_M + padded(e % G::M)];
         }
     }
 }
