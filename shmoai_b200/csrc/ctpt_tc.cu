@@ -53,8 +53,9 @@ struct ModTab {
     uint32_t c24[kMaxMods];  // 2^20 mod m_t
     uint32_t c48[kMaxMods];  // 2^40 mod m_t
     uint32_t magic[kMaxMods];  // ceil(2^32 / m_t)
+    int rnd[kMaxMods];         // round(2^32 / m_t)
+    uint32_t vbase[kMaxMods + 1];  // [T]: the CRT's v before the residues (crt_kernel)
     double inv[kMaxMods];    // 1 / m_t
-    float invf[kMaxMods];
 };
 
 __constant__ ModTab c_mods;
@@ -73,23 +74,24 @@ __device__ __forceinline__ uint32_t mod_small(uint64_t x, uint32_t t) {
     return (uint32_t)(r < 0 ? r + (int)m : r);
 }
 
-// a mod m_t in [0, m_t) for any int32 accumulator: a + m * 2^24 (a multiple of m above
-// 2^31, the moduli being > 128) is non-negative and below 2^33, then the 32-bit fold above
-// a mod m_t for |a| < 2^24 (every accumulator: n_in * 125^2 < 2^24 up to n_in = 1073): a is
-// exact in float, floor(a / m) from one float multiply is off by at most one (relative error
-// ~2^-24 of a quotient below 2^17), and two conditional corrections finish it
-__device__ __forceinline__ uint32_t mod_acc24(int a, uint32_t t) {
-    const int m = (int)c_mods.m[t];
-    const int q = __float2int_rd((float)a * c_mods.invf[t]);
-    int r = a - q * m;
-    r += r < 0 ? m : 0;
-    r -= r >= m ? m : 0;
-    return (uint32_t)r;
+// The residue planes of the products hold a balanced residue of S mod m_t plus 128, a byte.
+//
+// An accumulator's residue in [-127, 127] for |a| <= kAccSmall (n_in up to 4,160 inputs): q = round(a / m)
+// from one wide multiply-add with round(2^32 / m) (|q - a / m| <= 1/2 + |a| 2^-33), so |a - q m| <= m / 2 +
+// m |a| 2^-33 < 127.5 with no correction; its low byte is the residue.  Two operations an accumulator and
+// none on the conversion pipe: an int -> float -> int quotient (16 conversions a clock per SM) held a 128 x 256
+// tile's epilogue to 2.1 us at least, the tile's MMAs at K = 768 to 1.6 us.
+constexpr uint64_t kAccSmall = 65000000;
+__device__ __forceinline__ uint32_t acc_residue(int a, int rnd, uint32_t m) {
+    const int64_t p = (int64_t)a * rnd + 0x80000000ll;
+    return (uint32_t)a - (uint32_t)(p >> 32) * m;
 }
 
-__device__ __forceinline__ uint32_t mod_acc(int a, uint32_t t) {
-    const uint64_t x = (uint64_t)((int64_t)a + ((int64_t)c_mods.m[t] << 24));
-    return mod_small(x, t);
+// any int32 accumulator: a + m * 2^24 (a multiple of m above 2^31, the moduli being > 128) is
+// non-negative and below 2^33, then the 32-bit fold above
+__device__ __forceinline__ uint32_t acc_residue_any(int a, uint32_t t) {
+    const uint32_t r = mod_small((uint64_t)((int64_t)a + ((int64_t)c_mods.m[t] << 24)), t);
+    return (uint32_t)(int)balanced(r, c_mods.m[t]);
 }
 
 // The balanced residue of x mod m_t (in (-m/2, m/2), m odd) for x < 2^51 given as the exact double
@@ -107,6 +109,21 @@ __device__ __forceinline__ uint32_t balanced_f64(double xd, uint32_t xlo, uint32
 // the low bytes of four words as one word
 __device__ __forceinline__ uint32_t pack_low_bytes(uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3) {
     return __byte_perm(__byte_perm(b0, b1, 0x0040), __byte_perm(b2, b3, 0x0040), 0x5410);
+}
+
+// four accumulators as four bytes of the plane
+__device__ __forceinline__ uint32_t acc_bytes(const uint32_t *v, uint32_t t, int small) {
+    uint32_t r[4];
+    if (small) {
+        const int rnd = c_mods.rnd[t];
+        const uint32_t m = c_mods.m[t];
+#pragma unroll
+        for (int b = 0; b < 4; b++) r[b] = acc_residue((int)v[b], rnd, m);
+    } else {
+#pragma unroll
+        for (int b = 0; b < 4; b++) r[b] = acc_residue_any((int)v[b], t);
+    }
+    return pack_low_bytes(r[0], r[1], r[2], r[3]) ^ 0x80808080u;
 }
 
 // X [n_in][R] (uint64) -> XP [t][R][Kp] (int8), via 64 x 64 shared-memory transposes.  A block
@@ -236,7 +253,7 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
 __global__ void __launch_bounds__(kThreads, 2) mma_kernel(const int8_t *__restrict__ XP, const int8_t *__restrict__ WP,
                                                           uint8_t *__restrict__ RES, uint32_t Kp, uint32_t Np,
                                                           uint32_t n_out, uint64_t chunk, int *__restrict__ err,
-                                                          int acc24) {
+                                                          int acc_small) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], done;
     __shared__ uint32_t tmem_base;
@@ -355,13 +372,7 @@ __global__ void __launch_bounds__(kThreads, 2) mma_kernel(const int8_t *__restri
             if (o < n_out) {
                 uint32_t pk[8];
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    uint32_t w = 0;
-#pragma unroll
-                    for (int b = 0; b < 4; b++)
-                        w |= (acc24 ? mod_acc24((int)v[4 * j + b], t) : mod_acc((int)v[4 * j + b], t)) << (8 * b);
-                    pk[j] = w;
-                }
+                for (int j = 0; j < 8; j++) pk[j] = acc_bytes(v + 4 * j, t, acc_small);
                 uint4 *dst = reinterpret_cast<uint4 *>(RES + ((uint64_t)t * n_out + o) * chunk + rbase + c0);
                 dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                 dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
@@ -389,6 +400,7 @@ __global__ void __launch_bounds__(kThreads, 2) mma_kernel(const int8_t *__restri
 constexpr uint32_t kResKp = 768;
 constexpr int kAStages = 4;  // one ring slot per producer warp
 constexpr uint32_t kXBlock = kBN * kKB;  // 16 KB
+constexpr uint32_t kXTiles = 6;          // most X tiles held at a time
 constexpr uint32_t kSmemP = (kResKp / kKB) * kXBlock + kAStages * kStageA + 1024;
 constexpr uint32_t kEpiWarp0 = 5;
 constexpr uint32_t kThreadsP = (kEpiWarp0 + 8) * 32;
@@ -400,18 +412,22 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
                                                                       const int8_t *__restrict__ WP,
                                                                       uint8_t *__restrict__ RES, uint32_t Kp,
                                                                       uint32_t Np, uint32_t n_out, uint64_t chunk,
-                                                                      uint32_t T, int *__restrict__ err, int acc24,
+                                                                      uint32_t T, int *__restrict__ err, int acc_small,
                                                                       const __grid_constant__ CUtensorMap tmA,
                                                                       const __grid_constant__ CUtensorMap tmX) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);  // swizzle atoms need 1 KB alignment
-    __shared__ __align__(8) uint64_t full[kAStages], empty[kAStages], x_full, x_empty, acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t full[kAStages], empty[kAStages], x_full[kXTiles], x_empty[kXTiles], acc_full[2],
+        acc_empty[2];
     __shared__ uint32_t tmem_base;
     __shared__ int failed;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t *sX = smem, *sA = smem + (kResKp / kKB) * kXBlock;
     const uint32_t nkb = Kp / kKB, n_ot = Np / kBM;
     const uint64_t n_ct = chunk / kBN, n_tiles = (uint64_t)T * n_ct;
+    // X tiles held: tile i of this CTA in slot i % ns.  At K = 768 one fits; small K (where a tile's load, MMAs and
+    // epilogue came one after another: 4.7 us per tile of 128 inputs) has the next ones loaded ahead.
+    const uint32_t ns = min(kXTiles, kResKp / Kp);
     constexpr uint32_t kProducers = 128, kEpi = 256;
 
     if (warp == 0) {
@@ -425,8 +441,11 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&full[s])), "r"(TMA_A ? 1 : 32));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&empty[s])));
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&x_full)), "r"(TMA_A ? 1 : kProducers));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&x_empty)));
+        for (uint32_t x = 0; x < kXTiles; x++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&x_full[x])),
+                         "r"(TMA_A ? 1 : kProducers));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&x_empty[x])));
+        }
         for (int b = 0; b < 2; b++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&acc_full[b])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&acc_empty[b])), "r"(kEpi));
@@ -447,46 +466,53 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
         // TMA: thread 0 issues every load (the X tile as Kp / 64 boxes of 256 rows, then the A
         // stages), its warp prefetches the next X tile into L2
         bool ok = true;
-        uint64_t g = 0;   // A stages so far (ring position)
+        uint32_t g = 0;   // A stages so far (ring position)
         uint32_t ti = 0;  // column tiles of this CTA so far
+        uint32_t xi = 0;  // X tiles asked for so far (TMA)
         const uint32_t kx16 = Kp / 16;
+        // every MMA of the slot's previous tile must have read it
+        auto x_free = [&](uint32_t i) {
+            return i < ns || mbar_wait(smem_u32(&x_empty[i % ns]), (i / ns - 1) & 1);
+        };
         for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ti++) {
             const uint32_t t = (uint32_t)(tile / n_ct);
             const uint64_t rbase = (tile % n_ct) * kBN;
             if constexpr (TMA_A) {
-                if (tid == 0) {
-                    // every MMA of the previous column tile must have read the X tile
-                    if (ok && ti > 0 && !mbar_wait(smem_u32(&x_empty), (ti - 1) & 1)) ok = false;
-                    const uint32_t bar = smem_u32(&x_full);
-                    if (ok) {
-                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar),
-                                     "r"(kBN * Kp));
-                        for (uint32_t kb = 0; kb < nkb; kb++)  // x = kb * 64 bytes: 16-byte aligned
-                            asm volatile(
-                                "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-                                "[%0], [%1, {%2, %3}], [%4];\n" ::"r"(smem_u32(sX + kb * kXBlock)),
-                                "l"(reinterpret_cast<uint64_t>(&tmX)), "r"((int)(kb * kKB)),
-                                "r"((int)((uint64_t)t * chunk + rbase)), "r"(bar)
-                                : "memory");
-                    } else {
-                        arrive(bar);
+                // ahead of this tile's weights: the X tiles whose slots' last readers came two tiles ago
+                if (tid == 0)
+                    for (; xi <= (ns > 1 ? ti + ns - 2 : ti); xi++) {
+                        const uint64_t xt = blockIdx.x + (uint64_t)xi * gridDim.x;
+                        if (xt >= n_tiles) break;
+                        if (ok && !x_free(xi)) ok = false;
+                        const uint32_t bar = smem_u32(&x_full[xi % ns]);
+                        if (ok) {
+                            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar),
+                                         "r"(kBN * Kp));
+                            for (uint32_t kb = 0; kb < nkb; kb++)  // x = kb * 64 bytes: 16-byte aligned
+                                asm volatile(
+                                    "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+                                    "[%0], [%1, {%2, %3}], [%4];\n" ::"r"(smem_u32(sX + (xi % ns * nkb + kb) * kXBlock)),
+                                    "l"(reinterpret_cast<uint64_t>(&tmX)), "r"((int)(kb * kKB)),
+                                    "r"((int)((xt / n_ct) * chunk + (xt % n_ct) * kBN)), "r"(bar)
+                                    : "memory");
+                        } else {
+                            arrive(bar);
+                        }
                     }
-                }
                 __syncwarp();
             } else {
-                // every MMA of the previous column tile must have read the X tile
-                if (ok && ti > 0 && !mbar_wait(smem_u32(&x_empty), (ti - 1) & 1)) ok = false;
+                if (ok && !x_free(ti)) ok = false;
                 const int8_t *B = XP + ((uint64_t)t * chunk + rbase) * Kp;
                 if (ok)
                     for (uint32_t c = tid; c < kBN * kx16; c += kProducers) {
                         const uint32_t row = c / kx16, k16 = c % kx16;
-                        cp_async16(smem_u32(sX + (k16 >> 2) * kXBlock) + core_off(row, k16 & 3),
+                        cp_async16(smem_u32(sX + (ti % ns * nkb + (k16 >> 2)) * kXBlock) + core_off(row, k16 & 3),
                                    B + (uint64_t)row * Kp + k16 * 16);
                     }
                 asm volatile("cp.async.commit_group;\n");
                 asm volatile("cp.async.wait_group 0;\n");
                 asm volatile("fence.proxy.async.shared::cta;\n");
-                arrive(smem_u32(&x_full));
+                arrive(smem_u32(&x_full[ti % ns]));
             }
             // the next column tile's X into L2 while this one's MMAs run
             const uint64_t next = tile + gridDim.x;
@@ -502,7 +528,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
                     const uint32_t s = (uint32_t)(g % kAStages);
                     if constexpr (TMA_A) {
                         if (tid != 0) continue;
-                        if (ok && g >= (uint64_t)kAStages && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((g / kAStages) - 1) & 1))
+                        if (ok && g >= (uint32_t)kAStages && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((g / kAStages) - 1) & 1))
                             ok = false;
                         const uint32_t bar = smem_u32(&full[s]);
                         if (ok) {
@@ -521,7 +547,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
                         continue;
                     }
                     if (s != warp) continue;
-                    if (ok && g >= (uint64_t)kAStages && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((g / kAStages) - 1) & 1))
+                    if (ok && g >= (uint32_t)kAStages && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((g / kAStages) - 1) & 1))
                         ok = false;
                     if (ok)
                         for (uint32_t c = lane; c < kBM * (kKB / 16); c += 32) {
@@ -539,10 +565,10 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
         if (!ok) failed = 1;
     } else if (tid == kProducers) {
         bool ok = true;
-        uint64_t g = 0;
-        uint32_t ti = 0, ai = 0;  // column tiles, accumulator tiles
+        uint32_t g = 0, ti = 0, ai = 0;  // A stages, column tiles, accumulator tiles
         for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ti++) {
-            if (ok && !mbar_wait(smem_u32(&x_full), ti & 1)) ok = false;
+            const uint32_t xs = ti % ns;
+            if (ok && !mbar_wait(smem_u32(&x_full[xs]), (ti / ns) & 1)) ok = false;
             asm volatile("tcgen05.fence::after_thread_sync;\n");
             for (uint32_t o = 0; o < n_ot; o++, ai++) {
                 const uint32_t buf = ai & 1;
@@ -553,7 +579,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
                     if (ok && !mbar_wait(smem_u32(&full[s]), (uint32_t)(g / kAStages) & 1)) ok = false;
                     asm volatile("tcgen05.fence::after_thread_sync;\n");
                     if (ok) {
-                        const uint32_t a0 = smem_u32(sA + s * kStageA), b0 = smem_u32(sX + kb * kXBlock);
+                        const uint32_t a0 = smem_u32(sA + s * kStageA), b0 = smem_u32(sX + (xs * nkb + kb) * kXBlock);
 #pragma unroll
                         for (uint32_t k = 0; k < kKB / 32; k++) {
                             const uint64_t ad = TMA_A ? smem_desc_sw64(a0 + k * 32) : smem_desc(a0 + k * 256);
@@ -573,7 +599,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
                     smem_u32(&acc_full[buf])));
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                smem_u32(&x_empty)));
+                smem_u32(&x_empty[xs])));
         }
         if (!ok) failed = 1;
     } else if (warp >= kEpiWarp0) {
@@ -606,14 +632,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
                         if (out < n_out) {
                             uint32_t pk[8];
 #pragma unroll
-                            for (int j = 0; j < 8; j++) {
-                                uint32_t w = 0;
-#pragma unroll
-                                for (int b = 0; b < 4; b++)
-                                    w |= (acc24 ? mod_acc24((int)v[4 * j + b], t) : mod_acc((int)v[4 * j + b], t))
-                                         << (8 * b);
-                                pk[j] = w;
-                            }
+                            for (int j = 0; j < 8; j++) pk[j] = acc_bytes(v + 4 * j, t, acc_small);
                             uint4 *dst = reinterpret_cast<uint4 *>(RES + ((uint64_t)t * n_out + out) * chunk + rbase + c0);
                             dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                             dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
@@ -637,12 +656,14 @@ struct CrtLimb {
     uint64_t c[kMaxMods];  // c_t mod q_l
     uint64_t M;            // M mod q_l
     uint64_t Mneg;         // q_l - (M mod q_l), below q_l
+    uint64_t base;         // 128 T M - 128 sum_t c_t mod q_l
 };
 
-// Fraction bits of the fixed-point CRT fractions F_t = round(2^19 [(M/m_t)^-1]_{m_t} / m_t): with
-// r_t < 251 and T <= 20, sum_t r_t F_t + 2^18 < 2^32, and the sum's rounding error
-// T 251 2^-20 < 0.005 keeps v = round(sum_t r_t frac_t) exact (M > 2.02 |S| leaves the true sum
-// within 0.495 of an integer).
+// Fraction bits of the fixed-point CRT fractions F_t = round(2^19 [(M/m_t)^-1]_{m_t} / m_t).  The planes hold
+// u_t = r_t + 128 with |r_t| <= 127, so v = round(sum_t r_t frac_t) is found as v + 128 T from
+// sum_t u_t F_t + vbase, vbase = 128 T 2^19 - 128 sum_t F_t + 2^18: non-negative and below 2^32 for T <= 20.
+// The rounding error T 128 2^-20 < 0.003 keeps v exact (M > 2.02 |S| leaves the true sum within 0.495 of
+// an integer).
 constexpr uint32_t kCrtFracBits = 19;
 
 // workspace bytes before the residue planes: the error flag, then the CRT tables for every
@@ -653,11 +674,12 @@ constexpr size_t kCrtTabBytes = 256 + sizeof(CrtLimb) * 64 * kMaxMods;
 // stores).  The host sizes the block so that its 4 blockDim.x columns lie in one limb: the limb's
 // constants (the 32-bit halves of c_t and the fixed-point fractions) are staged in shared memory
 // once per block.  Per residue and column three integer multiply-adds:
-//   lo += r_t (c_t mod 2^32),  hi += r_t (c_t >> 32)   (exact sums),
-//   v  += r_t F_t                                        (32-bit fixed point),
-// then S = lo + hi 2^32 - v M = lo + hi 2^32 + v (q - M mod q) mod q, one Barrett reduction
-// (the sum is below 20 251 2^61 + 2^13 2^61 < 2^75).  HI32: the host has checked that
-// T 250 max(c_t >> 32) < 2^32, so hi is summed in 32 bits.  The residue words (one per modulus,
+//   lo += u_t (c_t mod 2^32),  hi += u_t (c_t >> 32)   (exact sums),
+//   v  += u_t F_t                                        (32-bit fixed point),
+// then S = sum_t r_t c_t - v M = base + lo + hi 2^32 + (v + 128 T) (q - M mod q) mod q, base taking the
+// offsets back, one Barrett reduction (the sum is below 20 255 2^61 + 2^13 2^61 < 2^75).  HI32: the host has
+// checked that (T 255 + 1) max(q >> 32) < 2^32 and every q >= 2^40, so hi is summed in 32 bits and one FP64
+// quotient replaces Barrett's two 64 x 64-bit high products.  The residue words (one per modulus,
 // read once: streaming loads) are requested before the fold.
 template <bool HI32>
 __global__ void __launch_bounds__(256) crt_kernel(const uint8_t *__restrict__ RES, uint64_t *__restrict__ Y,
@@ -682,17 +704,20 @@ __global__ void __launch_bounds__(256) crt_kernel(const uint8_t *__restrict__ RE
     const uint64_t rg = r0 + r;
     const PrimeConst p = pc[limb];
     const uint64_t Mneg = tab[limb].Mneg;
+    const double k32 = __dmul_rn(4294967296.0, p.qinv);
     constexpr uint32_t kAhead = 16;  // residue words requested before the fold
     uint32_t res[kAhead];
 #pragma unroll
     for (uint32_t t = 0; t < kAhead; t++)
         res[t] = t < T ? __ldcs(reinterpret_cast<const uint32_t *>(RES + ((uint64_t)t * n_out + o) * chunk + r)) : 0u;
     using HiT = typename std::conditional<HI32, uint32_t, uint64_t>::type;
-    uint64_t lo[4] = {0, 0, 0, 0};
-    HiT hi[4] = {0, 0, 0, 0};
+    const uint64_t base = tab[limb].base;
+    const uint32_t vbase = c_mods.vbase[T];
+    uint64_t lo[4];
+    HiT hi[4];
     uint32_t v[4];
 #pragma unroll
-    for (int e = 0; e < 4; e++) v[e] = 1u << (kCrtFracBits - 1);
+    for (int e = 0; e < 4; e++) lo[e] = (uint32_t)base, hi[e] = (HiT)(base >> 32), v[e] = vbase;
 #pragma unroll
     for (uint32_t t = 0; t < (uint32_t)kMaxMods; t++) {
         if (t < T) {
@@ -712,11 +737,23 @@ __global__ void __launch_bounds__(256) crt_kernel(const uint8_t *__restrict__ RE
     uint64_t y[4];
 #pragma unroll
     for (int e = 0; e < 4; e++) {
-        const uint64_t h = hi[e];
-        const uint64_t plo = lo[e] + (h << 32);
-        u128 pos = {plo, (h >> 32) + (plo < lo[e] ? 1ull : 0ull)};
-        mac(pos, v[e] >> kCrtFracBits, Mneg);
-        y[e] = barrett(pos, p);
+        const uint32_t w = v[e] >> kCrtFracBits;
+        if constexpr (HI32) {
+            // S = H 2^32 + l with H < 2^34: Q = round(H 2^32 / q) from the FP64 pipe, S - Q q is within
+            // q/2 + 2^32 of zero (q >= 2^40)
+            const uint64_t l = lo[e] + (uint64_t)w * (uint32_t)Mneg;
+            const uint64_t H = (uint64_t)w * (uint32_t)(Mneg >> 32) + hi[e] + (l >> 32);
+            const double hd = __dsub_rn(as_dbl(0x4330000000000000ull | H), kTwo52);
+            const uint32_t Q = (uint32_t)as_bits(__fma_rn(hd, k32, kTwo52));
+            const uint64_t x = ((H << 32) | (uint32_t)l) - Q * p.q;
+            y[e] = x + ((uint64_t)((int64_t)x >> 63) & p.q);
+        } else {
+            const uint64_t h = hi[e];
+            const uint64_t plo = lo[e] + (h << 32);
+            u128 pos = {plo, (h >> 32) + (plo < lo[e] ? 1ull : 0ull)};
+            mac(pos, w, Mneg);
+            y[e] = barrett(pos, p);
+        }
     }
     ulonglong2 *out = reinterpret_cast<ulonglong2 *>(Y + (uint64_t)o * R + rg);
     out[0] = make_ulonglong2(y[0], y[1]);
@@ -734,7 +771,7 @@ struct Plan {
     uint32_t T_min = 0, T_max = 0;   // the moduli counts the limbs need
     std::vector<uint32_t> limb_T;    // per limb
     std::vector<CrtLimb> limbs;      // [T - T_min][L]: the CRT constants for each count in use
-    bool hi32 = false;               // T_max 250 max(c_t >> 32) < 2^32: the CRT's high sums in 32 bits
+    bool hi32 = false;               // the CRT's high sums in 32 bits (crt_kernel)
 };
 
 // The moduli count of each limb: |S| = |sum_i x_i w_io| <= (q_l - 1) max_o sum_i |w_io| = B_l, and
@@ -746,7 +783,7 @@ Plan make_plan(const Context &c, uint32_t L, uint64_t max_l1) {
     Plan p{};
     p.limb_T.resize(L);
     p.T_min = kMaxMods;
-    uint64_t max_hi = 0;
+    uint64_t max_hi = 0, min_q = ~0ull;
     for (uint32_t l = 0; l < L; l++) {
         const uint64_t q = c.primes[l];
         const double need = std::log2((double)(q - 1)) + std::log2((double)std::max<uint64_t>(max_l1, 1)) + 1.05;
@@ -761,8 +798,9 @@ Plan make_plan(const Context &c, uint32_t L, uint64_t max_l1) {
         p.T_min = std::min(p.T_min, T);
         p.T_max = std::max(p.T_max, T);
         max_hi = std::max(max_hi, (q - 1) >> 32);
+        min_q = std::min(min_q, q);
     }
-    p.hi32 = (uint64_t)p.T_max * 250 * max_hi < (1ull << 32);
+    p.hi32 = ((uint64_t)p.T_max * 255 + 1) * max_hi < (1ull << 32) && min_q >= (1ull << 40);
     for (uint32_t t = 0; t < (uint32_t)kMaxMods; t++) {
         const uint32_t m = cand[t];
         p.mods.m[t] = m;
@@ -770,7 +808,7 @@ Plan make_plan(const Context &c, uint32_t L, uint64_t max_l1) {
         p.mods.c48[t] = (uint32_t)((uint64_t)p.mods.c24[t] * p.mods.c24[t] % m);
         p.mods.magic[t] = (uint32_t)(((1ull << 32) + m - 1) / m);
         p.mods.inv[t] = 1.0 / m;
-        p.mods.invf[t] = 1.0f / (float)m;
+        p.mods.rnd[t] = (int)(((1ull << 32) + m / 2) / m);
     }
     // CRT fractions [(M/m_t)^-1 mod m_t] / m_t in fixed point, for every modulus count
     for (uint32_t n = 1; n <= (uint32_t)kMaxMods; n++)
@@ -782,6 +820,11 @@ Plan make_plan(const Context &c, uint32_t L, uint64_t max_l1) {
             const uint32_t inv = (uint32_t)host::powmod(Mt_mod_m, m - 2, m);  // m prime
             p.mods.fracq[n][t] = (uint32_t)((((uint64_t)inv << kCrtFracBits) + m / 2) / m);
         }
+    for (uint32_t n = 1; n <= (uint32_t)kMaxMods; n++) {
+        int64_t v = ((int64_t)(128 * n) << kCrtFracBits) + (1 << (kCrtFracBits - 1));
+        for (uint32_t t = 0; t < n; t++) v -= 128 * (int64_t)p.mods.fracq[n][t];
+        p.mods.vbase[n] = (uint32_t)v;
+    }
     // CRT constants for each count T in use: c_t = (M/m_t) * [(M/m_t)^-1 mod m_t] mod q_l
     p.limbs.resize((size_t)(p.T_max - p.T_min + 1) * L);
     for (uint32_t T = p.T_min; T <= p.T_max; T++)
@@ -801,7 +844,9 @@ Plan make_plan(const Context &c, uint32_t L, uint64_t max_l1) {
                     }
                 uint32_t inv = (uint32_t)host::powmod(Mt_mod_m, m - 2, m);
                 cl.c[t] = host::mulmod(Mt, inv, q);
+                cl.base = (cl.base + q - host::mulmod(128, cl.c[t], q)) % q;
             }
+            cl.base = (cl.base + host::mulmod(128 * T, M, q)) % q;
         }
     return p;
 }
@@ -876,8 +921,6 @@ void ctpt_matmul_tc(const Context &c, const uint64_t *X, const int64_t *W, uint6
     if (plan.limbs.size() > (size_t)64 * kMaxMods) throw std::invalid_argument("ct-pt matmul: too many limbs");
     SHM_CUDA(cudaMemcpyAsync(tab, plan.limbs.data(), sizeof(CrtLimb) * plan.limbs.size(), cudaMemcpyHostToDevice, st));
     SHM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
-    // zero-padded K tail of the X planes stays zero: clear once per call
-    if (Kp != n_in) SHM_CUDA(cudaMemsetAsync(XP, 0, (size_t)T * chunk * Kp, st));
     SHM_LAUNCHED(1);
     wres_kernel<<<dim3((Kp + 255) / 256, Np), 256, 0, st>>>(W, WP, n_in, n_out, Kp, Np, T);
     SHM_CUDA(cudaGetLastError());
@@ -893,7 +936,7 @@ void ctpt_matmul_tc(const Context &c, const uint64_t *X, const int64_t *W, uint6
         SHM_CUDA(cudaFuncSetAttribute(mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     int sms = 0;
     SHM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
-    const int acc24 = (uint64_t)Kp * 125 * 125 < (1ull << 24) ? 1 : 0;  // accumulators exact in float
+    const int acc_small = (uint64_t)Kp * 125 * 125 <= kAccSmall ? 1 : 0;
     bool f64_res = true;  // every limb prime below 2^51: the X residues on the FP64 pipe
     for (uint32_t l = 0; l < L; l++) f64_res = f64_res && c.primes[l] < (1ull << 51);
     SHM_CUDA(cudaFuncSetAttribute(f64_res ? xres_kernel<true> : xres_kernel<false>,
@@ -923,13 +966,13 @@ void ctpt_matmul_tc(const Context &c, const uint64_t *X, const int64_t *W, uint6
             const bool tma = tma_a && operand_tensor_map(&tmX, XP, Kp, (uint64_t)Tc * cur, kBN);
             if (tma)
                 mma_persistent_kernel<true>
-                    <<<grid, kThreadsP, kSmemP, st>>>(XP, WP, RES, Kp, Np, n_out, cur, Tc, err, acc24, tmA, tmX);
+                    <<<grid, kThreadsP, kSmemP, st>>>(XP, WP, RES, Kp, Np, n_out, cur, Tc, err, acc_small, tmA, tmX);
             else
                 mma_persistent_kernel<false>
-                    <<<grid, kThreadsP, kSmemP, st>>>(XP, WP, RES, Kp, Np, n_out, cur, Tc, err, acc24, tmA, tmX);
+                    <<<grid, kThreadsP, kSmemP, st>>>(XP, WP, RES, Kp, Np, n_out, cur, Tc, err, acc_small, tmA, tmX);
         } else {
             mma_kernel<<<dim3(Np / kBM, (uint32_t)(cur / kBN), Tc), kThreads, kSmem, st>>>(XP, WP, RES, Kp, Np, n_out,
-                                                                                          cur, err, acc24);
+                                                                                          cur, err, acc_small);
         }
         SHM_CUDA(cudaGetLastError());
         SHM_LAUNCHED(1);
