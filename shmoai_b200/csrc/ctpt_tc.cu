@@ -132,14 +132,15 @@ __device__ __forceinline__ uint32_t acc_bytes(const uint32_t *v, uint32_t t, int
 // Each thread writes four consecutive inputs' residues of one column as one 32-bit word, so a
 // warp's store covers 64 contiguous bytes of each of two columns for every modulus.  F64 (every
 // limb prime below 2^51): each residue from one FP64 and one integer multiply-add (balanced_f64),
-// else in 32-bit integer arithmetic (mod_small).
+// else in 32-bit integer arithmetic (mod_small).  T, the moduli, at compile time: a loop to the largest
+// count under guards issued the guarded iterations too.
 constexpr uint32_t kXresTiles = 2;
 constexpr uint32_t kXresSmem = 2 * 64 * 65 * 8;
 
-template <bool F64>
+template <bool F64, uint32_t T>
 __global__ void __launch_bounds__(256, 3) xres_kernel(const uint64_t *__restrict__ X, int8_t *__restrict__ XP,
                                                       uint32_t n_in, uint32_t Kp, uint64_t R, uint64_t r0,
-                                                      uint64_t chunk, uint32_t T) {
+                                                      uint64_t chunk) {
     extern __shared__ uint64_t xres_smem[];
     uint64_t(*tile)[64][65] = reinterpret_cast<uint64_t(*)[64][65]>(xres_smem);
     const uint32_t i0 = blockIdx.y * 64;
@@ -182,11 +183,9 @@ __global__ void __launch_bounds__(256, 3) xres_kernel(const uint64_t *__restrict
                     xd[j] = __dsub_rn(__longlong_as_double((long long)(0x4330000000000000ull | x[j])), two52);
                     xl[j] = (uint32_t)x[j];
                 }
-                // unrolled over every candidate modulus (a uniform guard): the constants become operands
 #pragma unroll
-                for (uint32_t t = 0; t < (uint32_t)kMaxMods; t++) {
-                    if (t < T)
-                        *reinterpret_cast<uint32_t *>(dst + (uint64_t)t * chunk * Kp) =
+                for (uint32_t t = 0; t < T; t++) {
+                    *reinterpret_cast<uint32_t *>(dst + (uint64_t)t * chunk * Kp) =
                             pack_low_bytes(balanced_f64(xd[0], xl[0], t), balanced_f64(xd[1], xl[1], t),
                                            balanced_f64(xd[2], xl[2], t), balanced_f64(xd[3], xl[3], t));
                 }
@@ -680,23 +679,24 @@ constexpr size_t kCrtTabBytes = 256 + sizeof(CrtLimb) * 64 * kMaxMods;
 // offsets back, one Barrett reduction (the sum is below 20 255 2^61 + 2^13 2^61 < 2^75).  HI32: the host has
 // checked that (T 255 + 1) max(q >> 32) < 2^32 and every q >= 2^40, so hi is summed in 32 bits and one FP64
 // quotient replaces Barrett's two 64 x 64-bit high products.  The residue words (one per modulus,
-// read once: streaming loads) are requested before the fold.
-template <bool HI32>
+// read once: streaming loads) are requested before the fold.  T at compile time, as in xres_kernel (232
+// instructions a column were issued for 12 moduli under guards up to 20: 0.77 ms a pass of 768 x 131,072).
+template <bool HI32, uint32_t T>
 __global__ void __launch_bounds__(256) crt_kernel(const uint8_t *__restrict__ RES, uint64_t *__restrict__ Y,
                                                   const CrtLimb *__restrict__ tab, uint32_t n_out, uint64_t chunk,
                                                   uint64_t r0, uint64_t R, uint32_t L, uint32_t log_n,
-                                                  const PrimeConst *__restrict__ pc, uint32_t T) {
+                                                  const PrimeConst *__restrict__ pc) {
     __shared__ uint32_t s_lo[kMaxMods], s_hi[kMaxMods], s_f[kMaxMods];
     const uint64_t rb = (uint64_t)blockIdx.x * blockDim.x * 4;
     const uint32_t o = blockIdx.y;
     const uint32_t row = (uint32_t)((r0 + rb) >> log_n);  // h L + limb, below 2 L
     const uint32_t limb = row >= L ? row - L : row;
-    if (threadIdx.x < (uint32_t)kMaxMods) {
+    if (threadIdx.x < T) {
         const uint32_t t = threadIdx.x;
-        const uint64_t c = t < T ? tab[limb].c[t] : 0;
+        const uint64_t c = tab[limb].c[t];
         s_lo[t] = (uint32_t)c;
         s_hi[t] = (uint32_t)(c >> 32);
-        s_f[t] = t < T ? c_mods.fracq[T][t] : 0u;
+        s_f[t] = c_mods.fracq[T][t];
     }
     __syncthreads();
     const uint64_t r = rb + (uint64_t)threadIdx.x * 4;
@@ -705,11 +705,10 @@ __global__ void __launch_bounds__(256) crt_kernel(const uint8_t *__restrict__ RE
     const PrimeConst p = pc[limb];
     const uint64_t Mneg = tab[limb].Mneg;
     const double k32 = __dmul_rn(4294967296.0, p.qinv);
-    constexpr uint32_t kAhead = 16;  // residue words requested before the fold
-    uint32_t res[kAhead];
+    uint32_t res[T];  // requested before the fold
 #pragma unroll
-    for (uint32_t t = 0; t < kAhead; t++)
-        res[t] = t < T ? __ldcs(reinterpret_cast<const uint32_t *>(RES + ((uint64_t)t * n_out + o) * chunk + r)) : 0u;
+    for (uint32_t t = 0; t < T; t++)
+        res[t] = __ldcs(reinterpret_cast<const uint32_t *>(RES + ((uint64_t)t * n_out + o) * chunk + r));
     using HiT = typename std::conditional<HI32, uint32_t, uint64_t>::type;
     const uint64_t base = tab[limb].base;
     const uint32_t vbase = c_mods.vbase[T];
@@ -719,19 +718,14 @@ __global__ void __launch_bounds__(256) crt_kernel(const uint8_t *__restrict__ RE
 #pragma unroll
     for (int e = 0; e < 4; e++) lo[e] = (uint32_t)base, hi[e] = (HiT)(base >> 32), v[e] = vbase;
 #pragma unroll
-    for (uint32_t t = 0; t < (uint32_t)kMaxMods; t++) {
-        if (t < T) {
-            const uint32_t r4 =
-                t < kAhead ? res[t]
-                           : __ldcs(reinterpret_cast<const uint32_t *>(RES + ((uint64_t)t * n_out + o) * chunk + r));
-            const uint32_t cl = s_lo[t], ch = s_hi[t], f = s_f[t];
+    for (uint32_t t = 0; t < T; t++) {
+        const uint32_t cl = s_lo[t], ch = s_hi[t], f = s_f[t];
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const uint32_t rt = (r4 >> (8 * e)) & 0xFF;
-                lo[e] += (uint64_t)rt * cl;
-                hi[e] += (HiT)rt * ch;
-                v[e] += rt * f;
-            }
+        for (int e = 0; e < 4; e++) {
+            const uint32_t rt = (res[t] >> (8 * e)) & 0xFF;
+            lo[e] += (uint64_t)rt * cl;
+            hi[e] += (HiT)rt * ch;
+            v[e] += rt * f;
         }
     }
     uint64_t y[4];
@@ -898,6 +892,20 @@ size_t ctpt_tc_ws_bytes(const Context &c, uint32_t n_in, uint32_t n_out, uint32_
     return (size_t)kMaxMods * (chunk * Kp + (uint64_t)Np * Kp + (uint64_t)n_out * chunk) + kCrtTabBytes;
 }
 
+// f(T) with the modulus count as a compile-time constant
+template <class F>
+static void with_moduli(uint32_t T, F &&f) {
+#define SHM_T_CASE(n) \
+    case n: f(std::integral_constant<uint32_t, n>{}); break;
+    switch (T) {
+        SHM_T_CASE(1) SHM_T_CASE(2) SHM_T_CASE(3) SHM_T_CASE(4) SHM_T_CASE(5) SHM_T_CASE(6) SHM_T_CASE(7)
+        SHM_T_CASE(8) SHM_T_CASE(9) SHM_T_CASE(10) SHM_T_CASE(11) SHM_T_CASE(12) SHM_T_CASE(13) SHM_T_CASE(14)
+        SHM_T_CASE(15) SHM_T_CASE(16) SHM_T_CASE(17) SHM_T_CASE(18) SHM_T_CASE(19) SHM_T_CASE(20)
+        default: throw std::invalid_argument("ct-pt matmul: modulus count out of range");
+    }
+#undef SHM_T_CASE
+}
+
 // Chunks of 131,072 columns run one after the other on `st`.  (Alternating them over two
 // streams, so that one chunk's residue and CRT kernels could run beside the other's GEMM,
 // measured no faster: the GEMM's grid fills every SM.)
@@ -939,8 +947,6 @@ void ctpt_matmul_tc(const Context &c, const uint64_t *X, const int64_t *W, uint6
     const int acc_small = (uint64_t)Kp * 125 * 125 <= kAccSmall ? 1 : 0;
     bool f64_res = true;  // every limb prime below 2^51: the X residues on the FP64 pipe
     for (uint32_t l = 0; l < L; l++) f64_res = f64_res && c.primes[l] < (1ull << 51);
-    SHM_CUDA(cudaFuncSetAttribute(f64_res ? xres_kernel<true> : xres_kernel<false>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kXresSmem));
     for (uint64_t r0 = 0; r0 < R; r0 += chunk) {
         // a shorter last pass (2 L N not a multiple of the chunk, e.g. at N = 2^12) lays its planes out
         // with its own column count; every count here is a multiple of 256
@@ -952,10 +958,11 @@ void ctpt_matmul_tc(const Context &c, const uint64_t *X, const int64_t *W, uint6
         const CrtLimb *tab_c = tab + (size_t)(Tc - plan.T_min) * L;
         SHM_LAUNCHED(1);
         const dim3 xgrid((uint32_t)(cur / (64 * kXresTiles)), (n_in + 63) / 64);
-        if (f64_res)
-            xres_kernel<true><<<xgrid, 256, kXresSmem, st>>>(X, XP, n_in, Kp, R, r0, cur, Tc);
-        else
-            xres_kernel<false><<<xgrid, 256, kXresSmem, st>>>(X, XP, n_in, Kp, R, r0, cur, Tc);
+        with_moduli(Tc, [&](auto n) {
+            const auto f = f64_res ? xres_kernel<true, decltype(n)::value> : xres_kernel<false, decltype(n)::value>;
+            SHM_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kXresSmem));
+            f<<<xgrid, 256, kXresSmem, st>>>(X, XP, n_in, Kp, R, r0, cur);
+        });
         SHM_CUDA(cudaGetLastError());
         SHM_LAUNCHED(1);
         if (resident) {
@@ -979,12 +986,55 @@ void ctpt_matmul_tc(const Context &c, const uint64_t *X, const int64_t *W, uint6
         // 4 columns a thread; a block's columns within one limb (N and r0 are multiples of the block's)
         const uint32_t crt_threads = chunk % 1024 == 0 ? 256 : 64;
         const dim3 cgrid((uint32_t)((cur / 4 + crt_threads - 1) / crt_threads), n_out);
-        if (plan.hi32)
-            crt_kernel<true><<<cgrid, crt_threads, 0, st>>>(RES, Y, tab_c, n_out, cur, r0, R, L, c.log_n, c.pc, Tc);
-        else
-            crt_kernel<false><<<cgrid, crt_threads, 0, st>>>(RES, Y, tab_c, n_out, cur, r0, R, L, c.log_n, c.pc, Tc);
+        with_moduli(Tc, [&](auto n) {
+            const auto f = plan.hi32 ? crt_kernel<true, decltype(n)::value> : crt_kernel<false, decltype(n)::value>;
+            f<<<cgrid, crt_threads, 0, st>>>(RES, Y, tab_c, n_out, cur, r0, R, L, c.log_n, c.pc);
+        });
         SHM_CUDA(cudaGetLastError());
     }
+}
+
+namespace {
+
+// l1[o] += sum of |w_io| over 32 inputs, mx = max |w|.  Grid (n_out / 128, n_in / 32)
+__global__ void weight_sums(const int64_t *__restrict__ W, uint32_t n_in, uint32_t n_out,
+                            unsigned long long *__restrict__ l1, unsigned long long *__restrict__ mx) {
+    const uint32_t o = blockIdx.x * 128 + threadIdx.x, i0 = blockIdx.y * 32;
+    if (o >= n_out) return;
+    unsigned long long s = 0, m = 0;
+#pragma unroll 8
+    for (uint32_t i = i0; i < min(n_in, i0 + 32); i++) {
+        const int64_t w = W[(uint64_t)i * n_out + o];
+        const unsigned long long a = w < 0 ? 0ull - (unsigned long long)w : (unsigned long long)w;
+        s += a;
+        m = a > m ? a : m;
+    }
+    atomicAdd(l1 + o, s);
+    atomicMax(mx, m);
+}
+
+__global__ void max_sum(const unsigned long long *__restrict__ l1, uint32_t n_out, unsigned long long *__restrict__ out) {
+    unsigned long long m = 0;
+    for (uint32_t o = threadIdx.x; o < n_out; o += blockDim.x) m = l1[o] > m ? l1[o] : m;
+    atomicMax(out, m);
+}
+
+}  // namespace
+
+// the largest column sum of |W| (below n_in 2^40) and the largest |W|; uses the plane area of ws
+void ctpt_weight_norms(const int64_t *W, uint32_t n_in, uint32_t n_out, void *ws, uint64_t &max_l1, uint64_t &max_w,
+                       cudaStream_t st) {
+    auto *t = reinterpret_cast<unsigned long long *>(static_cast<uint8_t *>(ws) + kCrtTabBytes);  // max w, max l1, l1[]
+    SHM_CUDA(cudaMemsetAsync(t, 0, ((size_t)n_out + 2) * 8, st));
+    SHM_LAUNCHED(2);
+    weight_sums<<<dim3((n_out + 127) / 128, (n_in + 31) / 32), 128, 0, st>>>(W, n_in, n_out, t + 2, t);
+    max_sum<<<1, 256, 0, st>>>(t + 2, n_out, t + 1);
+    SHM_CUDA(cudaGetLastError());
+    uint64_t h[2];
+    SHM_CUDA(cudaMemcpyAsync(h, t, sizeof h, cudaMemcpyDeviceToHost, st));
+    SHM_CUDA(cudaStreamSynchronize(st));
+    max_w = h[0];
+    max_l1 = h[1];
 }
 
 int ctpt_tc_error(void *ws, cudaStream_t st) {
