@@ -42,9 +42,19 @@ constexpr int kMaxB = 16;
 constexpr int kIpT = 128;
 constexpr size_t kIpSmemMax = 96 * 1024;  // largest chunk the autotuner may pick
 
-template <int B, int A>
+//
+// ADD: the b rows (h < H - 1) get the rotated b of the group added, sigma(b) over every limb of an
+// extended input (pmod null), else P sigma(b) on the Q limbs: the extended Sh-Rot output without a pass of its
+// own over the sums.
+struct ExtAdd {
+    const uint64_t *b = nullptr;     // [groups][H][L or LP][N]
+    const uint64_t *pmod = nullptr;  // [nq][2]: P mod q_j and its Shoup companion
+};
+
+template <int B, int A, bool ADD>
 __global__ void __launch_bounds__(kIpT) ip_multi_kernel(const uint64_t *__restrict__ up, OwnLimbs own,
                                                         const uint64_t *__restrict__ key, uint64_t *__restrict__ acc,
+                                                        ExtAdd add,
                                                         uint32_t n_cts, uint32_t chunk, uint32_t L, uint32_t np,
                                                         uint32_t nq, uint32_t H, uint32_t log_n,
                                                         const PrimeConst *__restrict__ pc,
@@ -62,6 +72,8 @@ __global__ void __launch_bounds__(kIpT) ip_multi_kernel(const uint64_t *__restri
     const I ip(pc[pj]);
     const uint32_t c0 = blockIdx.z * chunk, nc = min(chunk, n_cts - c0);
     const uint32_t ob = own.p && j < L ? j / np : B;
+    const uint64_t q = pc[pj].q, pm = ADD && add.pmod && j < L ? add.pmod[2 * j] : 0,
+                   pms = ADD && add.pmod && j < L ? add.pmod[2 * j + 1] : 0;
     const uint64_t *kp = key + (size_t)pj * n + k;
     uint64_t next[B];
 #pragma unroll
@@ -86,10 +98,15 @@ __global__ void __launch_bounds__(kIpT) ip_multi_kernel(const uint64_t *__restri
             for (int b = 0; b < B; b++) next[b] = __ldg(kp + (size_t)b * H * QP * n);
         }
         for (uint32_t ct = 0; ct < nc; ct++) {
+            uint64_t s = 0;
+            const bool plus = ADD && h + 1 < H && (!add.pmod || j < L);
+            if (plus) s = add.b[(((size_t)(c0 + ct) * H + h) * (add.pmod ? L : LP) + j) * n + ks];
             typename I::Acc a;
 #pragma unroll
             for (int b = 0; b < B; b++) ip.add(a, b, su[(ct * B + b) * kIpT], kk[b]);
-            out[(size_t)ct * H * LP * n] = ip.reduce(a);
+            uint64_t v = ip.reduce(a);
+            if (plus) v = add_mod(v, add.pmod ? shoup(s, pm, pms, q) : s, q);
+            out[(size_t)ct * H * LP * n] = v;
         }
     }
 }
@@ -186,8 +203,10 @@ ExtConsts ext_consts(Context &c, uint32_t L) {
 
 // The Sh-Rot / FmtSwitch inner products: groups are served in chunks that fit
 // c.ip_chunk_bytes of shared memory, each chunk reading the key once.
-void ip_multi(const Context &c, const uint64_t *up, OwnLimbs own, const uint64_t *key, uint64_t *acc, uint32_t n_cts,
-              uint32_t L, uint32_t beta, uint32_t H, const uint32_t *perm, cudaStream_t st) {
+template <bool ADD>
+static void ip_multi_any(const Context &c, const uint64_t *up, OwnLimbs own, const uint64_t *key, uint64_t *acc,
+                         ExtAdd add, uint32_t n_cts, uint32_t L, uint32_t beta, uint32_t H, const uint32_t *perm,
+                         cudaStream_t st) {
     const uint32_t LP = L + c.np;
     const size_t cap = std::min<size_t>(c.ip_chunk_bytes, kIpSmemMax);
     const uint32_t chunk = std::max<uint32_t>(1, std::min<uint32_t>(n_cts, (uint32_t)(cap / (beta * kIpT * 8))));
@@ -195,16 +214,21 @@ void ip_multi(const Context &c, const uint64_t *up, OwnLimbs own, const uint64_t
     const size_t smem = (size_t)chunk * beta * kIpT * 8;
     SHM_LAUNCHED(1);
     ip_dispatch(c, beta, [&](auto b, auto a) {
-        const auto f = ip_multi_kernel<decltype(b)::value, decltype(a)::value>;
+        const auto f = ip_multi_kernel<decltype(b)::value, decltype(a)::value, ADD>;
         static std::atomic<uint64_t> ready{0};  // a bit per device: the attribute belongs to the device's module
         const uint64_t bit = 1ull << (c.device & 63);
         if (!(ready.load(std::memory_order_acquire) & bit)) {
             SHM_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kIpSmemMax));
             ready.fetch_or(bit, std::memory_order_release);
         }
-        f<<<grid, kIpT, smem, st>>>(up, own, key, acc, n_cts, chunk, L, c.np, c.nq, H, c.log_n, c.pc, perm);
+        f<<<grid, kIpT, smem, st>>>(up, own, key, acc, add, n_cts, chunk, L, c.np, c.nq, H, c.log_n, c.pc, perm);
     });
     SHM_CUDA(cudaGetLastError());
+}
+
+void ip_multi(const Context &c, const uint64_t *up, OwnLimbs own, const uint64_t *key, uint64_t *acc, uint32_t n_cts,
+              uint32_t L, uint32_t beta, uint32_t H, const uint32_t *perm, cudaStream_t st) {
+    ip_multi_any<false>(c, up, own, key, acc, {}, n_cts, L, beta, H, perm, st);
 }
 
 namespace {
@@ -338,28 +362,6 @@ __global__ void add_ext_kernel(const uint64_t *__restrict__ a, const uint64_t *_
     out[off] = add_mod(a[off], b[off], pc[j < L ? j : nq + (j - L)].q);
 }
 
-// The extended Sh-Rot output of one target: out[g][h] = acc[g][h] (+ for the b rows h < n the
-// rotated b: over every limb sigma(b_ext) when the input is extended, else P sigma(b) on the
-// Q limbs).  Grid (N/kT, LP, groups * H)
-__global__ void combine_ext_kernel(const uint64_t *__restrict__ acc, uint64_t *__restrict__ out,
-                                   const uint64_t *__restrict__ bsrc, int b_ext, const uint32_t *__restrict__ perm,
-                                   uint32_t H, uint32_t L, uint32_t np, uint32_t nq, uint32_t log_n,
-                                   const PrimeConst *__restrict__ pc, const uint64_t *__restrict__ pmod) {
-    const uint32_t j = blockIdx.y, gh = blockIdx.z, h = gh % H, LP = L + np;
-    const uint32_t k = blockIdx.x * kT + threadIdx.x;
-    const size_t off = (((size_t)gh * LP + j) << log_n) + k;
-    uint64_t v = acc[off];
-    if (h + 1 < H) {
-        const uint32_t ks = perm ? __ldg(perm + k) : k;
-        const uint64_t q = pc[j < L ? j : nq + (j - L)].q;
-        if (b_ext)
-            v = add_mod(v, bsrc[(((size_t)gh * LP + j) << log_n) + ks], q);
-        else if (j < L)
-            v = add_mod(v, shoup(bsrc[(((size_t)gh * L + j) << log_n) + ks], pmod[2 * j], pmod[2 * j + 1], q), q);
-    }
-    out[off] = v;
-}
-
 // ModDown of n_polys extended polynomials (their special-prime limbs are overwritten by the
 // inverse NTT) into out [n_polys][L][N]; delta: [n_polys][L][N] scratch
 void moddown_rows(const Context &c, uint64_t *ext, uint64_t *out, uint32_t n_polys, uint32_t L, uint64_t *delta,
@@ -435,11 +437,8 @@ void shared_rotate_ext(const Context &c, const uint64_t *in, bool in_ext, uint32
     }
     for (uint32_t e = 0; e < n_elts; e++) {
         const uint32_t *perm = const_cast<Context &>(c).perm(elts[e]);
-        ip_multi(c, up, own, keys[e], acc, n_groups, L, beta, H, perm, st);
-        SHM_LAUNCHED(1);
-        combine_ext_kernel<<<dim3(N / kT, LP, n_groups * H), kT, 0, st>>>(acc, outs[e], in, in_ext ? 1 : 0, perm, H, L,
-                                                                          c.np, c.nq, c.log_n, c.pc, c.p_mod);
-        SHM_CUDA(cudaGetLastError());
+        ip_multi_any<true>(c, up, own, keys[e], outs[e], ExtAdd{in, in_ext ? nullptr : c.p_mod}, n_groups, L, beta, H,
+                           perm, st);
     }
 }
 
