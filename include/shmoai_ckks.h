@@ -297,8 +297,8 @@ int shm_drop_limbs(const shm_context *ctx, const uint64_t *in, uint64_t *out, ui
 size_t shm_ctpt_matmul_workspace_bytes(const shm_context *ctx, uint32_t n_in, uint32_t n_out, uint32_t L);
 /* Computed on the INT8 tensor cores (tcgen05.mma kind::i8) through a small-modulus
  * residue system: exact for |W| < 2^40 (larger weights: SHM_EINVAL).  The call
- * reads W back to the host once to size the residue system, so it synchronises
- * `stream`. */
+ * forms max |W| and the largest column sum of |W| on the device and reads these two
+ * words back to size the residue system, so it synchronises `stream`. */
 int shm_ctpt_matmul(const shm_context *ctx, const uint64_t *X, const int64_t *W, uint64_t *Y, uint32_t n_in,
                     uint32_t n_out, uint32_t L, void *workspace, size_t workspace_bytes, void *stream);
 /* The same contraction on the CUDA cores (64-bit multiply-accumulate, |W| < 2^40):
@@ -351,7 +351,7 @@ void shm_graph_destroy(shm_graph *g);
  * fastest for this context; later calls on any stream use it.  Synchronises the device.
  *   SHM_TUNE_NTT_TILE  tile variant of the NTT kernels, candidates 0..3 = (columns per CTA,
  *                      minimum resident CTAs per SM) (16, 4), (16, 3), (8, 8), (8, 6);
- *                      workload: forward + inverse NTT of `size` limbs.
+ *                      workload: forward + inverse NTT of `size` limbs.  3 until tuned or set.
  *   SHM_TUNE_IP_CHUNK  shared memory of one Sh-Rot inner-product block, candidates 0..3 =
  *                      16, 32, 64, 96 KB (more groups of a chunk share each key read);
  *                      workload: `size` groups of `members` at `level` primes.

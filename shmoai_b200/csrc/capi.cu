@@ -1206,7 +1206,6 @@ int shm_tune_set(shm_context *ctx, int knob, uint32_t index) {
             if (index >= (uint32_t)shm::kNttVariantCount) throw std::invalid_argument("tile variant out of range");
             SHM_CUDA(cudaDeviceSynchronize());  // launches in flight keep their shape
             c.ntt_variant = (int)index;
-            c.ntt_tuned = true;
         } else if (knob == SHM_TUNE_IP_CHUNK) {
             if (index >= std::size(shm::kIpChunkCandidates)) throw std::invalid_argument("chunk candidate out of range");
             SHM_CUDA(cudaDeviceSynchronize());

@@ -74,8 +74,7 @@ struct Context {
     uint32_t log_n = 0, n = 0, nq = 0, np = 0, dnum = 0;
     std::vector<uint64_t> primes;       // nq + np
     bool s52 = false;                   // every prime in [kS52PrimeMin, kS52PrimeLimit) (Acc<true> kernels)
-    int ntt_variant = 0;                // index into kNttVariants (set by the autotuner)
-    bool ntt_tuned = false;             // it has been set: every launch takes it
+    int ntt_variant = kNttDefault;      // index into kNttVariants (set by the autotuner)
     int ntt_families = 0;               // the NTT instantiation for the primes' butterfly families (kFam*)
     uint32_t ip_chunk_bytes = 32768;    // shared memory per Sh-Rot inner-product block (autotuned)
     std::vector<PrimeConst> h_pc;       // host copy

@@ -31,6 +31,11 @@ struct NttVariant {
 };
 constexpr NttVariant kNttVariants[] = {{16, 4}, {16, 3}, {8, 8}, {8, 6}};
 constexpr int kNttVariantCount = 4;
+// The tile until one is tuned or set: 8 x 6 (80 registers, no spills; the small tile spreads few rows more
+// evenly).  Medians of alternated runs at 16 x 4 and 8 x 6: forward and inverse of 117 x 35 limbs 3.93 and 3.56
+// ms, a product at 24 limbs 362 and 333 us, five rotations at 17 limbs 636 and 608 us, sixteen products at 27
+// limbs 4.21 and 4.13 ms; 8 x 5 and 8 x 7 lie between.
+constexpr int kNttDefault = 3;
 
 // The rows a launch transforms: slots [first, first + count) of each of `polys` polynomials of
 // `slots` limbs.  Slot s stands at position j = s % lp of its digit s / lp (lp = slots: one digit)

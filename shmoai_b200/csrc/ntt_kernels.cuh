@@ -414,17 +414,10 @@ void launch_inv_v(const Context &c, const InvArgs &v, const NttRows &rw, cudaStr
                                                           v.scale ? v.scale : c.inv_scale_plain, v.scale ? 0 : 1);
 }
 
-// The tile variants of kNttVariants (ntt.cuh): the context's, once one has been tuned or set, else 16 columns
-// x 4 CTAs per SM for large launches and 8 x 6 below 16 waves of the former (592 rows), where the smaller tile
-// spreads the rows more evenly: one rotation at 24 limbs 268 us at 16 x 4, 257 at 8 x 6; five at 17 limbs 626 and
-// 596; 16 products at 27 limbs 4.23 ms and 4.34.
-inline int ntt_tile(const Context &c, const NttRows &rw) {
-    return c.ntt_tuned ? c.ntt_variant : (uint64_t)rw.polys * rw.count < 592 ? 3 : 0;
-}
-
+// the tile variants of kNttVariants (ntt.cuh), selected per context by c.ntt_variant
 template <int R, int IOK, int FAM>
 void launch_fwd_f(const Context &c, uint64_t *data, const NttRows &rw, cudaStream_t st, const NttIO &io) {
-    switch (ntt_tile(c, rw)) {
+    switch (c.ntt_variant) {
 #ifndef SHM_NTT_ONE_TILE  // a development build may leave the other tiles out
         case 1: launch_fwd_v<R, 16, 3, IOK, FAM>(c, data, rw, st, io); break;
         case 2: launch_fwd_v<R, 8, 8, IOK, FAM>(c, data, rw, st, io); break;
@@ -448,7 +441,7 @@ void launch_fwd(const Context &c, int kind, uint64_t *data, const NttRows &rw, c
 
 template <int R, int FAM>
 void launch_inv(const Context &c, const InvArgs &v, const NttRows &rw, cudaStream_t st) {
-    switch (ntt_tile(c, rw)) {
+    switch (c.ntt_variant) {
 #ifndef SHM_NTT_ONE_TILE
         case 1: launch_inv_v<R, 16, 3, FAM>(c, v, rw, st); break;
         case 2: launch_inv_v<R, 8, 8, FAM>(c, v, rw, st); break;

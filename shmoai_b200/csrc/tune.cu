@@ -71,7 +71,6 @@ uint32_t tune_ntt_tile(Context &c, uint32_t rows, std::vector<float> &ms) {
     uint64_t *x = s.get((size_t)polys * L * c.n);
     sample_uniform(c, x, polys, L, 0x7E57, s.st);
     ms.clear();
-    c.ntt_tuned = true;
     for (int v = 0; v < kNttVariantCount; v++) {
         c.ntt_variant = v;
         ms.push_back(time_ms(s.st, 5, [&] {

@@ -88,3 +88,27 @@ def test_family_edges_match_oracle(log_n, families):
         assert np.array_equal(fwd[p], orc.ntt(x[p])), (p, "forward")
         assert np.array_equal(inv[p], orc.intt(x[p])), (p, "inverse")
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("polys,limbs", [(1, 1), (37, 4), (593, 1)])
+def test_every_tile_matches_oracle(polys, limbs):
+    """One row, the SMs' count and a row beyond whole waves, under the default tile and every tile set by
+    hand."""
+    from oracle import oracle as O
+    from shmoai_b200._lib import check, lib
+    from shmoai_b200.ckks import CKKSContext, to_device, to_host
+
+    pr = _primes_near(1 << 46, 12, 3) + _primes_near(1 << 51, 12, 1)
+    rng = np.random.default_rng(11)
+    x = rng.integers(0, 1 << 63, (polys, limbs, 4096), dtype=np.uint64) % np.array(pr[:limbs], np.uint64)[None, :, None]
+    orc = O.Oracle(12, np.array(pr, dtype=np.uint64), len(pr), 0)
+    want = np.stack([orc.ntt(v) for v in x])
+    ctx = CKKSContext(12, primes=pr)
+    for tile in (None, 0, 1, 2, 3):
+        if tile is not None:
+            check(lib().shm_tune_set(ctx._h, 0, tile))
+        d = ctx.ntt_forward_(to_device(x))
+        assert np.array_equal(to_host(d), want), (tile, "forward")
+        assert np.array_equal(to_host(ctx.ntt_inverse_(d)), x), (tile, "inverse")
+    ctx.close()
