@@ -1162,7 +1162,7 @@ def run_gelu(args, rank, world, dist):
     def e2e_step():
         ct.write_from_ptr(h_in.data_ptr())
         graph.launch()
-        (graph.out if c2s else out).to_ptr(h_out.data_ptr())
+        out.to_ptr(h_out.data_ptr())
 
     e2e_ms = timed_steps(torch, e2e_step, args.steps, dist, None)
     clocks = clk.summary()
