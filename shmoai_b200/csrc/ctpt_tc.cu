@@ -677,14 +677,16 @@ constexpr size_t kCrtTabBytes = 256 + sizeof(CrtLimb) * 64 * kMaxMods;
 
 // One thread folds 4 consecutive columns r of one output (4-byte residue loads, two 16-byte
 // stores).  The host sizes the block so that its 4 blockDim.x columns lie in one limb: the limb's
-// constants (the 32-bit halves of c_t and the fixed-point fractions) are staged in shared memory
-// once per block.  Per residue and column three integer multiply-adds:
-//   lo += u_t (c_t mod 2^32),  hi += u_t (c_t >> 32)   (exact sums),
-//   v  += u_t F_t                                        (32-bit fixed point),
+// constants are staged in shared memory once per block.  The sums over t, exact:
+//   lo = sum u_t (c_t mod 2^32),  hi = sum u_t (c_t >> 32),  v = sum u_t F_t  (32-bit fixed point),
 // then S = sum_t r_t c_t - v M = base + lo + hi 2^32 + (v + 128 T) (q - M mod q) mod q, base taking the
-// offsets back, one Barrett reduction (the sum is below 20 255 2^61 + 2^13 2^61 < 2^75).  HI32: the host has
-// checked that (T 255 + 1) max(q >> 32) < 2^32 and every q >= 2^40, so hi is summed in 32 bits and one FP64
-// quotient replaces Barrett's two 64 x 64-bit high products.  The residue words (one per modulus,
+// offsets back, one Barrett reduction (the sum is below 20 255 2^61 + 2^13 2^61 < 2^75).
+// HI32: the host has checked that (T 255 + 1) max(q >> 32) < 2^32 (so q < 2^56) and every q >= 2^40.  Then
+// hi fits 32 bits and one FP64 quotient replaces Barrett's two 64 x 64-bit high products, and the sums are
+// taken byte by byte: four moduli's residues of a column (a 4 x 4 byte transpose) times the same four moduli's
+// bytes of c_t (seven) and F_t (three) are ten four-way byte products, 30 a column for 12 moduli in place of
+// 12 wide and 24 plain multiply-adds and 12 byte extracts.  768 to 768 ciphertexts at 13 limbs 29.5 and 28.8 ms
+// in alternated runs, 100 to 70 at 7 limbs 1.78 and 1.74 ms.  The residue words (one per modulus,
 // read once: streaming loads) are requested before the fold.  T at compile time, as in xres_kernel (232
 // instructions a column were issued for 12 moduli under guards up to 20: 0.77 ms a pass of 768 x 131,072).
 template <bool HI32, uint32_t T>
@@ -692,12 +694,28 @@ __global__ void __launch_bounds__(256) crt_kernel(const uint8_t *__restrict__ RE
                                                   const CrtLimb *__restrict__ tab, uint32_t n_out, uint64_t chunk,
                                                   uint64_t r0, uint64_t R, uint32_t L, uint32_t log_n,
                                                   const PrimeConst *__restrict__ pc) {
+    constexpr uint32_t G = (T + 3) / 4;  // groups of four moduli
     __shared__ uint32_t s_lo[kMaxMods], s_hi[kMaxMods], s_f[kMaxMods];
+    __shared__ __align__(16) uint32_t s_k[G][12];
     const uint64_t rb = (uint64_t)blockIdx.x * blockDim.x * 4;
     const uint32_t o = blockIdx.y;
     const uint32_t row = (uint32_t)((r0 + rb) >> log_n);  // h L + limb, below 2 L
     const uint32_t limb = row >= L ? row - L : row;
-    if (threadIdx.x < T) {
+    if constexpr (HI32) {
+        for (uint32_t i = threadIdx.x; i < G * 12; i += blockDim.x) {
+            const uint32_t g = i / 12, b = i % 12;
+            uint32_t w = 0;
+#pragma unroll
+            for (uint32_t j = 0; j < 4; j++) {
+                const uint32_t t = 4 * g + j;
+                if (t < T && b < 10) {
+                    const uint32_t byte = b < 7 ? (uint32_t)(tab[limb].c[t] >> (8 * b)) : c_mods.fracq[T][t] >> (8 * (b - 7));
+                    w |= (byte & 0xFF) << (8 * j);
+                }
+            }
+            s_k[g][b] = w;
+        }
+    } else if (threadIdx.x < T) {
         const uint32_t t = threadIdx.x;
         const uint64_t c = tab[limb].c[t];
         s_lo[t] = (uint32_t)c;
@@ -711,44 +729,78 @@ __global__ void __launch_bounds__(256) crt_kernel(const uint8_t *__restrict__ RE
     const PrimeConst p = pc[limb];
     const uint64_t Mneg = tab[limb].Mneg;
     const double k32 = __dmul_rn(4294967296.0, p.qinv);
-    uint32_t res[T];  // requested before the fold
+    uint32_t res[4 * G];  // requested before the fold
 #pragma unroll
     for (uint32_t t = 0; t < T; t++)
         res[t] = __ldcs(reinterpret_cast<const uint32_t *>(RES + ((uint64_t)t * n_out + o) * chunk + r));
-    using HiT = typename std::conditional<HI32, uint32_t, uint64_t>::type;
+#pragma unroll
+    for (uint32_t t = T; t < 4 * G; t++) res[t] = 0;
     const uint64_t base = tab[limb].base;
     const uint32_t vbase = c_mods.vbase[T];
-    uint64_t lo[4];
-    HiT hi[4];
-    uint32_t v[4];
-#pragma unroll
-    for (int e = 0; e < 4; e++) lo[e] = (uint32_t)base, hi[e] = (HiT)(base >> 32), v[e] = vbase;
-#pragma unroll
-    for (uint32_t t = 0; t < T; t++) {
-        const uint32_t cl = s_lo[t], ch = s_hi[t], f = s_f[t];
+    uint64_t y[4];
+    if constexpr (HI32) {
+        uint32_t d[4][10];
 #pragma unroll
         for (int e = 0; e < 4; e++) {
-            const uint32_t rt = (res[t] >> (8 * e)) & 0xFF;
-            lo[e] += (uint64_t)rt * cl;
-            hi[e] += (HiT)rt * ch;
-            v[e] += rt * f;
-        }
-    }
-    uint64_t y[4];
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const uint32_t w = v[e] >> kCrtFracBits;
-        if constexpr (HI32) {
+            for (int b = 0; b < 10; b++) d[e][b] = 0;
+            d[e][0] = (uint32_t)base & 0xFFFF;
+            d[e][2] = (uint32_t)base >> 16;
+            d[e][4] = (uint32_t)(base >> 32);
+            d[e][7] = vbase & 0xFFFF;
+            d[e][9] = vbase >> 16;
+        }
+#pragma unroll
+        for (uint32_t g = 0; g < G; g++) {
+            const uint32_t *w = res + 4 * g;  // four moduli of four columns -> four columns of four moduli
+            const uint32_t a0 = __byte_perm(w[0], w[1], 0x5140), a1 = __byte_perm(w[2], w[3], 0x5140);
+            const uint32_t a2 = __byte_perm(w[0], w[1], 0x7362), a3 = __byte_perm(w[2], w[3], 0x7362);
+            const uint32_t u[4] = {__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632),
+                                   __byte_perm(a2, a3, 0x5410), __byte_perm(a2, a3, 0x7632)};
+            uint32_t k[12];
+#pragma unroll
+            for (int b = 0; b < 12; b += 4) {
+                const uint4 x = *reinterpret_cast<const uint4 *>(&s_k[g][b]);
+                k[b] = x.x, k[b + 1] = x.y, k[b + 2] = x.z, k[b + 3] = x.w;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+#pragma unroll
+                for (int b = 0; b < 10; b++) d[e][b] = __dp4a(u[e], k[b], d[e][b]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
             // S = H 2^32 + l with H < 2^34: Q = round(H 2^32 / q) from the FP64 pipe, S - Q q is within
             // q/2 + 2^32 of zero (q >= 2^40)
-            const uint64_t l = lo[e] + (uint64_t)w * (uint32_t)Mneg;
-            const uint64_t H = (uint64_t)w * (uint32_t)(Mneg >> 32) + hi[e] + (l >> 32);
+            const uint32_t w = (d[e][7] + (d[e][8] << 8) + (d[e][9] << 16)) >> kCrtFracBits;
+            const uint64_t l = (d[e][0] + (d[e][1] << 8)) + ((uint64_t)(d[e][2] + (d[e][3] << 8)) << 16) +
+                               (uint64_t)w * (uint32_t)Mneg;
+            const uint64_t H = (uint64_t)w * (uint32_t)(Mneg >> 32) +
+                               (d[e][4] + (d[e][5] << 8) + (d[e][6] << 16)) + (l >> 32);
             const double hd = __dsub_rn(as_dbl(0x4330000000000000ull | H), kTwo52);
             const uint32_t Q = (uint32_t)as_bits(__fma_rn(hd, k32, kTwo52));
             const uint64_t x = ((H << 32) | (uint32_t)l) - Q * p.q;
             y[e] = x + ((uint64_t)((int64_t)x >> 63) & p.q);
-        } else {
-            const uint64_t h = hi[e];
+        }
+    } else {
+        uint64_t lo[4], hi[4];
+        uint32_t v[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) lo[e] = (uint32_t)base, hi[e] = base >> 32, v[e] = vbase;
+#pragma unroll
+        for (uint32_t t = 0; t < T; t++) {
+            const uint32_t cl = s_lo[t], ch = s_hi[t], f = s_f[t];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const uint32_t rt = (res[t] >> (8 * e)) & 0xFF;
+                lo[e] += (uint64_t)rt * cl;
+                hi[e] += (uint64_t)rt * ch;
+                v[e] += rt * f;
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const uint64_t h = hi[e], w = v[e] >> kCrtFracBits;
             const uint64_t plo = lo[e] + (h << 32);
             u128 pos = {plo, (h >> 32) + (plo < lo[e] ? 1ull : 0ull)};
             mac(pos, w, Mneg);
