@@ -296,6 +296,11 @@ struct OwnLimbs {
 // own limbs (NTT form already: OwnLimbs{d, d_stride}); x: [n_cts][L][N] scratch
 void modup_into(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n_cts, uint32_t L, uint64_t *x,
                 uint64_t *up, cudaStream_t st);
+// Where the inner products after a ModUp find the own limbs of d.  outs: the outputs (out_words words each) that
+// are written before or by the last inner product; when one of them covers d, the own limbs are copied to their
+// rows of up first.
+OwnLimbs own_limbs(const Context &c, OwnLimbs d, uint32_t n_cts, uint32_t L, uint64_t *up, const uint64_t *const *outs,
+                   uint32_t n_outs, size_t out_words, cudaStream_t st);
 
 // shared-a batches [n_groups][n + 1][L][N] = (b_0 .. b_{n-1}, a) (shared.cu)
 size_t shared_rotate_ws_words(const Context &c, uint32_t n_groups, uint32_t n, uint32_t L);

@@ -22,7 +22,7 @@ constexpr int kMaxAlpha = 16;
 constexpr int kMaxBeta = 16;
 
 // acc[ct][h][j][k] = sum_b up[ct][b][j][perm[k]] * key[b][h][prime(j)][k]   (perm = identity if null);
-// limb j of its own digit j / np is read from d (ModUp leaves it there: it is unchanged)
+// limb j of its own digit j / np is read from d, when given (ModUp leaves it there: it is unchanged)
 // An NTT-domain automorphism maps every aligned block of 32 slots onto an aligned block
 // of 32 slots, so the permuted read of a warp stays within one 256-byte segment.
 // B = beta at compile time: the key rows held in registers for the whole batch are
@@ -41,7 +41,7 @@ __global__ void inner_product_kernel(const uint64_t *__restrict__ up, OwnLimbs d
     const uint32_t LP = L + np, QP = nq + np;
     const uint32_t pj = j < L ? j : nq + (j - L);
     const I ip(pc[pj]);
-    const uint32_t own = j < L ? j / np : B;
+    const uint32_t own = d.p && j < L ? j / np : B;
     typename I::T k0[B], k1[B];
 #pragma unroll
     for (int b = 0; b < B; b++) {
@@ -245,6 +245,22 @@ void modup_into(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n
     ntt_forward_modup(c, mu, up, n_cts, beta, st);
 }
 
+OwnLimbs own_limbs(const Context &c, OwnLimbs d, uint32_t n_cts, uint32_t L, uint64_t *up, const uint64_t *const *outs,
+                   uint32_t n_outs, size_t out_words, cudaStream_t st) {
+    if (n_cts == 0) return d;
+    const uint32_t np = c.np, beta = (L + np - 1) / np, LP = L + np;
+    const size_t n = c.n;
+    const uint64_t *end = d.p + (n_cts - 1) * d.stride + L * n;
+    bool covered = false;
+    for (uint32_t e = 0; e < n_outs; e++) covered = covered || (outs[e] < end && d.p < outs[e] + out_words);
+    if (!covered) return d;
+    for (uint32_t b = 0; b < beta; b++)
+        SHM_CUDA(cudaMemcpy2DAsync(up + (size_t)(b * LP + b * np) * n, (size_t)beta * LP * n * 8, d.p + (size_t)b * np * n,
+                                   d.stride * 8, (size_t)std::min(np, L - b * np) * n * 8, n_cts,
+                                   cudaMemcpyDeviceToDevice, st));
+    return {};
+}
+
 size_t hoisted_ws_words(const Context &c, uint32_t n_cts, uint32_t L) {
     // x, up (kept for every element), acc and a separate delta
     return keyswitch_ws_words(c, n_cts, L) + (size_t)n_cts * 2 * L * c.n;
@@ -268,10 +284,11 @@ void apply_galois_hoisted(const Context &c, const uint64_t *ct, uint32_t n_cts, 
 
     // ModUp once (identical to keyswitch steps 1-3)
     modup_into(c, d, 2 * ln, n_cts, L, x, up, st);
+    const OwnLimbs own = own_limbs(c, {d, 2 * ln}, n_cts, L, up, outs, n_elts - 1, n_cts * 2 * ln, st);
     // per element: permuted inner product, ModDown, combine with sigma(c0)
     for (uint32_t e = 0; e < n_elts; e++) {
         const uint32_t *perm = const_cast<Context &>(c).perm(elts[e]);
-        launch_ip(c, n_cts, L, up, {d, 2 * ln}, keys[e], acc, perm, st);
+        launch_ip(c, n_cts, L, up, own, keys[e], acc, perm, st);
         ntt_inverse(c, acc, special_rows(c, n_cts * 2, L), c.moddown_scale, st);
         KsOutput o{outs[e], outs[e] + ln, ct, nullptr, 2 * ln, perm};
         ntt_forward_moddown(c, moddown_io(c, acc, o), delta, n_cts * 2, L, st);

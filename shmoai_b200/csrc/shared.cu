@@ -284,10 +284,12 @@ void shared_rotate_hoisted(const Context &c, const uint64_t *sh, uint32_t n_grou
     uint64_t *x = ws, *up = x + (size_t)n_groups * ln, *acc = up + (size_t)n_groups * beta * LP * c.n;
     uint64_t *delta = acc + (size_t)n_groups * H * LP * c.n;
     modup_into(c, sh + (size_t)n * ln, (size_t)H * ln, n_groups, L, x, up, st);
+    const OwnLimbs own = own_limbs(c, {sh + (size_t)n * ln, (size_t)H * ln}, n_groups, L, up, outs,
+                                   n_elts ? n_elts - 1 : 0, n_groups * H * ln, st);
     for (uint32_t e = 0; e < n_elts; e++) {
         Target t{keys[e], const_cast<Context &>(c).perm(elts[e]), outs[e], (size_t)H * ln, ln, sh, (size_t)H * ln,
                  ln, n};
-        apply_target(c, up, {sh + (size_t)n * ln, (size_t)H * ln}, n_groups, L, beta, H, t, acc, delta, st);
+        apply_target(c, up, own, n_groups, L, beta, H, t, acc, delta, st);
     }
 }
 
@@ -332,11 +334,13 @@ void fmt_backward(const Context &c, const uint64_t *sh, uint32_t n_groups, uint3
     uint64_t *x = ws, *up = x + (size_t)n_groups * ln, *acc = up + (size_t)n_groups * beta * LP * c.n;
     uint64_t *delta = acc + (size_t)n_groups * 2 * LP * c.n;
     modup_into(c, sh + (size_t)n * ln, (size_t)H * ln, n_groups, L, x, up, st);
+    const OwnLimbs own = own_limbs(c, {sh + (size_t)n * ln, (size_t)H * ln}, n_groups, L, up, &out, n > 1 ? 1 : 0,
+                                   (size_t)n_groups * n * 2 * ln, st);
     for (uint32_t i = 0; i < n; i++) {
         // member i of group g -> ordinary ciphertext g * n + i = (b_i + cx0, cx1)
         Target t{keys[i], nullptr, out + (size_t)i * 2 * ln, (size_t)n * 2 * ln, ln, sh + (size_t)i * ln,
                  (size_t)H * ln, 0, 1};
-        apply_target(c, up, {sh + (size_t)n * ln, (size_t)H * ln}, n_groups, L, beta, 2, t, acc, delta, st);
+        apply_target(c, up, own, n_groups, L, beta, 2, t, acc, delta, st);
     }
 }
 
@@ -433,7 +437,8 @@ void shared_rotate_ext(const Context &c, const uint64_t *in, bool in_ext, uint32
         own = {aq, ln};
     } else {
         modup_into(c, in + (size_t)n * ln, g_words, n_groups, L, x, up, st);
-        own = {in + (size_t)n * ln, g_words};
+        own = own_limbs(c, {in + (size_t)n * ln, g_words}, n_groups, L, up, outs, n_elts, (size_t)n_groups * H * LP * N,
+                        st);
     }
     for (uint32_t e = 0; e < n_elts; e++) {
         const uint32_t *perm = const_cast<Context &>(c).perm(elts[e]);
