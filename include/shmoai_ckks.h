@@ -38,6 +38,14 @@ extern "C" {
 #define SHM_ENOMEM -3   /* device allocation failed */
 #define SHM_EINTERNAL -4
 
+/* Kernels that wait on the tensor cores bound their waits.  The key-switching calls (all that convert between
+ * bases) run asynchronously, so when one of their waits runs out, the call itself has returned: its results are
+ * missing, and SHM_ECUDA is reported by every later call on the context that launches, copies or waits,
+ * shm_graph_launch among them.  shm_synchronize and a shm_memcpy of host memory look after their wait: results
+ * produced before one of them returned SHM_OK are complete.  The state stays: such a context can only be
+ * destroyed (memory, streams and graphs are still released).  shm_ctpt_matmul waits for its own kernels and
+ * reports within the call. */
+
 typedef struct shm_context shm_context;
 
 /* Context over a prime chain given by bit sizes: n_q ciphertext primes then

@@ -129,6 +129,11 @@ class CKKSContext:
             raise
         return Graph(self, g, s)
 
+    def synchronize(self, stream=None):
+        """Wait for the stream; raises if a kernel of an earlier call gave up a wait (torch's own
+        synchronisation does not see that)."""
+        check(lib().shm_synchronize(self._h, _stream(stream)))
+
     # ---------------- helpers ----------------
     def empty(self, *shape) -> torch.Tensor:
         return torch.empty(shape, dtype=torch.int64, device=self.device)

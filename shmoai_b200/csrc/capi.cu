@@ -47,7 +47,6 @@ Context::~Context() {
     for (auto &kv : galois_perm) cudaFree(kv.second);
     for (auto &kv : ext_consts)
         for (void *p : kv.second) cudaFree(p);
-    if (fault) cudaFreeHost(fault);
     if (pool) {
         cudaDeviceSynchronize();
         cudaMemPoolDestroy(pool);
@@ -149,9 +148,11 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
     int sms = 0;
     SHM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     c->sms = (uint32_t)sms;
-    SHM_CUDA(cudaHostAlloc(&c->fault, sizeof(int), cudaHostAllocMapped));
-    *c->fault = 0;
-    SHM_CUDA(cudaHostGetDevicePointer(&c->fault_dev, c->fault, 0));
+    int *fault = nullptr;
+    SHM_CUDA(cudaHostAlloc(&fault, sizeof(int), cudaHostAllocMapped));
+    c->fault = std::shared_ptr<int>(fault, [](int *p) { cudaFreeHost(p); });
+    *fault = 0;
+    SHM_CUDA(cudaHostGetDevicePointer(&c->fault_dev, fault, 0));
     c->log_n = log_n;
     c->n = 1u << log_n;
     c->nq = nq;
@@ -392,6 +393,18 @@ uint64_t *ws_of(shm::Context &c, void *ws, size_t have, size_t need_words) {
 
 void set_device(const shm::Context &c) { SHM_CUDA(cudaSetDevice(c.device)); }
 
+// the start of a call that launches work or copies
+void enter(const shm::Context &c) {
+    set_device(c);
+    shm::check_fault(c.fault.get());
+}
+
+// a synchronising call's wait, after which the stream's results are looked at
+void wait_for(const shm::Context &c, cudaStream_t st) {
+    SHM_CUDA(cudaStreamSynchronize(st));
+    shm::check_fault(c.fault.get());
+}
+
 }  // namespace
 
 extern "C" {
@@ -445,7 +458,7 @@ int shm_ntt_forward(const shm_context *ctx, uint64_t *data, uint32_t n_polys, ui
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_level(c, L);
-        set_device(c);
+        enter(c);
         shm::ntt_forward(c, data, shm::rows_of(c, n_polys, L, L), S(stream));
     });
 }
@@ -454,7 +467,7 @@ int shm_ntt_inverse(const shm_context *ctx, uint64_t *data, uint32_t n_polys, ui
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_level(c, L);
-        set_device(c);
+        enter(c);
         shm::ntt_inverse(c, data, shm::rows_of(c, n_polys, L, L), nullptr, S(stream));
     });
 }
@@ -464,7 +477,7 @@ static int ew(const shm_context *ctx, shm::EwOp op, const uint64_t *a, const uin
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_level(c, L);
-        set_device(c);
+        enter(c);
         shm::elementwise(c, op, a, b, out, n_polys, L, b_polys, S(stream));
     });
 }
@@ -484,7 +497,7 @@ int shm_add_sizes(const shm_context *ctx, const uint64_t *a, uint32_t a_size, co
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_level(c, L);
-        set_device(c);
+        enter(c);
         shm::add_sizes(c, a, a_size, b, b_size, out, n_cts, L, S(stream));
     });
 }
@@ -503,7 +516,7 @@ int shm_multiply(const shm_context *ctx, const uint64_t *a, const uint64_t *b, u
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_level(c, L);
-        set_device(c);
+        enter(c);
         shm::tensor(c, a, b, out, n_cts, L, S(stream));
     });
 }
@@ -515,7 +528,7 @@ int shm_permute_galois(const shm_context *ctx, const uint64_t *in, uint32_t galo
         if (!(galois_elt & 1) || galois_elt >= 2 * c.n) throw std::invalid_argument("Galois element must be odd and < 2N");
         if ((!in || !out) && n_rows) throw std::invalid_argument("null pointer");
         if (in == out && n_rows) throw std::invalid_argument("permute_galois cannot work in place");
-        set_device(c);
+        enter(c);
         shm::apply_galois(c, in, out, n_rows, galois_elt, S(stream));
     });
 }
@@ -527,7 +540,7 @@ int shm_multiply_accumulate(const shm_context *ctx, const uint64_t *const *A, co
         check_level(c, L);
         if ((!A || !B) && k) throw std::invalid_argument("null term arrays");
         if (!out && n_cts) throw std::invalid_argument("null output");
-        set_device(c);
+        enter(c);
         // 2 * chunk products (the middle term) must stay below the Barrett bound 2^(63 + bits(q))
         uint32_t chunk = shm::kMaxAccTerms;
         for (uint32_t i = 0; i < L; i++) {
@@ -562,7 +575,7 @@ int shm_rescale(const shm_context *ctx, const uint64_t *in, uint64_t *out, uint3
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         check_level(c, L);
         if (L < 2 || L > c.nq) throw std::invalid_argument("rescale needs 2 <= L <= n_q limbs");
-        set_device(c);
+        enter(c);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, shm::rescale_ws_words(c, n_polys, L));
         shm::rescale(c, in, out, n_polys, L, ws, S(stream));
     });
@@ -577,7 +590,7 @@ int shm_keyswitch(const shm_context *ctx, const uint64_t *d, const uint64_t *key
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         check_level(c, L);
-        set_device(c);
+        enter(c);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, shm::keyswitch_ws_words(c, n_cts, L));
         const size_t ln = (size_t)L * c.n;
         shm::KsOutput o{out, out + ln, nullptr, nullptr, 2 * ln};
@@ -590,7 +603,7 @@ int shm_relinearize(const shm_context *ctx, const uint64_t *ct3, const uint64_t 
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         check_level(c, L);
-        set_device(c);
+        enter(c);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, shm::keyswitch_ws_words(c, n_cts, L));
         const size_t ln = (size_t)L * c.n;
         if (out == ct3 && n_cts > 1) throw std::invalid_argument("in-place relinearize needs n_cts == 1");
@@ -613,7 +626,7 @@ int shm_relinearize_rescale(const shm_context *ctx, const uint64_t *ct3, const u
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         check_level(c, L);
-        set_device(c);
+        enter(c);
         if (!ct3 || !relin_key || !out) throw std::invalid_argument("null argument");
         const size_t ln = (size_t)L * c.n;
         const uint64_t *a = ct3, *ae = ct3 + (size_t)n_cts * 3 * ln;
@@ -644,7 +657,7 @@ int shm_apply_galois(const shm_context *ctx, const uint64_t *ct, uint32_t galois
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         check_level(c, L);
-        set_device(c);
+        enter(c);
         const size_t ln = (size_t)L * c.n;
         const size_t ks_words = shm::keyswitch_ws_words(c, n_cts, L);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, ks_words + (size_t)n_cts * 2 * ln);
@@ -668,7 +681,7 @@ int shm_apply_galois_hoisted(const shm_context *ctx, const uint64_t *ct, uint32_
         if (!elts || !keys || !outs) throw std::invalid_argument("null element, key or output array");
         for (uint32_t e = 0; e < n_elts; e++)
             if (outs[e] == ct) throw std::invalid_argument("hoisted outputs must not alias the input");
-        set_device(c);
+        enter(c);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, shm::hoisted_ws_words(c, n_cts, L));
         shm::apply_galois_hoisted(c, ct, n_cts, L, n_elts, elts, keys, outs, ws, S(stream));
     });
@@ -687,7 +700,7 @@ int shm_shared_rotate_hoisted(const shm_context *ctx, const uint64_t *sh, uint32
         if (!elts || !keys || !outs || n_members == 0) throw std::invalid_argument("bad shared-a rotation arguments");
         for (uint32_t e = 0; e < n_elts; e++)
             if (outs[e] == sh) throw std::invalid_argument("outputs must not alias the input");
-        set_device(c);
+        enter(c);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, shm::shared_rotate_ws_words(c, n_groups, n_members, L));
         shm::shared_rotate_hoisted(c, sh, n_groups, n_members, L, n_elts, elts, keys, outs, ws, S(stream));
     });
@@ -712,7 +725,7 @@ int shm_shared_rotate(const shm_context *ctx, const uint64_t *sh, uint32_t n_gro
         if (!key || !out || n_members == 0) throw std::invalid_argument("bad shared-a rotation arguments");
         if (out == sh) throw std::invalid_argument("the output must not alias the input");
         if (elt % 2 == 0 || elt >= 2 * c.n) throw std::invalid_argument("Galois element must be odd and below 2N");
-        set_device(c);
+        enter(c);
         const size_t rot = (size_t)n_groups * (n_members + 1) * L * c.n;
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, rot + shm::shared_rotate_ws_words(c, n_groups, n_members, L));
         shm::apply_galois(c, sh, ws, (uint32_t)((size_t)n_groups * (n_members + 1) * L), elt, S(stream));
@@ -735,7 +748,7 @@ int shm_fmt_switch_forward(const shm_context *ctx, const uint64_t *cts, uint32_t
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         check_level(c, L);
         if (!key || n_members == 0) throw std::invalid_argument("bad format-switch arguments");
-        set_device(c);
+        enter(c);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, shm::fmt_forward_ws_words(c, n_groups, n_members, L));
         shm::fmt_forward(c, cts, n_groups, n_members, L, key, out, ws, S(stream));
     });
@@ -753,7 +766,7 @@ int shm_fmt_switch_backward(const shm_context *ctx, const uint64_t *sh, uint32_t
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         check_level(c, L);
         if (!keys || n_members == 0) throw std::invalid_argument("bad format-switch arguments");
-        set_device(c);
+        enter(c);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, shm::fmt_backward_ws_words(c, n_groups, n_members, L));
         shm::fmt_backward(c, sh, n_groups, n_members, L, keys, out, ws, S(stream));
     });
@@ -771,7 +784,7 @@ int shm_extend(const shm_context *ctx, const uint64_t *in, uint64_t *out, uint32
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_ext(c, L);
-        set_device(c);
+        enter(c);
         shm::extend(c, in, out, n_polys, L, S(stream));
     });
 }
@@ -781,7 +794,7 @@ int shm_add_ext(const shm_context *ctx, const uint64_t *a, const uint64_t *b, ui
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_ext(c, L);
-        set_device(c);
+        enter(c);
         shm::add_ext(c, a, b, out, n_polys, L, S(stream));
     });
 }
@@ -795,7 +808,7 @@ int shm_moddown_ext(const shm_context *ctx, uint64_t *ext, uint64_t *out, uint32
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         check_ext(c, L);
-        set_device(c);
+        enter(c);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, shm::moddown_ext_ws_words(c, n_polys, L));
         shm::moddown_ext(c, ext, out, n_polys, L, ws, S(stream));
     });
@@ -808,7 +821,7 @@ int shm_multiply_plain_accumulate_ext(const shm_context *ctx, const uint64_t *co
         auto &c = ctx_of(ctx);
         check_ext(c, L);
         if (!X || !P) throw std::invalid_argument("null term arrays");
-        set_device(c);
+        enter(c);
         // sum of `chunk` products must stay below the Barrett bound 2^(63 + bits(q)) of every limb
         uint32_t chunk = shm::kMaxAccTerms;
         for (uint32_t i = 0; i < L + c.np; i++) {
@@ -834,7 +847,7 @@ int shm_lift_signed_ext(const shm_context *ctx, const int64_t *coeffs, uint64_t 
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_ext(c, L);
-        set_device(c);
+        enter(c);
         shm::lift_signed_ext(c, coeffs, out, n_polys, L, S(stream));
     });
 }
@@ -843,7 +856,7 @@ int shm_ntt_forward_ext(const shm_context *ctx, uint64_t *data, uint32_t n_polys
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_ext(c, L);
-        set_device(c);
+        enter(c);
         const uint32_t LP = L + c.np;
         shm::ntt_forward(c, data, shm::rows_of(c, n_polys, LP, L), S(stream));
     });
@@ -862,7 +875,7 @@ int shm_shared_rotate_ext(const shm_context *ctx, const uint64_t *in, int in_ext
         check_ext(c, L);
         if (n_elts && (!elts || !keys || !outs)) throw std::invalid_argument("null element arrays");
         if (n_members == 0) throw std::invalid_argument("groups need at least one member");
-        set_device(c);
+        enter(c);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, shm::shared_rotate_ext_ws_words(c, n_groups, n_members, L));
         shm::shared_rotate_ext(c, in, in_ext != 0, n_groups, n_members, L, n_elts, elts, keys, outs, ws, S(stream));
     });
@@ -896,7 +909,7 @@ int shm_multiply_scalar(const shm_context *ctx, const uint64_t *a, const uint64_
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_level(c, L);
-        set_device(c);
+        enter(c);
         shm::mul_scalar(c, a, out, scalar_tab(c, scalars, L), n_polys, L, S(stream));
     });
 }
@@ -906,7 +919,7 @@ int shm_add_scalar(const shm_context *ctx, const uint64_t *a, const uint64_t *sc
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_level(c, L);
-        set_device(c);
+        enter(c);
         shm::add_scalar(c, a, out, scalar_tab(c, scalars, L), n_cts, L, S(stream));
     });
 }
@@ -920,7 +933,7 @@ int shm_linear_combination(const shm_context *ctx, const uint64_t *const *X, con
         if (!X || !X_levels || !w) throw std::invalid_argument("null term arrays");
         if (k < 1 || k > (uint32_t)shm::kMaxLinTerms) throw std::invalid_argument("linear combination of 1..8 terms");
         if (L > 64) throw std::invalid_argument("level out of range");
-        set_device(c);
+        enter(c);
         std::unique_ptr<shm::LinTerms> t(new shm::LinTerms{});
         t->k = k;
         for (uint32_t i = 0; i < k; i++) {
@@ -949,7 +962,7 @@ int shm_multiply_plain_accumulate(const shm_context *ctx, const uint64_t *const 
         auto &c = ctx_of(ctx);
         check_level(c, L);
         if (!X || !P) throw std::invalid_argument("null term arrays");
-        set_device(c);
+        enter(c);
         // sum of `chunk` products must stay below the Barrett bound 2^(63 + bits(q))
         uint32_t chunk = shm::kMaxAccTerms;
         for (uint32_t i = 0; i < L; i++) {
@@ -978,7 +991,7 @@ int shm_modraise(const shm_context *ctx, const uint64_t *in, uint64_t *out, uint
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         check_level(c, L);
-        set_device(c);
+        enter(c);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, (size_t)n_polys * c.n);
         shm::modraise(c, in, out, n_polys, L, ws, S(stream));
     });
@@ -990,7 +1003,7 @@ int shm_drop_limbs(const shm_context *ctx, const uint64_t *in, uint64_t *out, ui
         auto &c = ctx_of(ctx);
         check_level(c, L_in);
         if (L_out < 1 || L_out > L_in) throw std::invalid_argument("L_out must be in [1, L_in]");
-        set_device(c);
+        enter(c);
         const size_t n = c.n;
         SHM_CUDA(cudaMemcpy2DAsync(out, L_out * n * 8, in, L_in * n * 8, L_out * n * 8, n_polys,
                                    cudaMemcpyDeviceToDevice, S(stream)));
@@ -1077,16 +1090,17 @@ int shm_memcpy(const shm_context *ctx, void *dst, const void *src, size_t bytes,
                            : kind == SHM_COPY_D2D ? cudaMemcpyDeviceToDevice
                                                   : throw std::invalid_argument("bad copy kind");
         if (!bytes) return;
-        set_device(c);
+        enter(c);
         SHM_CUDA(cudaMemcpyAsync(dst, src, bytes, k, S(stream)));
-        if (kind != SHM_COPY_D2D) SHM_CUDA(cudaStreamSynchronize(S(stream)));  // host buffers may be pageable
+        if (kind != SHM_COPY_D2D) wait_for(c, S(stream));  // host buffers may be pageable
     });
 }
 
 int shm_synchronize(const shm_context *ctx, void *stream) {
     return guard([&] {
-        set_device(ctx_of(ctx));
-        SHM_CUDA(cudaStreamSynchronize(S(stream)));
+        auto &c = ctx_of(ctx);
+        set_device(c);
+        wait_for(c, S(stream));
     });
 }
 
@@ -1114,13 +1128,14 @@ struct shm_graph {
     cudaGraphExec_t exec = nullptr;
     uint64_t kernels = 0;
     int device = 0;
+    std::shared_ptr<int> fault;  // the context's
 };
 
 int shm_graph_begin(const shm_context *ctx, void *stream) {
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         if (!stream) throw std::invalid_argument("the legacy default stream cannot be captured");
-        set_device(c);
+        enter(c);
         // blocks the pool keeps for reuse would sit beside the graph's own allocations
         SHM_CUDA(cudaStreamSynchronize(S(stream)));
         SHM_CUDA(cudaMemPoolTrimTo(c.mempool(), 0));
@@ -1136,6 +1151,7 @@ int shm_graph_end(const shm_context *ctx, void *stream, shm_graph **out) {
         set_device(c);
         std::unique_ptr<shm_graph> g(new shm_graph);
         g->device = c.device;
+        g->fault = c.fault;
         SHM_CUDA(cudaStreamEndCapture(S(stream), &g->graph));
         size_t n = 0;
         SHM_CUDA(cudaGraphGetNodes(g->graph, nullptr, &n));
@@ -1155,6 +1171,7 @@ int shm_graph_end(const shm_context *ctx, void *stream, shm_graph **out) {
 int shm_graph_launch(const shm_graph *g, void *stream) {
     return guard([&] {
         if (!g || !g->exec) throw std::invalid_argument("null graph");
+        shm::check_fault(g->fault.get());
         SHM_CUDA(cudaSetDevice(g->device));
         SHM_CUDA(cudaGraphLaunch(g->exec, S(stream)));
         SHM_LAUNCHED(g->kernels);
@@ -1169,7 +1186,7 @@ int shm_autotune(shm_context *ctx, int knob, uint32_t size, uint32_t level, uint
                  uint32_t cap, uint32_t *chosen) {
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
-        set_device(c);
+        enter(c);
         std::vector<float> ms;
         uint32_t best;
         if (knob == SHM_TUNE_NTT_TILE)
@@ -1201,7 +1218,7 @@ int shm_tune_get(const shm_context *ctx, int knob, uint32_t *index) {
 int shm_tune_set(shm_context *ctx, int knob, uint32_t index) {
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
-        set_device(c);
+        enter(c);
         if (knob == SHM_TUNE_NTT_TILE) {
             if (index >= (uint32_t)shm::kNttVariantCount) throw std::invalid_argument("tile variant out of range");
             SHM_CUDA(cudaDeviceSynchronize());  // launches in flight keep their shape
@@ -1236,7 +1253,7 @@ int shm_sample_uniform(const shm_context *ctx, uint64_t *out, uint32_t n_polys, 
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_level(c, L);
-        set_device(c);
+        enter(c);
         shm::sample_uniform(c, out, n_polys, L, seed, S(stream));
     });
 }
@@ -1246,7 +1263,7 @@ int shm_sample_cbd(const shm_context *ctx, uint64_t *out, uint32_t n_polys, uint
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_level(c, L);
-        set_device(c);
+        enter(c);
         shm::sample_cbd(c, out, n_polys, L, seed, S(stream));
     });
 }
@@ -1260,7 +1277,7 @@ int shm_encode(const shm_context *ctx, const double *re, const double *im, uint3
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         if (n_values && (!re || !im)) throw std::invalid_argument("null slot arrays");
-        set_device(c);
+        enter(c);
         void *ws = ws_of(c, workspace, workspace_bytes, (shm::encode_ws_bytes(c, n_vectors) + 7) / 8);
         if (!shm::encode(c, re, im, n_vectors, n_values, scale, coeffs, ws, S(stream)))
             throw std::invalid_argument("encoded values are too large");
@@ -1271,7 +1288,7 @@ int shm_decode(const shm_context *ctx, const double *coeffs, uint32_t n_vectors,
                void *workspace, size_t workspace_bytes, void *stream) {
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
-        set_device(c);
+        enter(c);
         void *ws = ws_of(c, workspace, workspace_bytes, (shm::encode_ws_bytes(c, n_vectors) + 7) / 8);
         shm::decode(c, coeffs, n_vectors, scale, re, im, ws, S(stream));
     });
@@ -1282,7 +1299,7 @@ int shm_lift_signed(const shm_context *ctx, const int64_t *coeffs, uint64_t *out
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_level(c, L);
-        set_device(c);
+        enter(c);
         shm::lift_signed(c, coeffs, out, n_polys, L, S(stream));
     });
 }
@@ -1296,7 +1313,7 @@ int shm_ctpt_matmul(const shm_context *ctx, const uint64_t *X, const int64_t *W,
     return guard([&] {
         auto &c = const_cast<shm::Context &>(ctx_of(ctx));
         check_level(c, L);
-        set_device(c);
+        enter(c);
         uint64_t *ws = ws_of(c, workspace, workspace_bytes, shm::ctpt_ws_words(c, n_in, n_out, L));
         shm::ctpt_matmul(c, X, W, Y, n_in, n_out, L, ws, S(stream));
     });
@@ -1307,7 +1324,7 @@ int shm_ctpt_matmul_cuda_core(const shm_context *ctx, const uint64_t *X, const i
     return guard([&] {
         auto &c = ctx_of(ctx);
         check_level(c, L);
-        set_device(c);
+        enter(c);
         shm::ctpt_matmul_cuda_core(c, X, W, Y, n_in, n_out, L, S(stream));
     });
 }
@@ -1361,7 +1378,7 @@ extern "C" int shm_rescale_noalloc(const shm_context *ctx, const uint64_t *in, u
         if (need > kNoAllocScratchBytes / 8)
             throw std::invalid_argument("shm_rescale_noalloc: n_polys * L * N exceeds the fixed scratch of " +
                                         std::to_string(kNoAllocScratchBytes / 8) + " words (32 MiB)");
-        set_device(c);
+        enter(c);
         shm::rescale(c, in, out, n_polys, L, noalloc_scratch(c.device), S(stream));
     });
 }

@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstdint>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -93,7 +94,9 @@ struct Context {
     std::map<uint32_t, uint32_t *> galois_perm;  // elt -> [N] permutation
     std::map<uint32_t, std::vector<void *>> ext_consts;  // L -> exact Ql->P extension tables (shared.cu)
     std::mutex mu;
-    int *fault = nullptr, *fault_dev = nullptr;  // set by a kernel whose wait ran out (host-mapped)
+    // Set (and kept) by a kernel whose bounded wait ran out: host-mapped, shared with the graphs that replay it
+    std::shared_ptr<int> fault;
+    int *fault_dev = nullptr;
 
     // internal arena for calls that pass no workspace
     void *arena = nullptr;
@@ -108,6 +111,12 @@ struct Context {
     void *workspace(size_t bytes);
     cudaMemPool_t mempool();
 };
+
+// throws once a kernel has given up a wait: results of calls since the last look may be missing
+inline void check_fault(const int *fault) {
+    if (*(const volatile int *)fault)
+        throw CudaError("a kernel of an earlier call on this context gave up a wait: results since then are missing");
+}
 
 Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uint32_t nq, uint32_t np, int device);
 

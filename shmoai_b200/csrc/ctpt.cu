@@ -91,6 +91,7 @@ void ctpt_matmul(const Context &c, const uint64_t *X, const int64_t *W, uint64_t
     if (mx >= (1ull << 40)) throw std::invalid_argument("ct-pt matmul: |W| must be below 2^40");
     ctpt_matmul_tc(c, X, W, Y, n_in, n_out, L, ws, l1, st);
     if (ctpt_tc_error(ws, st)) throw CudaError("ct-pt matmul: tensor-core pipeline wait timed out");
+    check_fault(c.fault.get());  // the stream has been waited for: X too is what the calls before this one left
 }
 
 }  // namespace shm
