@@ -66,13 +66,16 @@ __device__ __forceinline__ uint64_t mad_low(uint32_t a, uint64_t b, uint32_t lo,
 // Grid: sets x coefficient blocks of `tiles` tiles of kTile.  Dynamic shared memory: the rows' constants
 // (steps of kRows rows), then their RowConst and output rows.  A CTA goes through (tile, step) pairs: wait
 // for the step's sums, read them, issue the next step's MMAs once all four warps have read, convert and
-// store; the next tile's limb words go to the other A buffer during a tile's first step.
-// ALL_FP: every row's butterflies run on doubles (every prime below 2^51).
-template <bool ALL_FP>
+// store; the next tile's limb words go to the other A buffer during a tile's first step.  A thread whose wait runs
+// out stores nothing from then on and sets *fault; the issuing thread issues no more, and its MMAs in flight are
+// waited for (with a bound too) before the TMEM is freed.
+// ALL_FP: every row's butterflies run on doubles (every prime below 2^51).  LIMITED: `limit` polls a wait instead
+// of kSpinLimit (a run-time bound of every wait costs 2 % of the kernel).
+template <bool ALL_FP, bool LIMITED>
 __global__ void __launch_bounds__(kT, 4) conv_kernel(ConvIO io, uint32_t log_n, uint32_t tiles, uint32_t k16,
-                                                     const PrimeConst *__restrict__ pc, int *__restrict__ fault) {
+                                                     const PrimeConst *__restrict__ pc, int *__restrict__ fault, int limit) {
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ __align__(8) uint64_t full;
+    __shared__ __align__(8) uint64_t full, drained;
     __shared__ uint32_t tmem_base;
     const uint32_t tid = threadIdx.x, warp = tid / 32;
     const uint32_t blocks = (1u << log_n) / (kTile * tiles), set = blockIdx.x / blocks, blk = blockIdx.x % blocks;
@@ -147,8 +150,9 @@ __global__ void __launch_bounds__(kT, 4) conv_kernel(ConvIO io, uint32_t log_n, 
     // s32 accumulators, A (TMEM) and B unsigned bytes, K-major, N = 32, M = 128
     const uint32_t idesc = (2u << 4) | ((kRows * 8 >> 3) << 17) | ((128u >> 4) << 24);
     const uint32_t bar = smem_u32(&full), b_addr = smem_u32(smem);
+    bool ok = true;
     auto issue = [&](uint32_t t, uint32_t c) {  // the MMAs of tile t, step c
-        if (tid == 0) {
+        if (tid == 0 && ok) {
 #pragma unroll
             for (uint32_t e = 0; e < kPer; e++)
                 for (uint32_t k = 0; k < nk; k++)
@@ -168,13 +172,12 @@ __global__ void __launch_bounds__(kT, 4) conv_kernel(ConvIO io, uint32_t log_n, 
     issue(0, 0);
     if (tiles > 1) load(1);
 
-    bool ok = true;
     uint32_t phase = 0;
     const uint32_t row_bytes = 8u << log_n;
     char *out = reinterpret_cast<char *>(io.out + (((size_t)set * io.rows) << log_n) + (size_t)blk * tiles * kTile + tid);
     for (uint32_t t = 0; t < tiles; t++, out += kTile * 8) {
         for (uint32_t c = 0; c < steps; c++) {
-            if (ok && !mbar_wait(bar, phase)) ok = false;
+            if (ok && !mbar_wait(bar, phase, LIMITED ? limit : kSpinLimit)) ok = false;
             phase ^= 1;
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;\n");
@@ -222,7 +225,17 @@ __global__ void __launch_bounds__(kT, 4) conv_kernel(ConvIO io, uint32_t log_n, 
             }
         }
     }
-    if (!ok) *fault = 1;
+    if (!ok) {
+        *fault = 1;
+        if (tid == 0) {  // the MMAs in flight
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&drained)));
+            asm volatile("fence.mbarrier_init.release.cluster;\n");
+            asm volatile("fence.proxy.async.shared::cta;\n");
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                smem_u32(&drained)));
+            mbar_wait(smem_u32(&drained), 0);
+        }
+    }
     asm volatile("tcgen05.fence::before_thread_sync;\n");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kCols));
@@ -239,17 +252,20 @@ void conv_rows(const Context &c, const ConvIO &io, cudaStream_t st) {
     while (tiles < 32 && tiles * 2 <= all && (uint64_t)io.sets * (all / (tiles * 2)) >= 16ull * c.sms) tiles *= 2;
     // the last step's rows past the end are in the buffer, unwritten: their sums are not used
     const size_t smem = (io.rows + kRows - 1) / kRows * kRows * (kRowBytes + sizeof(RowConst) + sizeof(uint32_t));
+    const bool fp = c.ntt_families == kFamSmall, limited = c.wait_limit != kSpinLimit;
+    const auto f = limited ? (fp ? conv_kernel<true, true> : conv_kernel<false, true>)
+                           : (fp ? conv_kernel<true, false> : conv_kernel<false, false>);
     static std::atomic<uint64_t> ready{0};  // a bit per device: the attribute belongs to the device's module
     const uint64_t bit = 1ull << (c.device & 63);
     if (!(ready.load(std::memory_order_acquire) & bit)) {
-        for (const void *f : {(const void *)conv_kernel<true>, (const void *)conv_kernel<false>})
-            SHM_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        for (const auto k : {conv_kernel<true, true>, conv_kernel<false, true>, conv_kernel<true, false>,
+                             conv_kernel<false, false>})
+            SHM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         ready.fetch_or(bit, std::memory_order_release);
     }
     SHM_LAUNCHED(1);
     const dim3 grid(io.sets * (all / tiles));
-    if (c.ntt_families == kFamSmall) conv_kernel<true><<<grid, kT, smem, st>>>(io, c.log_n, tiles, 65536u, c.pc, c.fault_dev);
-    else conv_kernel<false><<<grid, kT, smem, st>>>(io, c.log_n, tiles, 65536u, c.pc, c.fault_dev);
+    f<<<grid, kT, smem, st>>>(io, c.log_n, tiles, 65536u, c.pc, c.fault_dev, c.wait_limit);
     SHM_CUDA(cudaGetLastError());
 }
 

@@ -15,6 +15,7 @@
 
 #include "modarith.cuh"
 #include "ntt.cuh"
+#include "tcgen05.cuh"
 
 namespace shm {
 
@@ -97,6 +98,7 @@ struct Context {
     // Set (and kept) by a kernel whose bounded wait ran out: host-mapped, shared with the graphs that replay it
     std::shared_ptr<int> fault;
     int *fault_dev = nullptr;
+    int wait_limit = kSpinLimit;  // polls of a tensor-core kernel's waits
 
     // internal arena for calls that pass no workspace
     void *arena = nullptr;

@@ -258,7 +258,7 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
 __global__ void __launch_bounds__(kThreads, 2) mma_kernel(const int8_t *__restrict__ XP, const int8_t *__restrict__ WP,
                                                           uint8_t *__restrict__ RES, uint32_t Kp, uint32_t Np,
                                                           uint32_t n_out, uint64_t chunk, int *__restrict__ err,
-                                                          int acc_small) {
+                                                          int acc_small, int limit) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], done;
     __shared__ uint32_t tmem_base;
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kThreads, 2) mma_kernel(const int8_t *__restri
         bool ok = true;
         for (uint32_t kb = 0; kb < nkb; kb++) {
             const uint32_t s = kb % kStages;
-            if (kb >= (uint32_t)kStages && !mbar_wait(smem_u32(&empty[s]), ((kb / kStages) - 1) & 1)) ok = false;
+            if (ok && kb >= (uint32_t)kStages && !mbar_wait(smem_u32(&empty[s]), ((kb / kStages) - 1) & 1, limit)) ok = false;
             const uint32_t a_dst = smem_u32(sA + s * kStageA), b_dst = smem_u32(sB + s * kStageB);
             const uint64_t koff = (uint64_t)kb * kKB;
             if (ok) {
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(kThreads, 2) mma_kernel(const int8_t *__restri
         bool ok = true;
         for (uint32_t kb = 0; kb < nkb; kb++) {
             const uint32_t s = kb % kStages;
-            if (!mbar_wait(smem_u32(&full[s]), (kb / kStages) & 1)) ok = false;
+            if (ok && !mbar_wait(smem_u32(&full[s]), (kb / kStages) & 1, limit)) ok = false;
             asm volatile("tcgen05.fence::after_thread_sync;\n");
             if (ok) {
                 const uint32_t a0 = smem_u32(sA + s * kStageA), b0 = smem_u32(sB + s * kStageB);
@@ -351,10 +351,11 @@ __global__ void __launch_bounds__(kThreads, 2) mma_kernel(const int8_t *__restri
     }
     // the idle warps wait here instead of spinning beside the producers and the MMA thread
     __syncthreads();  // also publishes `failed` from the producer and MMA roles
-    const bool landed = mbar_wait(smem_u32(&done), 0);
+    const bool landed = __all_sync(0xffffffffu, mbar_wait(smem_u32(&done), 0, limit));
     asm volatile("tcgen05.fence::after_thread_sync;\n");
     if (!landed || failed) {
-        if (tid == 0) atomicExch(err, 1);
+        if (lane == 0) atomicExch(err, 1);
+        if (!landed) mbar_wait(smem_u32(&done), 0);  // once more, for the MMAs in flight: the TMEM is freed next
     } else {
         // epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (outputs); warpgroup w / 4 takes one
         // half of the 256 X columns, 32 at a time
@@ -399,9 +400,9 @@ __global__ void __launch_bounds__(kThreads, 2) mma_kernel(const int8_t *__restri
 // the A stages, warp w filling ring slot w and arriving on its barrier once its copies land, the
 // next X tile prefetched into L2 meanwhile), one thread of warp 4
 // issues the MMAs, warps 5-12 read the accumulators back (two warps per 32-lane quarter, one
-// per half of the columns).  Every wait is bounded; after a timeout a role waits no more and
-// carries on without its work, still arriving on its barriers, so the other roles finish too,
-// and the call reports the failure through *err.
+// per half of the columns).  Every wait is bounded; a role whose wait runs out leaves its loops, and the
+// others, whose polls look at `failed`, leave theirs.  The loads and MMAs in flight are then waited for (again
+// with a bound) before the CTA frees its TMEM and ends, and the call reports the failure through *err.
 constexpr uint32_t kResKp = 768;
 constexpr int kAStages = 4;  // one ring slot per producer warp
 constexpr uint32_t kXBlock = kBN * kKB;  // 16 KB
@@ -409,6 +410,16 @@ constexpr uint32_t kXTiles = 6;          // most X tiles held at a time
 constexpr uint32_t kSmemP = (kResKp / kKB) * kXBlock + kAStages * kStageA + 1024;
 constexpr uint32_t kEpiWarp0 = 5;
 constexpr uint32_t kThreadsP = (kEpiWarp0 + 8) * 32;
+
+// a role's wait: false, with *failed set, once it or another role's has run out
+__device__ __forceinline__ bool role_wait(uint32_t bar, uint32_t parity, int limit, volatile int *failed) {
+    for (int it = 0; it < limit; it++) {
+        if (mbar_try(bar, parity)) return true;
+        if (*failed) return false;
+    }
+    *failed = 1;
+    return false;
+}
 
 // TMA_A: both operands come by TMA (one thread issues the X tile's and the weight stages' loads,
 // 64-byte swizzle, completion on their mbarriers) instead of the producer warps' cp.async
@@ -418,12 +429,13 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
                                                                       uint8_t *__restrict__ RES, uint32_t Kp,
                                                                       uint32_t Np, uint32_t n_out, uint64_t chunk,
                                                                       uint32_t T, int *__restrict__ err, int acc_small,
+                                                                      int limit,
                                                                       const __grid_constant__ CUtensorMap tmA,
                                                                       const __grid_constant__ CUtensorMap tmX) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);  // swizzle atoms need 1 KB alignment
     __shared__ __align__(8) uint64_t full[kAStages], empty[kAStages], x_full[kXTiles], x_empty[kXTiles], acc_full[2],
-        acc_empty[2];
+        acc_empty[2], drained;
     __shared__ uint32_t tmem_base;
     __shared__ int failed;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -455,6 +467,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&acc_full[b])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&acc_empty[b])), "r"(kEpi));
         }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&drained)));
         asm volatile("fence.mbarrier_init.release.cluster;\n");
         failed = 0;
     }
@@ -463,6 +476,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
     asm volatile("tcgen05.fence::after_thread_sync;\n");
     const uint32_t tmem = tmem_base;
     const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((kBM >> 4) << 24);
+    auto wait = [&](uint64_t *bar, uint32_t parity) { return role_wait(smem_u32(bar), parity, limit, &failed); };
     auto arrive = [](uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar)); };
 
     if (tid < kProducers && !(TMA_A && warp > 0)) {
@@ -476,44 +490,41 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
         uint32_t xi = 0;  // X tiles asked for so far (TMA)
         const uint32_t kx16 = Kp / 16;
         // every MMA of the slot's previous tile must have read it
-        auto x_free = [&](uint32_t i) {
-            return i < ns || mbar_wait(smem_u32(&x_empty[i % ns]), (i / ns - 1) & 1);
-        };
+        auto x_free = [&](uint32_t i) { return i < ns || wait(&x_empty[i % ns], (i / ns - 1) & 1); };
         for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ti++) {
             const uint32_t t = (uint32_t)(tile / n_ct);
             const uint64_t rbase = (tile % n_ct) * kBN;
             if constexpr (TMA_A) {
                 // ahead of this tile's weights: the X tiles whose slots' last readers came two tiles ago
                 if (tid == 0)
-                    for (; xi <= (ns > 1 ? ti + ns - 2 : ti); xi++) {
+                    for (; ok && xi <= (ns > 1 ? ti + ns - 2 : ti); xi++) {
                         const uint64_t xt = blockIdx.x + (uint64_t)xi * gridDim.x;
                         if (xt >= n_tiles) break;
-                        if (ok && !x_free(xi)) ok = false;
-                        const uint32_t bar = smem_u32(&x_full[xi % ns]);
-                        if (ok) {
-                            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar),
-                                         "r"(kBN * Kp));
-                            for (uint32_t kb = 0; kb < nkb; kb++)  // x = kb * 64 bytes: 16-byte aligned
-                                asm volatile(
-                                    "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-                                    "[%0], [%1, {%2, %3}], [%4];\n" ::"r"(smem_u32(sX + (xi % ns * nkb + kb) * kXBlock)),
-                                    "l"(reinterpret_cast<uint64_t>(&tmX)), "r"((int)(kb * kKB)),
-                                    "r"((int)((xt / n_ct) * chunk + (xt % n_ct) * kBN)), "r"(bar)
-                                    : "memory");
-                        } else {
-                            arrive(bar);
+                        if (!x_free(xi)) {
+                            ok = false;
+                            break;
                         }
+                        const uint32_t bar = smem_u32(&x_full[xi % ns]);
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar),
+                                     "r"(kBN * Kp));
+                        for (uint32_t kb = 0; kb < nkb; kb++)  // x = kb * 64 bytes: 16-byte aligned
+                            asm volatile(
+                                "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+                                "[%0], [%1, {%2, %3}], [%4];\n" ::"r"(smem_u32(sX + (xi % ns * nkb + kb) * kXBlock)),
+                                "l"(reinterpret_cast<uint64_t>(&tmX)), "r"((int)(kb * kKB)),
+                                "r"((int)((xt / n_ct) * chunk + (xt % n_ct) * kBN)), "r"(bar)
+                                : "memory");
                     }
-                __syncwarp();
+                ok = __shfl_sync(0xffffffffu, ok, 0);  // thread 0's, also from the tile before
+                if (!ok) break;
             } else {
-                if (ok && !x_free(ti)) ok = false;
+                if (!x_free(ti)) break;
                 const int8_t *B = XP + ((uint64_t)t * chunk + rbase) * Kp;
-                if (ok)
-                    for (uint32_t c = tid; c < kBN * kx16; c += kProducers) {
-                        const uint32_t row = c / kx16, k16 = c % kx16;
-                        cp_async16(smem_u32(sX + (ti % ns * nkb + (k16 >> 2)) * kXBlock) + core_off(row, k16 & 3),
-                                   B + (uint64_t)row * Kp + k16 * 16);
-                    }
+                for (uint32_t c = tid; c < kBN * kx16; c += kProducers) {
+                    const uint32_t row = c / kx16, k16 = c % kx16;
+                    cp_async16(smem_u32(sX + (ti % ns * nkb + (k16 >> 2)) * kXBlock) + core_off(row, k16 & 3),
+                               B + (uint64_t)row * Kp + k16 * 16);
+                }
                 asm volatile("cp.async.commit_group;\n");
                 asm volatile("cp.async.wait_group 0;\n");
                 asm volatile("fence.proxy.async.shared::cta;\n");
@@ -527,75 +538,79 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
                 for (uint32_t off = tid * 128; off < kBN * Kp; off += nthr * 128)
                     asm volatile("prefetch.global.L2 [%0];\n" ::"l"(Bn + off));
             }
-            for (uint32_t o = 0; o < n_ot; o++) {
+            for (uint32_t o = 0; ok && o < n_ot; o++) {
                 const int8_t *A = WP + ((uint64_t)t * Np + o * kBM) * Kp;
                 for (uint32_t kb = 0; kb < nkb; kb++, g++) {
                     const uint32_t s = (uint32_t)(g % kAStages);
-                    if constexpr (TMA_A) {
-                        if (tid != 0) continue;
-                        if (ok && g >= (uint32_t)kAStages && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((g / kAStages) - 1) & 1))
-                            ok = false;
-                        const uint32_t bar = smem_u32(&full[s]);
-                        if (ok) {
-                            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar),
-                                         "r"(kStageA));
-                            // x = kb * 64 bytes: 16-byte aligned as a tiled TMA load requires
-                            asm volatile(
-                                "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-                                "[%0], [%1, {%2, %3}], [%4];\n" ::"r"(smem_u32(sA + s * kStageA)),
-                                "l"(reinterpret_cast<uint64_t>(&tmA)), "r"((int)(kb * kKB)),
-                                "r"((int)(t * Np + o * kBM)), "r"(bar)
-                                : "memory");
-                        } else {
-                            arrive(bar);  // no copy: the barrier still completes
-                        }
-                        continue;
-                    }
-                    if (s != warp) continue;
-                    if (ok && g >= (uint32_t)kAStages && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((g / kAStages) - 1) & 1))
+                    if (TMA_A ? tid != 0 : s != warp) continue;
+                    if (g >= (uint32_t)kAStages && !wait(&empty[s], (uint32_t)((g / kAStages) - 1) & 1)) {
                         ok = false;
-                    if (ok)
+                        break;
+                    }
+                    const uint32_t bar = smem_u32(&full[s]);
+                    if constexpr (TMA_A) {
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar),
+                                     "r"(kStageA));
+                        // x = kb * 64 bytes: 16-byte aligned as a tiled TMA load requires
+                        asm volatile(
+                            "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+                            "[%0], [%1, {%2, %3}], [%4];\n" ::"r"(smem_u32(sA + s * kStageA)),
+                            "l"(reinterpret_cast<uint64_t>(&tmA)), "r"((int)(kb * kKB)),
+                            "r"((int)(t * Np + o * kBM)), "r"(bar)
+                            : "memory");
+                    } else {
                         for (uint32_t c = lane; c < kBM * (kKB / 16); c += 32) {
                             const uint32_t row = c / (kKB / 16), kc = c % (kKB / 16);
                             cp_async16(smem_u32(sA + s * kStageA) + core_off(row, kc),
                                        A + (uint64_t)row * Kp + (uint64_t)kb * kKB + kc * 16);
                         }
-                    asm volatile("cp.async.commit_group;\n");
-                    asm volatile("cp.async.wait_group 0;\n");
-                    asm volatile("fence.proxy.async.shared::cta;\n");
-                    arrive(smem_u32(&full[s]));
+                        asm volatile("cp.async.commit_group;\n");
+                        asm volatile("cp.async.wait_group 0;\n");
+                        asm volatile("fence.proxy.async.shared::cta;\n");
+                        arrive(bar);
+                    }
                 }
             }
+            if (!TMA_A && !ok) break;
         }
-        if (!ok) failed = 1;
+        if (TMA_A && tid == 0) {  // every load asked for has landed (normally long ago) before the CTA can end
+            for (uint32_t s = 0; s < (uint32_t)kAStages; s++)
+                if (g > s) mbar_wait(smem_u32(&full[s]), ((g - 1 - s) / kAStages) & 1);
+            for (uint32_t x = 0; x < ns; x++)
+                if (xi > x) mbar_wait(smem_u32(&x_full[x]), ((xi - 1 - x) / ns) & 1);
+        }
     } else if (tid == kProducers) {
         bool ok = true;
         uint32_t g = 0, ti = 0, ai = 0;  // A stages, column tiles, accumulator tiles
-        for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ti++) {
+        for (uint64_t tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x, ti++) {
             const uint32_t xs = ti % ns;
-            if (ok && !mbar_wait(smem_u32(&x_full[xs]), (ti / ns) & 1)) ok = false;
+            ok = wait(&x_full[xs], (ti / ns) & 1);
             asm volatile("tcgen05.fence::after_thread_sync;\n");
-            for (uint32_t o = 0; o < n_ot; o++, ai++) {
+            for (uint32_t o = 0; ok && o < n_ot; o++, ai++) {
                 const uint32_t buf = ai & 1;
-                if (ok && ai >= 2 && !mbar_wait(smem_u32(&acc_empty[buf]), ((ai >> 1) - 1) & 1)) ok = false;
+                if (ai >= 2 && !wait(&acc_empty[buf], ((ai >> 1) - 1) & 1)) {
+                    ok = false;
+                    break;
+                }
                 asm volatile("tcgen05.fence::after_thread_sync;\n");
                 for (uint32_t kb = 0; kb < nkb; kb++, g++) {
                     const uint32_t s = (uint32_t)(g % kAStages);
-                    if (ok && !mbar_wait(smem_u32(&full[s]), (uint32_t)(g / kAStages) & 1)) ok = false;
+                    if (!wait(&full[s], (uint32_t)(g / kAStages) & 1)) {
+                        ok = false;
+                        break;
+                    }
                     asm volatile("tcgen05.fence::after_thread_sync;\n");
-                    if (ok) {
-                        const uint32_t a0 = smem_u32(sA + s * kStageA), b0 = smem_u32(sX + (xs * nkb + kb) * kXBlock);
+                    const uint32_t a0 = smem_u32(sA + s * kStageA), b0 = smem_u32(sX + (xs * nkb + kb) * kXBlock);
 #pragma unroll
-                        for (uint32_t k = 0; k < kKB / 32; k++) {
-                            const uint64_t ad = TMA_A ? smem_desc_sw64(a0 + k * 32) : smem_desc(a0 + k * 256);
-                            const uint64_t bd = TMA_A ? smem_desc_sw64(b0 + k * 32) : smem_desc(b0 + k * 256);
-                            const uint32_t accum = (kb | k) ? 1u : 0u;
-                            asm volatile(
-                                "{\n\t.reg .pred p;\n\t"
-                                "setp.ne.b32 p, %4, 0;\n\t"
-                                "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem + buf * kBN),
-                                "l"(ad), "l"(bd), "r"(idesc), "r"(accum));
-                        }
+                    for (uint32_t k = 0; k < kKB / 32; k++) {
+                        const uint64_t ad = TMA_A ? smem_desc_sw64(a0 + k * 32) : smem_desc(a0 + k * 256);
+                        const uint64_t bd = TMA_A ? smem_desc_sw64(b0 + k * 32) : smem_desc(b0 + k * 256);
+                        const uint32_t accum = (kb | k) ? 1u : 0u;
+                        asm volatile(
+                            "{\n\t.reg .pred p;\n\t"
+                            "setp.ne.b32 p, %4, 0;\n\t"
+                            "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem + buf * kBN),
+                            "l"(ad), "l"(bd), "r"(idesc), "r"(accum));
                     }
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
                         smem_u32(&empty[s])));
@@ -606,53 +621,59 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
                 smem_u32(&x_empty[xs])));
         }
-        if (!ok) failed = 1;
     } else if (warp >= kEpiWarp0) {
         bool ok = true;
         const uint32_t quarter = warp & 3, half = (warp - kEpiWarp0) >> 2;
         uint32_t ai = 0;
-        for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+        for (uint64_t tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x) {
             const uint32_t t = (uint32_t)(tile / n_ct);
             const uint64_t rbase = (tile % n_ct) * kBN;
             for (uint32_t o = 0; o < n_ot; o++, ai++) {
                 const uint32_t buf = ai & 1;
-                if (ok && !mbar_wait(smem_u32(&acc_full[buf]), (ai >> 1) & 1)) ok = false;
+                ok = __all_sync(0xffffffffu, wait(&acc_full[buf], (ai >> 1) & 1));
+                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n");
                 const uint32_t out = o * kBM + quarter * 32 + lane;
-                if (ok) {
-                    for (uint32_t c0 = half * (kBN / 2); c0 < (half + 1) * (kBN / 2); c0 += 32) {
-                        uint32_t v[32];
-                        const uint32_t taddr = tmem + ((quarter * 32) << 16) + buf * kBN + c0;
-                        asm volatile(
-                            "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                            "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                              "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                              "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
-                              "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
-                              "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                            : "r"(taddr));
-                        asm volatile("tcgen05.wait::ld.sync.aligned;\n");
-                        if (out < n_out) {
-                            uint32_t pk[8];
+                for (uint32_t c0 = half * (kBN / 2); c0 < (half + 1) * (kBN / 2); c0 += 32) {
+                    uint32_t v[32];
+                    const uint32_t taddr = tmem + ((quarter * 32) << 16) + buf * kBN + c0;
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+                        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+                          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+                          "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
+                          "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
+                          "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                        : "r"(taddr));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n");
+                    if (out < n_out) {
+                        uint32_t pk[8];
 #pragma unroll
-                            for (int j = 0; j < 8; j++) pk[j] = acc_bytes(v + 4 * j, t, acc_small);
-                            uint4 *dst = reinterpret_cast<uint4 *>(RES + ((uint64_t)t * n_out + out) * chunk + rbase + c0);
-                            dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                            dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-                        }
+                        for (int j = 0; j < 8; j++) pk[j] = acc_bytes(v + 4 * j, t, acc_small);
+                        uint4 *dst = reinterpret_cast<uint4 *>(RES + ((uint64_t)t * n_out + out) * chunk + rbase + c0);
+                        dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                        dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
                     }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;\n");
                 arrive(smem_u32(&acc_empty[buf]));
             }
         }
-        if (!ok) failed = 1;
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n");
     __syncthreads();
-    if (tid == 0 && failed) atomicExch(err, 1);
+    if (failed) {
+        if (tid == 0) atomicExch(err, 1);
+        if (tid == kProducers) {  // the MMAs in flight
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                smem_u32(&drained)));
+            mbar_wait(smem_u32(&drained), 0);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\n");
+        __syncthreads();
+    }
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(2 * kBN));
 }
 
@@ -1031,13 +1052,15 @@ void ctpt_matmul_tc(const Context &c, const uint64_t *X, const int64_t *W, uint6
             const bool tma = tma_a && operand_tensor_map(&tmX, XP, Kp, (uint64_t)Tc * cur, kBN);
             if (tma)
                 mma_persistent_kernel<true>
-                    <<<grid, kThreadsP, kSmemP, st>>>(XP, WP, RES, Kp, Np, n_out, cur, Tc, err, acc_small, tmA, tmX);
+                    <<<grid, kThreadsP, kSmemP, st>>>(XP, WP, RES, Kp, Np, n_out, cur, Tc, err, acc_small, c.wait_limit,
+                                                      tmA, tmX);
             else
                 mma_persistent_kernel<false>
-                    <<<grid, kThreadsP, kSmemP, st>>>(XP, WP, RES, Kp, Np, n_out, cur, Tc, err, acc_small, tmA, tmX);
+                    <<<grid, kThreadsP, kSmemP, st>>>(XP, WP, RES, Kp, Np, n_out, cur, Tc, err, acc_small, c.wait_limit,
+                                                      tmA, tmX);
         } else {
             mma_kernel<<<dim3(Np / kBM, (uint32_t)(cur / kBN), Tc), kThreads, kSmem, st>>>(XP, WP, RES, Kp, Np, n_out,
-                                                                                          cur, err, acc_small);
+                                                                                          cur, err, acc_small, c.wait_limit);
         }
         SHM_CUDA(cudaGetLastError());
         SHM_LAUNCHED(1);
