@@ -47,7 +47,7 @@ __global__ void add_scalar_kernel(const uint64_t *__restrict__ a, uint64_t *__re
 // Limb-major block order: blockIdx.y = limb * n_polys + poly, so the polynomials that share a
 // plaintext limb run together and the k plaintext limbs stay in L2 for all of them.
 // L = limbs per row; limb l uses prime l when l < Lq, else the special prime nq + l - Lq
-template <bool S52>
+template <int KIND>
 __global__ void mul_plain_acc_kernel(PtrTab X, PtrTab P, uint32_t k, uint64_t *__restrict__ out, uint32_t L,
                                      uint32_t log_n, const PrimeConst *__restrict__ pc, int accumulate, uint32_t Lq,
                                      uint32_t nq) {
@@ -55,7 +55,7 @@ __global__ void mul_plain_acc_kernel(PtrTab X, PtrTab P, uint32_t k, uint64_t *_
     const PrimeConst p = pc[limb < Lq ? limb : nq + (limb - Lq)];
     const size_t off = ((size_t)row << log_n) + blockIdx.x * kT + threadIdx.x;
     const size_t poff = ((size_t)limb << log_n) + blockIdx.x * kT + threadIdx.x;
-    Acc<S52> acc;
+    Acc<KIND> acc;
     // unrolled so that a group of terms' loads is in flight together (the loads, not the
     // multiplies, bound this kernel)
 #pragma unroll 8
@@ -127,7 +127,7 @@ void mul_plain_acc(const Context &c, const PtrTab &X, const PtrTab &P, uint32_t 
     if (!n_polys || !k) return;
     const uint32_t rows = ext ? L + c.np : L;
     SHM_LAUNCHED(1);
-    const auto f = c.s52 ? mul_plain_acc_kernel<true> : mul_plain_acc_kernel<false>;
+    const auto f = c.acc == kAccHalves ? mul_plain_acc_kernel<kAccHalves> : mul_plain_acc_kernel<kAccWide>;
     f<<<dim3(c.n / kT, n_polys * rows), kT, 0, st>>>(X, P, k, out, rows, c.log_n, c.pc, accumulate ? 1 : 0, L, c.nq);
     SHM_CUDA(cudaGetLastError());
 }

@@ -166,8 +166,10 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
         if (np && (uint64_t)np * q >= (1ull << 63))
             throw std::invalid_argument("alpha * q must stay below 2^63 for the lazy base conversion");
     }
-    c->s52 = *std::max_element(primes.begin(), primes.end()) < kS52PrimeLimit &&
-             *std::min_element(primes.begin(), primes.end()) >= kS52PrimeMin;
+    if (*std::max_element(primes.begin(), primes.end()) < kS52PrimeLimit) {
+        c->acc = *std::min_element(primes.begin(), primes.end()) >= kHalvesMin ? kAccHalves : kAccWide;
+        c->split_acc = kAccSplit;
+    }
     {
         int fam = 0;
         for (uint64_t q : primes) fam |= 1 << bf_mode_of(q);

@@ -75,7 +75,8 @@ struct Context {
     uint32_t sms = 148;                 // multiprocessors of the device
     uint32_t log_n = 0, n = 0, nq = 0, np = 0, dnum = 0;
     std::vector<uint64_t> primes;       // nq + np
-    bool s52 = false;                   // every prime in [kS52PrimeMin, kS52PrimeLimit) (Acc<true> kernels)
+    int acc = kAccWide;                 // how inner products and plaintext sums are held (Acc): in halves, or wide
+    int split_acc = kAccWide;           // the tensor products' and base conversions' sums: split, or wide
     int ntt_variant = kNttDefault;      // index into kNttVariants (set by the autotuner)
     int ntt_families = 0;               // the NTT instantiation for the primes' butterfly families (kFam*)
     uint32_t ip_chunk_bytes = 32768;    // shared memory per Sh-Rot inner-product block (autotuned)
@@ -249,13 +250,13 @@ void lift_signed(const Context &c, const int64_t *in, uint64_t *out, uint32_t n_
 
 // How an inner product of `beta` digits with key rows is summed: on doubles when every prime is below 2^51
 // and the digits fit AccDbl (the bootstrapping chains), in 26-bit halves for the other chains of
-// Context::s52, else in 128 bits.
-constexpr int kIpWide = 0, kIpS52 = 1, kIpDbl = 2;
+// Context::acc kAccHalves, else in 128 bits.
+constexpr int kIpWide = 0, kIpHalves = 1, kIpDbl = 2;
 
 template <int A>
 struct IpSum {
-    using Acc = shm::Acc<A == kIpS52>;
-    using Op = Operand<A == kIpS52>;
+    using Acc = shm::Acc<A == kIpHalves ? kAccHalves : kAccWide>;
+    using Op = Operand<A == kIpHalves ? kAccHalves : kAccWide>;
     using T = typename Op::type;
     const PrimeConst p;
     __device__ __forceinline__ explicit IpSum(const PrimeConst &p_) : p(p_) {}
@@ -283,7 +284,7 @@ void ip_dispatch(const Context &c, uint32_t beta, F &&f) {
         constexpr int B = decltype(b)::value;
         if constexpr (B <= kMaxDblTerms)
             if (c.ntt_families == kFamSmall) return f(b, std::integral_constant<int, kIpDbl>{});
-        if (c.s52) f(b, std::integral_constant<int, kIpS52>{});
+        if (c.acc == kAccHalves) f(b, std::integral_constant<int, kIpHalves>{});
         else f(b, std::integral_constant<int, kIpWide>{});
     };
 #define SHM_IP_CASE(B) \

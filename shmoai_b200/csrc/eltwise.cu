@@ -79,8 +79,8 @@ __global__ void tensor_kernel(const uint64_t *__restrict__ a, const uint64_t *__
 // out[ct] (+)= sum_{t < k} A_t[ct a_step] x B_t[ct b_step]: the size-3 tensor products of k
 // ciphertext pairs summed before one reduction (step 0 broadcasts one ciphertext over the batch).
 // The host bounds k so that each sum (2k products for the middle term) stays below the Barrett
-// bound; S52: Context::s52.
-template <bool S52>
+// bound; KIND: Context::split_acc.
+template <int KIND>
 __global__ void tensor_acc_kernel(PtrTab A, PtrTab B, uint32_t k, uint32_t a_step, uint32_t b_step,
                                   uint64_t *__restrict__ out, uint32_t L, uint32_t log_n,
                                   const PrimeConst *__restrict__ pc, int accumulate) {
@@ -88,11 +88,10 @@ __global__ void tensor_acc_kernel(PtrTab A, PtrTab B, uint32_t k, uint32_t a_ste
     const PrimeConst p = pc[limb];
     const size_t ln = (size_t)L << log_n;
     const size_t kk = ((size_t)limb << log_n) + blockIdx.x * kEwThreads + threadIdx.x;
-    Acc<S52> s0, s1, s2;
+    Acc<KIND> s0, s1, s2;
     for (uint32_t t = 0; t < k; t++) {
         const uint64_t *a = A.p[t] + (size_t)ct * a_step * 2 * ln, *b = B.p[t] + (size_t)ct * b_step * 2 * ln;
-        using Op = Operand<S52>;
-        const auto a0 = Op::of(a[kk]), a1 = Op::of(a[ln + kk]), b0 = Op::of(b[kk]), b1 = Op::of(b[ln + kk]);
+        const uint64_t a0 = a[kk], a1 = a[ln + kk], b0 = b[kk], b1 = b[ln + kk];
         s0.add(a0, b0);
         s1.add(a0, b1);
         s1.add(a1, b0);
@@ -162,12 +161,8 @@ void tensor_accumulate(const Context &c, const PtrTab &A, const PtrTab &B, uint3
     if (n_cts == 0 || k == 0) return;
     const dim3 grid(c.n / kEwThreads, L, n_cts);
     SHM_LAUNCHED(1);
-    if (c.s52)
-        tensor_acc_kernel<true><<<grid, kEwThreads, 0, st>>>(A, B, k, a_step, b_step, out, L, c.log_n, c.pc,
-                                                             accumulate ? 1 : 0);
-    else
-        tensor_acc_kernel<false><<<grid, kEwThreads, 0, st>>>(A, B, k, a_step, b_step, out, L, c.log_n, c.pc,
-                                                              accumulate ? 1 : 0);
+    const auto f = c.split_acc == kAccSplit ? tensor_acc_kernel<kAccSplit> : tensor_acc_kernel<kAccWide>;
+    f<<<grid, kEwThreads, 0, st>>>(A, B, k, a_step, b_step, out, L, c.log_n, c.pc, accumulate ? 1 : 0);
     SHM_CUDA(cudaGetLastError());
 }
 

@@ -106,7 +106,7 @@ ModDownIO moddown_io(const Context &c, const uint64_t *acc, const KsOutput &o) {
     md.n_perm = 1;
     md.H = 2;
     md.np = c.np;
-    md.s52 = c.s52 ? 1 : 0;
+    md.sums = c.split_acc;
     md.bytes = c.moddown_bytes;
     return md;
 }
@@ -188,7 +188,7 @@ void relin_rescale(const Context &c, const uint64_t *ct3, uint32_t n_cts, uint32
     md.n_add = 2;
     md.H = 2;
     md.np = np + 1;
-    md.s52 = c.s52 ? 1 : 0;
+    md.sums = c.split_acc;
     md.bytes = ks.rr_bytes;
     md.vrow = vrow;
     md.vs = ks.rr_vs;
@@ -240,7 +240,7 @@ void modup_into(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n
     mu.L = L;
     mu.np = np;
     mu.LP = LP;
-    mu.s52 = c.s52 ? 1 : 0;
+    mu.sums = c.split_acc;
     mu.bytes = ks.modup_bytes;
     ntt_forward_modup(c, mu, up, n_cts, beta, st);
 }

@@ -20,7 +20,7 @@ struct PrimeConst {
     uint32_t red_m;  // floor(2^(32+s) / q), s = max(0, k - 25): the multiplier of reduce_small
     uint64_t n_inv;        // N^-1 mod q
     uint64_t n_inv_shoup;  // Shoup companion of n_inv
-    double qinv;           // 1 / q rounded (the FP64 paths; primes below 2^51)
+    double qinv;           // 1 / q rounded
 };
 
 __device__ __forceinline__ uint64_t mulhi64(uint64_t a, uint64_t b) { return __umul64hi(a, b); }
@@ -84,21 +84,32 @@ __device__ __forceinline__ uint64_t barrett(u128 x, const PrimeConst &p) {
     return csub(r, p.q);
 }
 
-// Sum of products: Acc<false> for any operands (a 128-bit accumulator, one Barrett reduction), or
-// Acc<true> for residues of primes in [2^40, 2^52).  There an operand is split at bit 26 into halves
-// below 2^26, and the 32 x 32-bit products go into three 64-bit sums of weights 1, 2^26 and 2^52 (hi,
-// mid, lo; no overflow below 2^10 terms): four wide multiply-adds per term with nothing beside them (split
-// at bit 32, each term's low product had to be taken apart and added in two places).  reduce() takes two
-// quotients from the FP64 pipe: hi 2^26 and then ((hi 2^26 mod q) + mid) 2^26 + lo are each brought within
-// about q/2 of zero.  With n terms both quotients stay below n 2^27, far inside the 2^51 that the rounding
-// through 1.5 2^52 takes exactly, and their errors (two roundings of a double) below 2^-17.  A 64 x 64-bit
-// high product as Barrett's quotient needs issues at 7 a clock per SM, a wide multiply at 32.
-constexpr uint64_t kS52PrimeMin = 1ull << 40, kS52PrimeLimit = 1ull << 52;
+// Sums of products, by how the terms are held:
+//
+// kAccWide: any operands; a 128-bit accumulator, one Barrett reduction.
+//
+// kAccHalves: residues of one prime in [2^28, 2^52), split at bit 26 into halves below 2^26; the 32 x 32-bit
+// products go into three 64-bit sums of weights 1, 2^26 and 2^52 (lo, mid, hi; no overflow below 2^10 terms): four
+// wide multiply-adds per term with nothing beside them.  reduce() takes two quotients from the FP64 pipe: hi 2^26
+// and then ((hi 2^26 mod q) + mid) 2^26 + lo are each brought within about q/2 of zero; a 64 x 64-bit high product as
+// Barrett's quotient needs issues at 7 a clock per SM, a wide multiply at 32.  With n <= 64 terms the quotients
+// stay below n 2^28 (the rounding through 1.5 2^52 takes 2^51 exactly), their errors (two roundings of a double)
+// below 2^-17, and lo's 26 bits, which the second quotient leaves out, below q / 4.
+//
+// kAccSplit: operands below 2^52, split at bit 32: hi = sum a1 b1, mid = sum (a0 b1 + a1 b0 + hi32(a0 b0)),
+// lo = sum lo32(a0 b0), no overflow below 2^11 terms; four wide multiplies and no carry chain per term, one fold and
+// one Barrett reduction at the end.  For the sums whose reduction kAccHalves does not shorten: the tensor
+// products' (eight sums of four at 35 limbs 485 us, in halves 508: they read and write more than they multiply) and
+// the base conversions' in the transform's load, whose operands belong to different primes besides (eight key
+// switches of 18 limbs in digits of nine 1.35 ms, in halves 1.34, in 128 bits 1.60).
+constexpr int kAccWide = 0, kAccHalves = 1, kAccSplit = 2;
+constexpr uint64_t kS52PrimeLimit = 1ull << 52;    // kAccHalves, kAccSplit
+constexpr uint64_t kHalvesMin = 1ull << 28;        // kAccHalves
 constexpr uint32_t kMask26 = (1u << 26) - 1;
 
 __device__ __forceinline__ uint2 split26(uint64_t a) { return make_uint2((uint32_t)a & kMask26, (uint32_t)(a >> 26)); }
 
-template <bool S52>
+template <int KIND>
 struct Acc {
     u128 v{0, 0};
     __device__ __forceinline__ void add(uint64_t a, uint64_t b) { mac(v, a, b); }
@@ -106,7 +117,23 @@ struct Acc {
 };
 
 template <>
-struct Acc<true> {
+struct Acc<kAccSplit> {
+    uint64_t lo = 0, mid = 0, hi = 0;
+    __device__ __forceinline__ void add(uint64_t a, uint64_t b) {
+        const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
+        const uint64_t t = (uint64_t)a0 * b0;
+        lo += (uint32_t)t;
+        mid += (t >> 32) + (uint64_t)a0 * b1 + (uint64_t)a1 * b0;
+        hi += (uint64_t)a1 * b1;
+    }
+    __device__ __forceinline__ uint64_t reduce(const PrimeConst &p) const {
+        const uint64_t l = lo + (mid << 32);
+        return barrett({l, hi + (mid >> 32) + (l < lo ? 1 : 0)}, p);
+    }
+};
+
+template <>
+struct Acc<kAccHalves> {
     uint64_t lo = 0, mid = 0, hi = 0;
     __device__ __forceinline__ void add(uint2 a, uint2 b) {
         lo += (uint64_t)a.x * b.x;
@@ -128,13 +155,13 @@ struct Acc<true> {
 };
 
 // an operand as the accumulator takes it
-template <bool S52>
+template <int KIND>
 struct Operand {
     using type = uint64_t;
     __device__ __forceinline__ static type of(uint64_t a) { return a; }
 };
 template <>
-struct Operand<true> {
+struct Operand<kAccHalves> {
     using type = uint2;
     __device__ __forceinline__ static type of(uint64_t a) { return split26(a); }
 };

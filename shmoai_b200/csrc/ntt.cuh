@@ -83,7 +83,7 @@ struct ModDownIO {
     const uint64_t *vs = nullptr;  // [slots][16]
     long long out_ct = 0, out_h = 0, add_ct = 0, add_h = 0;  // word strides
     uint32_t H = 2, np = 0, n_add = 0, n_perm = 0;
-    int s52 = 0;  // Context::s52: Acc<true>
+    int sums = 0;  // Context::split_acc
     const uint8_t *bytes = nullptr;  // the conversion's (and v's) constants for ConvIO; null: the load transform
 };
 
@@ -96,7 +96,7 @@ struct ModUpIO {
     const uint64_t *x = nullptr;     // [n_cts][L][N]
     const uint64_t *conv = nullptr;  // [beta][LP][np]: qhat_i mod t_j of the level's digits
     uint32_t L = 0, np = 0, LP = 0;
-    int s52 = 0;
+    int sums = 0;
     const uint8_t *bytes = nullptr;  // as ModDownIO's
 };
 

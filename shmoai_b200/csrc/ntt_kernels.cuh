@@ -46,19 +46,24 @@ struct Limb {
 // sum_{i < n} x[i << log_n] c[i] mod p (a base conversion's term for one coefficient; n <= 16).  The
 // first eight terms' loads are issued together before any product, so one load latency is exposed
 // per coefficient instead of one per term.
-template <bool S52>
+template <int KIND>
 __device__ __forceinline__ uint64_t conv_sum(const uint64_t *__restrict__ x, const uint64_t *c, uint32_t n,
                                              int log_n, const PrimeConst &p) {
     constexpr uint32_t kBatch = 8;
     uint64_t v[kBatch];
 #pragma unroll
     for (uint32_t i = 0; i < kBatch; i++) v[i] = i < n ? x[(size_t)i << log_n] : 0;
-    Acc<S52> acc;
+    Acc<KIND> acc;
 #pragma unroll
     for (uint32_t i = 0; i < kBatch; i++)
         if (i < n) acc.add(v[i], c[i]);
     for (uint32_t i = kBatch; i < n; i++) acc.add(x[(size_t)i << log_n], c[i]);
     return acc.reduce(p);
+}
+
+__device__ __forceinline__ uint64_t conv_sum(int kind, const uint64_t *__restrict__ x, const uint64_t *c, uint32_t n,
+                                             int log_n, const PrimeConst &p) {
+    return kind == kAccSplit ? conv_sum<kAccSplit>(x, c, n, log_n, p) : conv_sum<kAccWide>(x, c, n, log_n, p);
 }
 
 // CTAs are issued limb-major: consecutive CTAs work on the same slot (one prime) of successive
@@ -98,8 +103,7 @@ __global__ void __launch_bounds__(Geo<R, S>::THREADS, MINB)
 #pragma unroll
         for (int m = 0; m < G::E; m++) {
             const size_t pos = sig + (size_t)G::M * (lane + m * G::E);
-            a[m] = mu.s52 ? conv_sum<true>(y + pos, sconv, na, G::LOGN, p)
-                          : conv_sum<false>(y + pos, sconv, na, G::LOGN, p);
+            a[m] = conv_sum(mu.sums, y + pos, sconv, na, G::LOGN, p);
         }
     } else if constexpr (IOK == kIoRescale) {
         const PrimeConst p = pc[pidx];
@@ -117,8 +121,7 @@ __global__ void __launch_bounds__(Geo<R, S>::THREADS, MINB)
 #pragma unroll
         for (int m = 0; m < G::E; m++) {
             const size_t pos = sig + (size_t)G::M * (lane + m * G::E);
-            a[m] = io.md.s52 ? conv_sum<true>(z + pos, sconv, np, G::LOGN, p)
-                             : conv_sum<false>(z + pos, sconv, np, G::LOGN, p);
+            a[m] = conv_sum(io.md.sums, z + pos, sconv, np, G::LOGN, p);
         }
         if (io.md.vrow) {
             const uint8_t *vr = io.md.vrow + ((size_t)poly << G::LOGN) + chunk * S;

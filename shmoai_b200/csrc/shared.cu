@@ -262,7 +262,7 @@ void apply_target(const Context &c, const uint64_t *up, OwnLimbs own, uint32_t n
     md.n_perm = md.n_add;
     md.H = H;
     md.np = np;
-    md.s52 = c.s52 ? 1 : 0;
+    md.sums = c.split_acc;
     md.bytes = c.moddown_bytes;
     ntt_forward_moddown(c, md, delta, n_cts * H, L, st);
 }
@@ -379,7 +379,7 @@ void moddown_rows(const Context &c, uint64_t *ext, uint64_t *out, uint32_t n_pol
     md.out_ct = (long long)L * c.n;
     md.H = 1;
     md.np = c.np;
-    md.s52 = c.s52 ? 1 : 0;
+    md.sums = c.split_acc;
     md.bytes = c.moddown_bytes;
     ntt_forward_moddown(c, md, delta, n_polys, L, st);
 }
