@@ -398,10 +398,21 @@ void launch_fwd_v(const Context &c, uint64_t *data, const NttRows &rw, cudaStrea
     constexpr int BLK = IOK == kIoModUp ? kIoPlain : IOK;  // ModUp's block phase is a plain one
     SHM_LAUNCHED(1);
     // rows converted by conv_rows: the plain column phase, whose input is in the butterflies' form
-    if ((IOK == kIoModUp || IOK == kIoModDown) && io.converted)
-        fwd_col<R, S, MINB, kIoConverted, FAM><<<grid, G::THREADS, 0, st>>>(data, rw, c.tw, c.twd, c.pc, io);
-    else
+    if constexpr (IOK == kIoModUp || IOK == kIoModDown) {
+        if (io.converted) {
+            fwd_col<R, S, MINB, kIoConverted, FAM><<<grid, G::THREADS, 0, st>>>(data, rw, c.tw, c.twd, c.pc, io);
+        } else {
+            // a conversion in the loads (more than eight limbs) waits for them longer than the 24 warps an SM of
+            // 8 x 6 cover: 18 limbs in digits of nine, eight key switches at 50 bits 1.35 ms with 8 x 6, 1.11 with
+            // 16 x 4 here; one at 58 bits 366 and 299 us
+            constexpr int SC = MINB == 6 ? 16 : S, MC = MINB == 6 ? 4 : MINB;
+            using GC = Geo<R, SC>;
+            const dim3 cg(rw.polys * rw.count * GC::CHUNKS);
+            fwd_col<R, SC, MC, IOK, FAM><<<cg, GC::THREADS, 0, st>>>(data, rw, c.tw, c.twd, c.pc, io);
+        }
+    } else {
         fwd_col<R, S, MINB, IOK, FAM><<<grid, G::THREADS, 0, st>>>(data, rw, c.tw, c.twd, c.pc, io);
+    }
     SHM_LAUNCHED(1);
     fwd_blk<R, S, MINB, BLK, FAM><<<grid, G::THREADS, 0, st>>>(data, rw, c.tw, c.twd, c.pc, io);
 }
