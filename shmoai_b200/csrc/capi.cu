@@ -3,7 +3,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <memory>
+#include <new>
 #include <string>
 
 #include "../../include/shmoai_ckks.h"
@@ -37,13 +39,8 @@ void push4(std::vector<uint64_t> &v, uint64_t c, uint64_t psi_half_inv, uint64_t
 Context::~Context() {
     cudaSetDevice(device);
     release_encode_tables(*this);
-    for (void *p : {(void *)pc, (void *)tw, (void *)twd, (void *)inv_scale_plain, (void *)moddown_scale, (void *)moddown_conv,
-                    (void *)moddown_bytes, (void *)p_inv, (void *)p_mod, (void *)rescale_inv, arena})
+    for (void *p : {tables, (void *)tw, (void *)twd, arena})
         if (p) cudaFree(p);
-    for (auto &l : ks)
-        for (void *p : {(void *)l.modup_scale, (void *)l.modup_conv, (void *)l.rr_scale, (void *)l.rr_conv,
-                        (void *)l.rr_sinv, (void *)l.rr_vs, (void *)l.rr_inv_s, (void *)l.modup_bytes, (void *)l.rr_bytes})
-            if (p) cudaFree(p);
     for (auto &kv : galois_perm) cudaFree(kv.second);
     for (auto &kv : ext_consts)
         for (void *p : kv.second) cudaFree(p);
@@ -102,37 +99,71 @@ void *Context::workspace(size_t bytes) {
 }
 
 // the tables of TwTab for the primes below kF64CentreLimit (zero for the others, which never read
-// them) from the integer tables [QP][4][N]
+// them) from the integer tables [QP][4][N].  Grid (entries / 256, prime and direction)
 template <int R>
-std::vector<double> fp64_twiddles(const std::vector<uint64_t> &primes, const std::vector<uint64_t> &tw) {
+__global__ void fp64_twiddles(const uint64_t *__restrict__ tw, const PrimeConst *__restrict__ pc, double *__restrict__ out) {
     using T = TwTab<R>;
-    std::vector<double> out(primes.size() * 2 * T::DIR, 0.0);
-    for (size_t i = 0; i < primes.size(); i++) {
-        const uint64_t q = primes[i];
-        if (q >= kF64CentreLimit) continue;
-        for (int dir = 0; dir < 2; dir++) {
-            const uint64_t *t = tw.data() + (i * 4 + 2 * dir) * T::N;
-            double *d = out.data() + (i * 2 + dir) * T::DIR;
-            auto centred = [&](uint64_t w) { return w > q / 2 ? (double)w - (double)q : (double)w; };
-            for (uint32_t k = 0; k < T::NAT; k++) d[k] = centred(t[k]);
-            for (uint32_t b = 0; b < T::M; b++)
-                for (uint32_t g = 0; g < T::E; g++) {
-                    const uint32_t u = ((T::M + b) << R) + g;
-                    for (int r = 0; r < R; r++)
-                        for (uint32_t k = 0; k < (1u << r); k++) d[T::slot(b, g, (1u << r) + k)] = centred(t[(u << r) + k]);
-                }
-        }
+    const uint32_t e = blockIdx.x * 256 + threadIdx.x, prime = blockIdx.y / 2, dir = blockIdx.y % 2;
+    const uint64_t q = pc[prime].q, *t = tw + ((size_t)prime * 4 + 2 * dir) * T::N;
+    double v = 0.0;
+    uint32_t at = e;
+    bool used = q < kF64CentreLimit;
+    if (e >= T::NAT) {  // TwTab::slot read backwards
+        const uint32_t x = e - T::NAT, g = (x >> 1) % T::E, b = (x >> 1) / (T::E * T::E / 2);
+        const uint32_t s = (x >> 1) / T::E % (T::E / 2) * 2 + (x & 1), r = 31 - __clz(s | 1);
+        at = (((((T::M + b) << R) + g) << r)) + s - (1u << r);
+        used = used && s;
     }
-    return out;
+    if (used) {
+        const uint64_t w = t[at];
+        v = w > q / 2 ? (double)w - (double)q : (double)w;
+    }
+    out[blockIdx.y * T::DIR + e] = v;
 }
+
+template <int R>
+double *make_fp64_twiddles(uint32_t primes, const uint64_t *tw, const PrimeConst *pc) {
+    double *d = nullptr;
+    SHM_CUDA(cudaMalloc(&d, primes * 2 * TwTab<R>::DIR * sizeof(double)));
+    static_assert(TwTab<R>::DIR % 256 == 0, "whole blocks");
+    fp64_twiddles<R><<<dim3(TwTab<R>::DIR / 256, primes * 2), 256>>>(tw, pc, d);
+    SHM_CUDA(cudaGetLastError());
+    return d;
+}
+
+// A context's constants, put into one buffer and uploaded at once: an allocation and a copy for each of the
+// nine tables of every level take 30 to 200 us a table.
+class Tables {
+    std::vector<uint8_t> bytes;
+    std::vector<std::function<void(uint8_t *)>> set;
+
+public:
+    template <typename T>
+    void add(T *&field, const std::vector<T> &v) {
+        const size_t off = (bytes.size() + 255) / 256 * 256;
+        bytes.resize(off + v.size() * sizeof(T));
+        if (!v.empty()) std::memcpy(bytes.data() + off, v.data(), v.size() * sizeof(T));
+        set.push_back([&field, off](uint8_t *base) { field = reinterpret_cast<T *>(base + off); });
+    }
+    void *finish() {
+        uint8_t *d = upload(bytes);
+        for (auto &f : set) f(d);
+        return d;
+    }
+};
 
 // Row j's block of ConvIO::bytes: slot i's constant c[i] (below q) times 2^(8b) mod q, cut into bytes
 void push_conv_bytes(std::vector<uint8_t> &out, const std::vector<uint64_t> &c, uint64_t q) {
     const size_t base = out.size();
     out.resize(base + 512, 0);
+    const uint64_t w = 256 % q, ws = host::shoup_of(w, q);
+    auto times256 = [&](uint64_t v) {
+        const uint64_t r = v * w - (uint64_t)(((unsigned __int128)v * ws) >> 64) * q;
+        return r >= q ? r - q : r;
+    };
     for (uint32_t i = 0; i < c.size(); i++) {
         uint64_t v = c[i];
-        for (uint32_t b = 0; b < 8; b++, v = host::mulmod(v, 256, q)) {
+        for (uint32_t b = 0; b < 8; b++, v = times256(v)) {
             const uint32_t k = 8 * i + b;
             for (uint32_t o = 0; o < 8; o++) out[base + k / 16 * 128 + o * 16 + k % 16] = (uint8_t)(v >> (8 * o));
         }
@@ -148,10 +179,19 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
     int sms = 0;
     SHM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     c->sms = (uint32_t)sms;
-    int *fault = nullptr;
-    SHM_CUDA(cudaHostAlloc(&fault, sizeof(int), cudaHostAllocMapped));
-    c->fault = std::shared_ptr<int>(fault, [](int *p) { cudaFreeHost(p); });
+    // a page of its own, mapped: cudaHostAlloc of a word takes three times as long (1.3 and 0.4 ms)
+    constexpr size_t kPage = 4096;
+    int *fault = static_cast<int *>(std::aligned_alloc(kPage, kPage));
+    if (!fault) throw std::bad_alloc();
     *fault = 0;
+    if (cudaHostRegister(fault, kPage, cudaHostRegisterMapped) != cudaSuccess) {
+        std::free(fault);
+        SHM_CUDA(cudaGetLastError());
+    }
+    c->fault = std::shared_ptr<int>(fault, [](int *p) {
+        cudaHostUnregister(p);
+        std::free(p);
+    });
     SHM_CUDA(cudaHostGetDevicePointer(&c->fault_dev, fault, 0));
     c->log_n = log_n;
     c->n = 1u << log_n;
@@ -175,6 +215,7 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
         for (uint64_t q : primes) fam |= 1 << bf_mode_of(q);
         c->ntt_families = (fam & ~kFamSmall) == 0 ? kFamSmall : (fam & ~kFamLarge) == 0 ? kFamLarge : kFamAll;
     }
+    Tables tab;
     // per-prime constants and twiddles
     std::vector<uint64_t> tw((size_t)QP * 4 * n), psi_half_inv(QP), sc_plain;
     for (uint32_t i = 0; i < QP; i++) {
@@ -195,10 +236,9 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
         c->h_pc.push_back(p);
         push4(sc_plain, p.n_inv, psi_half_inv[i], q);
     }
-    c->pc = upload(c->h_pc);
+    tab.add(c->pc, c->h_pc);
     c->tw = upload(tw);
-    c->twd = upload(log_n == 16 ? fp64_twiddles<4>(primes, tw) : fp64_twiddles<3>(primes, tw));
-    c->inv_scale_plain = upload(sc_plain);
+    tab.add(c->inv_scale_plain, sc_plain);
 
     // rescale: row L-1 holds q_{L-1}^-1 mod q_j
     std::vector<uint64_t> rinv((size_t)nq * nq * 2, 0);
@@ -208,7 +248,7 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
             rinv[((size_t)(L - 1) * nq + j) * 2] = v;
             rinv[((size_t)(L - 1) * nq + j) * 2 + 1] = host::shoup_of(v, q);
         }
-    c->rescale_inv = upload(rinv);
+    tab.add(c->rescale_inv, rinv);
 
     c->ks.resize(nq + 1);
     if (np) {
@@ -236,16 +276,16 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
             pmod[2 * j] = prod;
             pmod[2 * j + 1] = host::shoup_of(prod, q);
         }
-        c->moddown_scale = upload(mds);
-        c->moddown_conv = upload(mdc);
+        tab.add(c->moddown_scale, mds);
+        tab.add(c->moddown_conv, mdc);
         if (np <= kConvSlots) {
             std::vector<uint8_t> by;
             for (uint32_t j = 0; j < nq; j++)
                 push_conv_bytes(by, {mdc.begin() + (size_t)j * np, mdc.begin() + (size_t)(j + 1) * np}, primes[j]);
-            c->moddown_bytes = upload(by);
+            tab.add(c->moddown_bytes, by);
         }
-        c->p_inv = upload(pinv);
-        c->p_mod = upload(pmod);
+        tab.add(c->p_inv, pinv);
+        tab.add(c->p_mod, pmod);
         c->h_p_mod = pmod;
         // ModUp constants per level
         for (uint32_t L = 1; L <= nq; L++) {
@@ -268,8 +308,8 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
                         conv[((size_t)b * LP + j) * np + i] = host::partial_product(D, i, t);
                 }
             }
-            ks.modup_scale = upload(msc);
-            ks.modup_conv = upload(conv);
+            tab.add(ks.modup_scale, msc);
+            tab.add(ks.modup_conv, conv);
             if (np <= kConvSlots) {
                 std::vector<uint8_t> by;
                 for (uint32_t b = 0; b < ks.beta; b++) {
@@ -278,7 +318,7 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
                         push_conv_bytes(by, {r, r + np}, primes[j < L ? j : nq + (j - L)]);
                     }
                 }
-                ks.modup_bytes = upload(by);
+                tab.add(ks.modup_bytes, by);
             }
             if (L < 2) continue;
             // ModDown by S = q_{L-1} P
@@ -319,17 +359,19 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
                     r.push_back(q - rvs[(size_t)j * 16 + 1]);
                     push_conv_bytes(by, r, q);
                 }
-                ks.rr_bytes = upload(by);
+                tab.add(ks.rr_bytes, by);
             }
             std::vector<double> rinvs(np + 1);
             for (uint32_t k = 0; k <= np; k++) rinvs[k] = 1.0 / (double)S[k];
-            ks.rr_scale = upload(rsc);
-            ks.rr_conv = upload(rconv);
-            ks.rr_sinv = upload(rsinv);
-            ks.rr_vs = upload(rvs);
-            ks.rr_inv_s = upload(rinvs);
+            tab.add(ks.rr_scale, rsc);
+            tab.add(ks.rr_conv, rconv);
+            tab.add(ks.rr_sinv, rsinv);
+            tab.add(ks.rr_vs, rvs);
+            tab.add(ks.rr_inv_s, rinvs);
         }
     }
+    c->tables = tab.finish();
+    c->twd = log_n == 16 ? make_fp64_twiddles<4>(QP, c->tw, c->pc) : make_fp64_twiddles<3>(QP, c->tw, c->pc);
     SHM_CUDA(cudaDeviceSynchronize());
     return c.release();
 }

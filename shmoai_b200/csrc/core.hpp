@@ -80,6 +80,7 @@ struct Context {
     int ntt_variant = kNttDefault;      // index into kNttVariants (set by the autotuner)
     int ntt_families = 0;               // the NTT instantiation for the primes' butterfly families (kFam*)
     uint32_t ip_chunk_bytes = 32768;    // shared memory per Sh-Rot inner-product block (autotuned)
+    void *tables = nullptr;             // holds every table below but tw and twd, and the levels'
     std::vector<PrimeConst> h_pc;       // host copy
     PrimeConst *pc = nullptr;           // [QP]
     uint64_t *tw = nullptr;             // [QP][4][N]
