@@ -234,7 +234,7 @@ int shm_fmt_switch_backward(const shm_context *ctx, const uint64_t *sh, uint32_t
  * shm_shared_rotate_ext: Sh-Rot of shared-a groups with extended outputs outs[e]
  *   [n_groups][n_members+1][L+n_p][N] (no ModDown); the input is ordinary groups
  *   [n_groups][n_members+1][L][N] (in_ext = 0) or extended groups (in_ext = 1, whose a rows
- *   are brought down once before the ModUp). */
+ *   are brought down once before the ModUp).  outs must not overlap the b rows of the input. */
 int shm_extend(const shm_context *ctx, const uint64_t *in, uint64_t *out, uint32_t n_polys, uint32_t L,
                void *stream);
 int shm_add_ext(const shm_context *ctx, const uint64_t *a, const uint64_t *b, uint64_t *out, uint32_t n_polys,

@@ -411,9 +411,10 @@ void moddown_ext(const Context &c, uint64_t *ext, uint64_t *out, uint32_t n_poly
 }
 
 size_t shared_rotate_ext_ws_words(const Context &c, uint32_t n_groups, uint32_t n, uint32_t L) {
-    const uint32_t beta = (L + c.np - 1) / c.np, LP = L + c.np, H = n + 1;
-    // x, up, acc, the a rows (extended input), their ModDown and its delta
-    return (size_t)n_groups * c.n * (L + (size_t)beta * LP + (size_t)H * LP + LP + 2 * (size_t)L);
+    const uint32_t beta = (L + c.np - 1) / c.np, LP = L + c.np;
+    (void)n;
+    // x, up, the a rows (extended input), their ModDown and its delta; the inner products go to the outputs
+    return (size_t)n_groups * c.n * (L + (size_t)beta * LP + LP + 2 * (size_t)L);
 }
 
 void shared_rotate_ext(const Context &c, const uint64_t *in, bool in_ext, uint32_t n_groups, uint32_t n, uint32_t L,
@@ -423,8 +424,8 @@ void shared_rotate_ext(const Context &c, const uint64_t *in, bool in_ext, uint32
     check_shape(c, L, beta, H);
     if (beta > c.dnum) throw std::invalid_argument("level needs more key digits than the key holds");
     const size_t N = c.n, ln = (size_t)L * N;
-    uint64_t *x = ws, *up = x + (size_t)n_groups * ln, *acc = up + (size_t)n_groups * beta * LP * N;
-    uint64_t *arow = acc + (size_t)n_groups * H * LP * N, *aq = arow + (size_t)n_groups * LP * N;
+    uint64_t *x = ws, *up = x + (size_t)n_groups * ln;
+    uint64_t *arow = up + (size_t)n_groups * beta * LP * N, *aq = arow + (size_t)n_groups * LP * N;
     uint64_t *delta = aq + (size_t)n_groups * ln;
     const size_t g_words = (size_t)H * (in_ext ? LP : L) * N;  // one input group
     OwnLimbs own;
