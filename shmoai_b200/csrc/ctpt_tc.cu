@@ -680,7 +680,6 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
 // ---------------------------------------------------------------- CRT fold
 struct CrtLimb {
     uint64_t c[kMaxMods];  // c_t mod q_l
-    uint64_t M;            // M mod q_l
     uint64_t Mneg;         // q_l - (M mod q_l), below q_l
     uint64_t base;         // 128 T M - 128 sum_t c_t mod q_l
 };
@@ -905,7 +904,6 @@ Plan make_plan(const Context &c, uint32_t L, uint64_t max_l1) {
             CrtLimb &cl = p.limbs[(size_t)(T - p.T_min) * L + l];
             uint64_t q = c.primes[l], M = 1;
             for (uint32_t u = 0; u < T; u++) M = host::mulmod(M, cand[u], q);
-            cl.M = M;
             cl.Mneg = (q - M) % q;
             for (uint32_t t = 0; t < T; t++) {
                 uint32_t m = cand[t], Mt_mod_m = 1;
@@ -971,13 +969,15 @@ size_t ctpt_tc_ws_bytes(const Context &c, uint32_t n_in, uint32_t n_out, uint32_
     return (size_t)kMaxMods * (chunk * Kp + (uint64_t)Np * Kp + (uint64_t)n_out * chunk) + kCrtTabBytes;
 }
 
-// f(T) with the modulus count as a compile-time constant
+// f(T) with the modulus count as a compile-time constant.  No prime takes one: 1 mod 2N, it is above 2^13, and
+// log2 |S| + 1.05 above 14 asks for two.
+constexpr uint32_t kLeastHi32Mods = 6;  // primes from 2^40 up ask for 41 bits, five moduli hold less than 40
 template <class F>
 static void with_moduli(uint32_t T, F &&f) {
 #define SHM_T_CASE(n) \
     case n: f(std::integral_constant<uint32_t, n>{}); break;
     switch (T) {
-        SHM_T_CASE(1) SHM_T_CASE(2) SHM_T_CASE(3) SHM_T_CASE(4) SHM_T_CASE(5) SHM_T_CASE(6) SHM_T_CASE(7)
+        SHM_T_CASE(2) SHM_T_CASE(3) SHM_T_CASE(4) SHM_T_CASE(5) SHM_T_CASE(6) SHM_T_CASE(7)
         SHM_T_CASE(8) SHM_T_CASE(9) SHM_T_CASE(10) SHM_T_CASE(11) SHM_T_CASE(12) SHM_T_CASE(13) SHM_T_CASE(14)
         SHM_T_CASE(15) SHM_T_CASE(16) SHM_T_CASE(17) SHM_T_CASE(18) SHM_T_CASE(19) SHM_T_CASE(20)
         default: throw std::invalid_argument("ct-pt matmul: modulus count out of range");
@@ -1068,7 +1068,10 @@ void ctpt_matmul_tc(const Context &c, const uint64_t *X, const int64_t *W, uint6
         const uint32_t crt_threads = chunk % 1024 == 0 ? 256 : 64;
         const dim3 cgrid((uint32_t)((cur / 4 + crt_threads - 1) / crt_threads), n_out);
         with_moduli(Tc, [&](auto n) {
-            const auto f = plan.hi32 ? crt_kernel<true, decltype(n)::value> : crt_kernel<false, decltype(n)::value>;
+            constexpr uint32_t kT = decltype(n)::value;
+            auto f = crt_kernel<false, kT>;
+            if constexpr (kT >= kLeastHi32Mods)
+                if (plan.hi32) f = crt_kernel<true, kT>;
             f<<<cgrid, crt_threads, 0, st>>>(RES, Y, tab_c, n_out, cur, r0, R, L, c.log_n, c.pc);
         });
         SHM_CUDA(cudaGetLastError());

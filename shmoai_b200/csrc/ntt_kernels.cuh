@@ -432,11 +432,9 @@ void launch_inv_v(const Context &c, const InvArgs &v, const NttRows &rw, cudaStr
 template <int R, int IOK, int FAM>
 void launch_fwd_f(const Context &c, uint64_t *data, const NttRows &rw, cudaStream_t st, const NttIO &io) {
     switch (c.ntt_variant) {
-#ifndef SHM_NTT_ONE_TILE  // a development build may leave the other tiles out
         case 1: launch_fwd_v<R, 16, 3, IOK, FAM>(c, data, rw, st, io); break;
         case 2: launch_fwd_v<R, 8, 8, IOK, FAM>(c, data, rw, st, io); break;
         case 3: launch_fwd_v<R, 8, 6, IOK, FAM>(c, data, rw, st, io); break;
-#endif
         default: launch_fwd_v<R, 16, 4, IOK, FAM>(c, data, rw, st, io); break;
     }
 }
@@ -456,11 +454,9 @@ void launch_fwd(const Context &c, int kind, uint64_t *data, const NttRows &rw, c
 template <int R, int FAM>
 void launch_inv(const Context &c, const InvArgs &v, const NttRows &rw, cudaStream_t st) {
     switch (c.ntt_variant) {
-#ifndef SHM_NTT_ONE_TILE
         case 1: launch_inv_v<R, 16, 3, FAM>(c, v, rw, st); break;
         case 2: launch_inv_v<R, 8, 8, FAM>(c, v, rw, st); break;
         case 3: launch_inv_v<R, 8, 6, FAM>(c, v, rw, st); break;
-#endif
         default: launch_inv_v<R, 16, 4, FAM>(c, v, rw, st); break;
     }
 }
