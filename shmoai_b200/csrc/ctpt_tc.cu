@@ -422,8 +422,9 @@ __device__ __forceinline__ bool role_wait(uint32_t bar, uint32_t parity, int lim
 }
 
 // TMA_A: both operands come by TMA (one thread issues the X tile's and the weight stages' loads,
-// 64-byte swizzle, completion on their mbarriers) instead of the producer warps' cp.async
-template <bool TMA_A>
+// 64-byte swizzle, completion on their mbarriers) instead of the producer warps' cp.async.  LIMITED: `limit` polls a
+// wait instead of kSpinLimit (a run-time bound of every wait: 1.33 ms for 1.26 a pass of 768 x 768)
+template <bool TMA_A, bool LIMITED>
 __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8_t *__restrict__ XP,
                                                                       const int8_t *__restrict__ WP,
                                                                       uint8_t *__restrict__ RES, uint32_t Kp,
@@ -476,7 +477,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) mma_persistent_kernel(const int8
     asm volatile("tcgen05.fence::after_thread_sync;\n");
     const uint32_t tmem = tmem_base;
     const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((kBM >> 4) << 24);
-    auto wait = [&](uint64_t *bar, uint32_t parity) { return role_wait(smem_u32(bar), parity, limit, &failed); };
+    auto wait = [&](uint64_t *bar, uint32_t parity) { return role_wait(smem_u32(bar), parity, LIMITED ? limit : kSpinLimit, &failed); };
     auto arrive = [](uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar)); };
 
     if (tid < kProducers && !(TMA_A && warp > 0)) {
@@ -1016,9 +1017,14 @@ void ctpt_matmul_tc(const Context &c, const uint64_t *X, const int64_t *W, uint6
     std::memset(&tmA, 0, sizeof tmA);
     std::memset(&tmX, 0, sizeof tmX);
     const bool tma_a = resident && operand_tensor_map(&tmA, WP, Kp, (uint64_t)T * Np, kBM);
+    const bool limited = c.wait_limit != kSpinLimit;
+    auto persistent = [limited](bool tma) {
+        return limited ? (tma ? mma_persistent_kernel<true, true> : mma_persistent_kernel<false, true>)
+                       : (tma ? mma_persistent_kernel<true, false> : mma_persistent_kernel<false, false>);
+    };
     if (resident)
-        SHM_CUDA(cudaFuncSetAttribute(tma_a ? mma_persistent_kernel<true> : mma_persistent_kernel<false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemP));
+        for (const bool tma : {false, tma_a})  // a pass whose X map is refused copies its operands
+            SHM_CUDA(cudaFuncSetAttribute(persistent(tma), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemP));
     else
         SHM_CUDA(cudaFuncSetAttribute(mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     int sms = 0;
@@ -1050,14 +1056,8 @@ void ctpt_matmul_tc(const Context &c, const uint64_t *X, const int64_t *W, uint6
             // the X planes of this pass, [T * cur][Kp], as 256-row boxes (a pass's planes have its own
             // column count)
             const bool tma = tma_a && operand_tensor_map(&tmX, XP, Kp, (uint64_t)Tc * cur, kBN);
-            if (tma)
-                mma_persistent_kernel<true>
-                    <<<grid, kThreadsP, kSmemP, st>>>(XP, WP, RES, Kp, Np, n_out, cur, Tc, err, acc_small, c.wait_limit,
-                                                      tmA, tmX);
-            else
-                mma_persistent_kernel<false>
-                    <<<grid, kThreadsP, kSmemP, st>>>(XP, WP, RES, Kp, Np, n_out, cur, Tc, err, acc_small, c.wait_limit,
-                                                      tmA, tmX);
+            persistent(tma)<<<grid, kThreadsP, kSmemP, st>>>(XP, WP, RES, Kp, Np, n_out, cur, Tc, err, acc_small,
+                                                             c.wait_limit, tmA, tmX);
         } else {
             mma_kernel<<<dim3(Np / kBM, (uint32_t)(cur / kBN), Tc), kThreads, kSmem, st>>>(XP, WP, RES, Kp, Np, n_out,
                                                                                           cur, err, acc_small, c.wait_limit);
