@@ -10,8 +10,8 @@
 // pipe leaves V - Q q within q/2 + 2^32 of zero: the double the FP64 butterflies take, written as such
 // (integer families add q to a negative one).
 //
-// What bounds it: issue (about 42 instructions a coefficient and row, a third of them the wait, address
-// and constant handling of a step) at 16 warps per SM, 0.45 of the HBM rate.  On the CUDA cores the same sum
+// What bounds it: issue (47 instructions a coefficient and row, a third of them the wait, address and
+// constant handling of a step) at 16 warps per SM and 128 registers, 0.53 of the measured copy rate.  On the CUDA cores the same sum
 // of five terms took 20 wide multiplies (which issue at a quarter of the rate), a 128-bit fold and a Barrett
 // reduction inside the NTT's column phase, where each row also re-read the set's limbs from L2: 190 issued
 // instructions per coefficient against 55 for the plain column phase.  Eight ciphertexts at 27 limbs (48

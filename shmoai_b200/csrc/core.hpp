@@ -148,12 +148,13 @@ void conv_rows(const Context &c, const ConvIO &io, cudaStream_t st);
 // t: [n_polys][L-1][N] scratch between the two phases
 void ntt_forward_rescale(const Context &c, const RescaleIO &io, uint64_t *t, uint32_t n_polys, uint32_t L,
                          cudaStream_t st);
-// ModDown's conversion, forward NTT and combine in one launch pair (ModDownIO); delta:
-// [n_polys][L][N] scratch between the two phases
-// ModUp's base conversion, forward NTT and the digit copies in one launch pair (ModUpIO): up
-// [n_cts][beta][LP][N]
+// ModUp's base conversions and forward NTT (ModUpIO) into up [n_cts][beta][LP][N], but for the digits' own
+// rows: conv_rows writes the converted rows in coefficient form and a plain transform follows, or, with more limbs
+// than conv_rows takes, the column phase's loads convert
 void ntt_forward_modup(const Context &c, const ModUpIO &mu, uint64_t *up, uint32_t n_cts, uint32_t beta,
                        cudaStream_t st);
+// ModDown's conversion (in the same two ways), forward NTT and combine (ModDownIO); delta: [n_polys][L][N]
+// scratch for the converted rows and between the phases
 void ntt_forward_moddown(const Context &c, const ModDownIO &md, uint64_t *delta, uint32_t n_polys, uint32_t L,
                          cudaStream_t st);
 

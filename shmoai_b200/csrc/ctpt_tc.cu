@@ -137,8 +137,8 @@ __device__ __forceinline__ uint32_t acc_bytes(const uint32_t *v, uint32_t t, int
 // What bounds it: HBM (768 inputs, 131,072 columns, 12 moduli: 2.0 GB a pass).  The input groups of a column
 // tile are consecutive blocks, so the 64-byte pieces of a plane's row are written at about the same time and
 // leave L2 as whole rows, and row i of a tile is rotated by i / 4 columns, so the 16 rows that a half-warp
-// reads lie in different banks (unrotated, padded rows: four to a bank).  768 to 768 ciphertexts at 13 limbs
-// went from 33.5 to 30.4 ms by the two, 100 to 70 at 7 limbs from 1.87 to 1.76 ms.
+// reads lie in different banks (unrotated, padded rows: four to a bank).  The two take 3.1 ms off 768 to 768
+// ciphertexts at 13 limbs (29.1 in all), 0.11 off 100 to 70 at 7 limbs (1.71).
 constexpr uint32_t kXresTiles = 2;
 constexpr uint32_t kXresSmem = 2 * 64 * 64 * 8;
 
@@ -706,8 +706,8 @@ constexpr size_t kCrtTabBytes = 256 + sizeof(CrtLimb) * 64 * kMaxMods;
 // hi fits 32 bits and one FP64 quotient replaces Barrett's two 64 x 64-bit high products, and the sums are
 // taken byte by byte: four moduli's residues of a column (a 4 x 4 byte transpose) times the same four moduli's
 // bytes of c_t (seven) and F_t (three) are ten four-way byte products, 30 a column for 12 moduli in place of
-// 12 wide and 24 plain multiply-adds and 12 byte extracts.  768 to 768 ciphertexts at 13 limbs 29.5 and 28.8 ms
-// in alternated runs, 100 to 70 at 7 limbs 1.78 and 1.74 ms.  The residue words (one per modulus,
+// 12 wide and 24 plain multiply-adds and 12 byte extracts.  They take 0.7 ms off
+// 768 to 768 ciphertexts at 13 limbs, 0.04 off 100 to 70 at 7 limbs (alternated runs).  The residue words (one per modulus,
 // read once: streaming loads) are requested before the fold.  T at compile time, as in xres_kernel (232
 // instructions a column were issued for 12 moduli under guards up to 20: 0.77 ms a pass of 768 x 131,072).
 template <bool HI32, uint32_t T>

@@ -232,8 +232,8 @@ void modup_into(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n
     if (np > kMaxAlpha || beta > kMaxBeta || LP > 64) throw std::invalid_argument("key-switching shape too large");
     const LevelKS &ks = c.ks[L];
     ntt_inverse(c, x, rows_of(c, n_cts, L, L), ks.modup_scale, st, d, d_stride);
-    // the conversion is computed in the forward NTT's load: the converted limbs never go through HBM in
-    // coefficient form.  The digits' own rows of up are not written: the inner products read d.
+    // the converted rows, then their NTT (ntt_forward_modup).  The digits' own rows of up are not written: the
+    // inner products read d (own_limbs).
     ModUpIO mu;
     mu.x = x;
     mu.conv = ks.modup_conv;

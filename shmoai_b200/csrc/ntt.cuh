@@ -32,9 +32,9 @@ struct NttVariant {
 constexpr NttVariant kNttVariants[] = {{16, 4}, {16, 3}, {8, 8}, {8, 6}};
 constexpr int kNttVariantCount = 4;
 // The tile until one is tuned or set: 8 x 6 (80 registers, no spills; the small tile spreads few rows more
-// evenly).  Medians of alternated runs at 16 x 4 and 8 x 6: forward and inverse of 117 x 35 limbs 3.93 and 3.56
-// ms, a product at 24 limbs 362 and 333 us, five rotations at 17 limbs 636 and 608 us, sixteen products at 27
-// limbs 4.21 and 4.13 ms; 8 x 5 and 8 x 7 lie between.
+// evenly).  Its share of the time at 16 x 4, medians of alternated runs: forward and inverse of 117 x 35 limbs
+// 0.91, a product at 24 limbs 0.92 (333 of 362 us), five rotations at 17 limbs 0.96, sixteen products at 27 limbs
+// 0.98; 8 x 5 and 8 x 7 lie between.
 constexpr int kNttDefault = 3;
 
 // The rows a launch transforms: slots [first, first + count) of each of `polys` polynomials of
@@ -64,10 +64,10 @@ struct RescaleIO {
     const uint64_t *inv = nullptr;   // [L-1][2]: q_{L-1}^-1 mod q_j and its Shoup companion
 };
 
-// The ModDown's forward NTT (ntt_forward_moddown): rows (poly, j < L) of the delta buffer are
-// read as the base conversion sum_k z_k (phat_k mod q_j) of the INTT'd special-prime limbs
-// z_k = acc[poly][L + k], and written as (acc[poly][j] - NTT(...)) P^-1 (+ add, or
-// + add * add_mul[j]) into out;
+// The ModDown's forward NTT (ntt_forward_moddown): rows (poly, j < L) of the delta buffer are the base
+// conversion sum_k z_k (phat_k mod q_j) of the INTT'd special-prime limbs z_k = acc[poly][L + k] (left there by
+// conv_rows when `bytes` is given, else formed by the column phase's loads), and written as
+// (acc[poly][j] - NTT(...)) P^-1 (+ add, or + add * add_mul[j]) into out;
 // poly = ct * H + h.  The add term of rows h < n_add is read at perm[pos] for rows h < n_perm.
 struct ModDownIO {
     const uint64_t *acc = nullptr;   // [polys][L + np][N]
@@ -88,10 +88,10 @@ struct ModDownIO {
 };
 
 // ModUp's forward NTT (ntt_forward_modup): row (ct, b, j) of up [n_cts][beta][LP][N].  For j
-// outside digit b (limbs [b alpha, min((b+1) alpha, L))) the column kernel reads the base
-// conversion sum_i y_i (qhat_i mod t_j) of the digit's INTT'd, qhat^-1-scaled limbs
-// y = x[ct][b alpha ..] (coefficient form) and the row is transformed; rows j inside the digit are
-// left alone (NttRows::skip).  The converted digits are never stored in coefficient form.
+// outside digit b (limbs [b alpha, min((b+1) alpha, L))) the row is the base conversion
+// sum_i y_i (qhat_i mod t_j) of the digit's INTT'd, qhat^-1-scaled limbs y = x[ct][b alpha ..] (coefficient form;
+// left in up by conv_rows when `bytes` is given, else formed by the column phase's loads) and is transformed;
+// rows j inside the digit are left alone (NttRows::skip).
 struct ModUpIO {
     const uint64_t *x = nullptr;     // [n_cts][L][N]
     const uint64_t *conv = nullptr;  // [beta][LP][np]: qhat_i mod t_j of the level's digits
@@ -162,9 +162,9 @@ __device__ __forceinline__ void ct_bf_grow(uint64_t &x, uint64_t &y, uint64_t w,
 //
 // What bounds it: the FP64 pipe (eight operations per butterfly and, for 51-bit primes, three per
 // centring) and HBM (each phase reads and writes every limb) within 1.5x of each other.  117 x 35
-// limbs at the bootstrapping primes, forward of one batch and inverse of another: 5.56 ms with two
-// table words per forward twiddle and integer Gentleman-Sande butterflies (whose low products kept
-// the integer-multiply pipe busy), 4.06 ms so.
+// limbs at the bootstrapping primes, forward of one batch and inverse of another, 16 x 4 tiles: 5.56 ms
+// with two table words per forward twiddle and integer Gentleman-Sande butterflies (whose low products
+// kept the integer-multiply pipe busy), 4.06 ms so (3.80 at 8 x 6).
 //
 // kBfF64, q < 2^52 / 36.  Forward: inputs below q, a stage adds less than 0.65 q, values stay below
 // 11 q over all 16 stages with no reduction.  Inverse (x + y, (x - y) w): from inputs below 1.8 q a
