@@ -140,8 +140,9 @@ class Tables {
 public:
     template <typename T>
     void add(T *&field, const std::vector<T> &v) {
-        const size_t off = (bytes.size() + 255) / 256 * 256;
-        bytes.resize(off + v.size() * sizeof(T));
+        const size_t off = (bytes.size() + 255) / 256 * 256, end = off + v.size() * sizeof(T);
+        if (end > bytes.capacity()) bytes.reserve(std::max(4 * bytes.capacity(), std::max<size_t>(end, 1 << 20)));
+        bytes.resize(end);
         if (!v.empty()) std::memcpy(bytes.data() + off, v.data(), v.size() * sizeof(T));
         set.push_back([&field, off](uint8_t *base) { field = reinterpret_cast<T *>(base + off); });
     }
@@ -152,21 +153,34 @@ public:
     }
 };
 
-// Row j's block of ConvIO::bytes: slot i's constant c[i] (below q) times 2^(8b) mod q, cut into bytes
-void push_conv_bytes(std::vector<uint8_t> &out, const std::vector<uint64_t> &c, uint64_t q) {
-    const size_t base = out.size();
-    out.resize(base + 512, 0);
+// bytes of eight words transposed: byte b of word o becomes byte o of word b
+void transpose_bytes(uint64_t (&x)[8]) {
+    const uint64_t mask[3] = {0x00FF00FF00FF00FFull, 0x0000FFFF0000FFFFull, 0x00000000FFFFFFFFull};
+    for (int s = 0; s < 3; s++)
+        for (int i = 0; i < 8; i++)
+            if (!(i >> s & 1)) {
+                uint64_t &a = x[i], &b = x[i | 1 << s];
+                const uint64_t t = ((a >> (8 << s)) ^ b) & mask[s];
+                b ^= t;
+                a ^= t << (8 << s);
+            }
+}
+
+constexpr size_t kConvRowBytes = 512;
+
+// A row's block of ConvIO::bytes (512 zeros before): slot i's constant c[i] (below q) times 2^(8b) mod q, cut
+// into bytes.  For a fixed byte o the eight b of a slot are neighbours.
+void conv_bytes_row(uint8_t *row, const uint64_t *c, uint32_t slots, uint64_t q) {
     const uint64_t w = 256 % q, ws = host::shoup_of(w, q);
-    auto times256 = [&](uint64_t v) {
-        const uint64_t r = v * w - (uint64_t)(((unsigned __int128)v * ws) >> 64) * q;
-        return r >= q ? r - q : r;
-    };
-    for (uint32_t i = 0; i < c.size(); i++) {
-        uint64_t v = c[i];
-        for (uint32_t b = 0; b < 8; b++, v = times256(v)) {
-            const uint32_t k = 8 * i + b;
-            for (uint32_t o = 0; o < 8; o++) out[base + k / 16 * 128 + o * 16 + k % 16] = (uint8_t)(v >> (8 * o));
+    for (uint32_t i = 0; i < slots; i++) {
+        uint64_t x[8], v = c[i];
+        for (uint32_t b = 0; b < 8; b++) {
+            x[b] = v;
+            v = v * w - (uint64_t)(((unsigned __int128)v * ws) >> 64) * q;
+            if (v >= q) v -= q;
         }
+        transpose_bytes(x);
+        for (uint32_t o = 0; o < 8; o++) std::memcpy(row + i / 2 * 128 + o * 16 + i % 2 * 8, &x[o], 8);
     }
 }
 
@@ -279,9 +293,9 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
         tab.add(c->moddown_scale, mds);
         tab.add(c->moddown_conv, mdc);
         if (np <= kConvSlots) {
-            std::vector<uint8_t> by;
+            std::vector<uint8_t> by(nq * kConvRowBytes);
             for (uint32_t j = 0; j < nq; j++)
-                push_conv_bytes(by, {mdc.begin() + (size_t)j * np, mdc.begin() + (size_t)(j + 1) * np}, primes[j]);
+                conv_bytes_row(by.data() + j * kConvRowBytes, mdc.data() + (size_t)j * np, np, primes[j]);
             tab.add(c->moddown_bytes, by);
         }
         tab.add(c->p_inv, pinv);
@@ -310,13 +324,15 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
             }
             tab.add(ks.modup_scale, msc);
             tab.add(ks.modup_conv, conv);
-            if (np <= kConvSlots) {
-                std::vector<uint8_t> by;
-                for (uint32_t b = 0; b < ks.beta; b++) {
-                    for (uint32_t j = 0; j < LP; j++) {
-                        const auto r = conv.begin() + ((size_t)b * LP + j) * np;
-                        push_conv_bytes(by, {r, r + np}, primes[j < L ? j : nq + (j - L)]);
-                    }
+            // half a kilobyte a row: only for levels that a key switch takes (on a chain of 120 primes all levels'
+            // rows would be 150 MB)
+            const bool switched = keyswitch_fits(np, L);
+            if (np <= kConvSlots && switched) {
+                std::vector<uint8_t> by((size_t)ks.beta * LP * kConvRowBytes);
+                for (uint32_t r = 0; r < ks.beta * LP; r++) {
+                    const uint32_t j = r % LP;
+                    conv_bytes_row(by.data() + r * kConvRowBytes, conv.data() + (size_t)r * np, np,
+                                   primes[j < L ? j : nq + (j - L)]);
                 }
                 tab.add(ks.modup_bytes, by);
             }
@@ -351,13 +367,13 @@ Context *create_context(uint32_t log_n, const std::vector<uint64_t> &primes, uin
                 for (uint32_t k = 0; k <= np; k++) Sq = host::mulmod(Sq, S[k] % q, q);
                 for (uint32_t v = 0; v < 16; v++) rvs[(size_t)j * 16 + v] = host::mulmod(v, Sq, q);
             }
-            if (np + 2 <= kConvSlots) {  // np + 1 limbs and the overflow count, whose constant is -S
-                std::vector<uint8_t> by;
+            if (np + 2 <= kConvSlots && switched) {  // np + 1 limbs and the overflow count, whose constant is -S
+                std::vector<uint8_t> by((L - 1) * kConvRowBytes);
+                std::vector<uint64_t> r(np + 2);
                 for (uint32_t j = 0; j + 1 < L; j++) {
-                    const uint64_t q = primes[j];
-                    std::vector<uint64_t> r(rconv.begin() + (size_t)j * (np + 1), rconv.begin() + (size_t)(j + 1) * (np + 1));
-                    r.push_back(q - rvs[(size_t)j * 16 + 1]);
-                    push_conv_bytes(by, r, q);
+                    std::copy_n(rconv.begin() + (size_t)j * (np + 1), np + 1, r.begin());
+                    r[np + 1] = primes[j] - rvs[(size_t)j * 16 + 1];
+                    conv_bytes_row(by.data() + j * kConvRowBytes, r.data(), np + 2, primes[j]);
                 }
                 tab.add(ks.rr_bytes, by);
             }

@@ -116,6 +116,11 @@ struct Context {
     cudaMemPool_t mempool();
 };
 
+// Levels that the key-switching kernels take: up to 16 digits of up to 16 limbs, 64 limbs in all
+inline bool keyswitch_fits(uint32_t np, uint32_t L) {
+    return np >= 1 && np <= 16 && (L + np - 1) / np <= 16 && L + np <= 64;
+}
+
 // throws once a kernel has given up a wait: results of calls since the last look may be missing
 inline void check_fault(const int *fault) {
     if (*(const volatile int *)fault)

@@ -18,8 +18,6 @@ namespace shm {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kMaxAlpha = 16;
-constexpr int kMaxBeta = 16;
 
 // acc[ct][h][j][k] = sum_b up[ct][b][j][perm[k]] * key[b][h][prime(j)][k]   (perm = identity if null);
 // limb j of its own digit j / np is read from d, when given (ModUp leaves it there: it is unchanged)
@@ -145,7 +143,7 @@ void relin_rescale(const Context &c, const uint64_t *ct3, uint32_t n_cts, uint32
     if (L < 2 || L > c.nq) throw std::invalid_argument("relinearize-rescale needs 2 <= L <= n_q");
     const uint32_t np = c.np, beta = (L + np - 1) / np, LP = L + np;
     if (beta > c.dnum) throw std::invalid_argument("level needs more key digits than the key holds");
-    if (np > kMaxAlpha || beta > kMaxBeta || LP > 64) throw std::invalid_argument("key-switching shape too large");
+    if (!keyswitch_fits(np, L)) throw std::invalid_argument("key-switching shape too large");
     const size_t n = c.n, ln = (size_t)L * n;
     uint64_t *x = ws;
     uint64_t *up = x + (size_t)n_cts * L * n;
@@ -207,7 +205,7 @@ void keyswitch(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n_
     if (L < 1 || L > c.nq) throw std::invalid_argument("level out of range");
     const uint32_t np = c.np, beta = (L + np - 1) / np, LP = L + np;
     if (beta > c.dnum) throw std::invalid_argument("level needs more key digits than the key holds");
-    if (np > kMaxAlpha || beta > kMaxBeta || LP > 64) throw std::invalid_argument("key-switching shape too large");
+    if (!keyswitch_fits(np, L)) throw std::invalid_argument("key-switching shape too large");
     const size_t n = c.n;
     uint64_t *x = ws;                                   // [n_cts][L][N]
     uint64_t *up = x + (size_t)n_cts * L * n;           // [n_cts][beta][LP][N]
@@ -229,7 +227,7 @@ void keyswitch(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n_
 void modup_into(const Context &c, const uint64_t *d, size_t d_stride, uint32_t n_cts, uint32_t L, uint64_t *x,
                 uint64_t *up, cudaStream_t st) {
     const uint32_t np = c.np, beta = (L + np - 1) / np, LP = L + np;
-    if (np > kMaxAlpha || beta > kMaxBeta || LP > 64) throw std::invalid_argument("key-switching shape too large");
+    if (!keyswitch_fits(np, L)) throw std::invalid_argument("key-switching shape too large");
     const LevelKS &ks = c.ks[L];
     ntt_inverse(c, x, rows_of(c, n_cts, L, L), ks.modup_scale, st, d, d_stride);
     // the converted rows, then their NTT (ntt_forward_modup).  The digits' own rows of up are not written: the
@@ -274,7 +272,7 @@ void apply_galois_hoisted(const Context &c, const uint64_t *ct, uint32_t n_cts, 
     if (L < 1 || L > c.nq) throw std::invalid_argument("level out of range");
     const uint32_t np = c.np, beta = (L + np - 1) / np, LP = L + np;
     if (beta > c.dnum) throw std::invalid_argument("level needs more key digits than the key holds");
-    if (np > kMaxAlpha || beta > kMaxBeta || LP > 64) throw std::invalid_argument("key-switching shape too large");
+    if (!keyswitch_fits(np, L)) throw std::invalid_argument("key-switching shape too large");
     const size_t n = c.n, ln = (size_t)L * n;
     uint64_t *x = ws;
     uint64_t *up = x + (size_t)n_cts * L * n;
